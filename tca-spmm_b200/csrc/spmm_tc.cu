@@ -11,26 +11,33 @@
 //
 // Work items are (job, window, NT-wide slice of N); persistent CTAs (one per
 // SM) stream the chunks of their items through a ring of kStages (A tile,
-// B tile, entry staging) stages, with decoupled roles:
-//   * four loader warps, taking chunks in turn, move every byte through the
-//     TMA engine: the 64 B rows of the chunk -- one tiled box per 64 columns
-//     of N when its columns are 64 consecutive rows of B, else tile::gather4
-//     of the condensed columns (4 rows x 128 bytes per instruction into a
-//     128-byte swizzled N-major tile; padding columns and n >= N are out of
-//     the tensor and arrive as zeros) -- and either the chunk's pre-rendered,
-//     pre-swizzled dense A tile (chunks with >= 512 nonzeros: one 16 KB
-//     cp.async.bulk) or its packed entries (cp.async.bulk into the stage's
-//     staging buffer);
-//   * scatter warps (two groups taking chunks in turn), once a stage's
-//     entries landed, zero its A tile and scatter them into the swizzled
-//     K-major layout;
+// B tile) stages, with decoupled roles:
+//   * two loader warps move every byte through the TMA engine: one the 64 B
+//     rows of the chunk -- one box for the whole slice when its columns are 64
+//     consecutive rows of B, else tile::gather4 of the condensed columns (4
+//     rows x 128 bytes per instruction into a 128-byte swizzled N-major tile;
+//     padding columns and n >= N are out of the tensor and arrive as zeros) --,
+//     the other the chunk's pre-rendered, pre-swizzled dense A tile (chunks
+//     with >= 512 nonzeros: one 16 KB cp.async.bulk) or its packed entries
+//     (cp.async.bulk into a staging slot, four chunks ahead);
+//   * scatter warps, once a sparse chunk's entries landed and its stage is
+//     free, zero its A tile and scatter them into the swizzled K-major layout;
 //   * one MMA lane issues 4 tcgen05.mma (K = 16 each) per chunk into the FP32
 //     accumulator in tensor memory and releases the stage with tcgen05.commit;
 //   * finally 4 warps read the accumulator (TMEM lane = row) and store
 //     alpha * D + beta * C to C[perm[row]] (FP16 or FP32).
-// Per-thread 16-byte cp.async was measured to issue only ~13 B/clock/SM for
-// the B gather, which left the tensor cores idle; the TMA engine does not
-// occupy the issuing threads.
+//
+// What bounds it: a chunk of 128 x 256 x 64 takes the tensor core 512 cycles
+// (0.27 us at 1.9 GHz), and loading its 48 KB takes a ring without MMAs 0.38
+// us when the images come from HBM (148 CTAs). The loaders decide whether that
+// rate is reached: the issue of one TMA instruction takes ~0.1 us, so the
+// chunk's two are issued by two warps, by one elected lane each that walks
+// ready-made records. %clock traces, 4096 x 4096 at 90 %, N = 1024 (128 CTAs,
+// 64 chunks each): one loader warp behind `lane == 0` 0.36 us per chunk,
+// elected lane 0.30, two loaders 0.27; the call went from 46.0 to 34.8 us with
+// the coalesced stores of store_rows (3.5 -> 2.4 us of a tile's epilogue), the
+// 32-problem sweep step from 60.6 to 55.2 us, the 24-layer batch from 100.9 to
+// 80.6 us.
 // Every mbarrier wait is bounded (about one second of %globaltimer); on
 // expiry the CTA records kStatusTimeout in the job's status word and runs to
 // completion without hanging. No load uses cluster multicast.
@@ -46,22 +53,25 @@
 namespace tca {
 namespace {
 
-constexpr int kScatterThreads = 128; // warps 0-3: sparse-entry scatter
-constexpr int kLoaderWarp = 4;       // TMA issue, chunks g = 0 (mod kLoaders)
-constexpr int kMmaWarp = 5;          // TMEM allocation, tcgen05.mma issue
-constexpr int kEpiThreads = 128;     // warps 6-9: epilogue
-constexpr int kLoaderWarp1 = 10;     // warps 10..: TMA issue, chunks g = 1, 2, .. (mod kLoaders)
-constexpr int kLoaders = 4;          // loader warps, each issuing every kLoaders-th chunk
-constexpr int kThreads = 320 + (kLoaders - 1) * 32;
+constexpr int kBLoaderWarp = 0;  // TMA issue of the B rows
+constexpr int kALoaderWarp = 1;  // TMA issue of the A images and entries
+constexpr int kMmaWarp = 2;      // TMEM allocation, tcgen05.mma issue
+constexpr int kScatterWarp0 = 3; // warps 3-6: sparse-entry scatter
+constexpr int kScatterWarps = 4;
+constexpr int kEpiWarp0 = 7;     // warps 7-10: epilogue
+constexpr int kEpiThreads = 128;
+constexpr int kThreads = 352;
+constexpr int kAhead = 4;        // chunks by which the entries of a sparse chunk precede its stage
+constexpr int kRecords = 64;     // chunk records kept: two batches of 32
 constexpr int kMaxCtaItems = 32;      // work items per persistent CTA
-constexpr int kEpiBar = 3;           // named barrier of the epilogue warps (1, 2: scatter groups)
-constexpr int kEpiWarp0 = 6;         // first epilogue warp
+constexpr int kEpiBar = 3;           // named barrier of the epilogue warps
+constexpr int kScatterBar = 1;       // named barrier of the scatter warps
 constexpr int kStagingBytes = ((kImageMinNnz + 3) * 4 + 15) & ~15; // entries of a sparse chunk, 16-byte rounded
 constexpr int kMaxJobs = 32;                                  // jobs per launch (kernel parameter space)
 
 struct TcJob {
     CUtensorMap tmap_b;    // B as a 2-D tensor {N, K}, box {64, 1}, 128-byte swizzle (gather4 source)
-    CUtensorMap tmap_tile; // the same tensor, box {64, 64}: 64 contiguous rows of B per instruction
+    CUtensorMap tmap_tile; // 64 contiguous rows of B: the same tensor, box {64, 64}, or (tile3d) {64, K, N / 64}, box {64, 64, NT / 64}
     const int4 *win_info; // per tensor-core window: window, first chunk, chunk count
     const int2 *pairs;    // pair kernel: tensor-core window pairs (second -1: alone)
     const int *tile_ptr, *win_cols, *img_idx, *perm, *p_row_ptr;
@@ -73,6 +83,7 @@ struct TcJob {
     void *C;
     int *status;
     int M, N, ldb, ldc, ntiles;
+    int tile3d;              // tmap_tile covers the whole NT-wide slice in one box
     float alpha, beta;
     unsigned flags;
 };
@@ -148,30 +159,31 @@ __device__ __forceinline__ void store8_out(float *p, const float *v, float alpha
 }
 
 // Shared memory (1024-byte aligned base): kStages x (A tile | B tile),
-// kStages entry staging buffers, per-stage chunk records, the CTA's item
-// table, mbarriers, four broadcast flags and the TMEM slot.
+// kSlots entry staging buffers, the chunk records of both loaders, the CTA's item table,
+// mbarriers and the TMEM slot.
 // F8: E4M3 operands -- an 8 KB A tile (64-byte swizzled K-major) and 64 x NT
 // byte B tiles, so the ring holds more stages.
 template <int NT, bool F8> struct TcCfg {
     static constexpr int kElem = F8 ? 1 : 2;
     static constexpr int kATileBytes = kWindowRows * kChunkCols * kElem;
     static constexpr int kBoxCols = 128 / kElem; // N columns per 128-byte swizzle atom / TMA box
-    static constexpr int kStages = F8 ? (NT == 256 ? 8 : 12) : (NT == 256 ? 4 : NT == 128 ? 6 : 8);
+    static constexpr int kStages = F8 ? (NT == 256 ? 8 : 11) : (NT == 256 ? 4 : NT == 128 ? 6 : 8);
     static constexpr int kBTileBytes = kChunkCols * NT * kElem;
     static constexpr int kStage = kATileBytes + kBTileBytes;
     static constexpr int kStagingOff = kStages * kStage;
-    static constexpr int kPendOff = kStagingOff + kStages * kStagingBytes; // int4 [kStages]: img, e0, e0a, e1
-    static constexpr int kPend2Off = kPendOff + kStages * 16;              // int4 [kStages]: flags, buffer, item
-    static constexpr int kItemOff = kPend2Off + kStages * 16;              // int4 [kMaxCtaItems]
-    static constexpr int kScaleOff = kItemOff + kMaxCtaItems * 16;         // E4M3: float [2][NT] column scales
+    static constexpr int kSlots = kStages + kAhead;                       // entry staging slots (see the scatter role)
+    static constexpr int kRecOff = kStagingOff + kSlots * kStagingBytes;  // TcRecordA, TcRecordB [kRecords]
+    static constexpr int kItemOff = kRecOff + kRecords * 32;              // int4 [kMaxCtaItems]
+    static constexpr int kPendOff = kItemOff + kMaxCtaItems * 16;         // int2 [kSlots]: stage, entries
+    static constexpr int kCumOff = kPendOff + kSlots * 8;                 // int [kMaxCtaItems + 4]: first chunk of each item
+    static constexpr int kScaleOff = kCumOff + (kMaxCtaItems + 4) * 4;    // E4M3: float [2][NT] column scales
     static constexpr int kBarOff = kScaleOff + (F8 ? 2 * NT * 4 : 0);
-    // full, empty, staged [kStages]; accum_full, accum_empty [2]; drain; 4 flags, TMEM slot
-    static constexpr int kSmem = kBarOff + (3 * kStages + 5) * 8 + 24;
+    // full, empty [kStages]; staged [kSlots]; accum_full, accum_empty [2]; drain; TMEM slot
+    static constexpr int kSmem = kBarOff + (2 * kStages + kSlots + 5) * 8 + 8;
     static_assert(kSmem <= 227 * 1024, "shared memory budget");
     static_assert(kStage % 1024 == 0 && kATileBytes % 1024 == 0, "swizzled tiles need 1024-byte alignment");
     static_assert(kStagingOff % 16 == 0 && kStagingBytes % 16 == 0 && kPendOff % 16 == 0, "16-byte alignment");
-    static_assert(kItemOff % 16 == 0 && kBarOff % 16 == 0, "16-byte aligned regions");
-    static_assert(kLoaders <= kStages, "a loader may not lap a stage that an earlier loader still fills");
+    static_assert(kRecOff % 16 == 0 && kItemOff % 16 == 0 && kBarOff % 8 == 0, "aligned regions");
 };
 
 // Work item (job, tensor-core window, N slice) -> table entry {window,
@@ -187,37 +199,126 @@ __device__ __forceinline__ int4 decode_item(const Batch &batch, int item)
     return make_int4(wi.x, wi.y, wi.z, (j << 16) | (local % a.ntiles));
 }
 
+// A chunk as the two loaders issue it (16 bytes of shared memory each).
+struct __align__(16) TcRecordA {
+    const void *src; // dense image or (16-byte aligned) first entry
+    int bytes;       // of src: kATileBytes for an image, fewer for entries
+    int ent;         // entries: count << 2 | entries before the first one
+};
+struct __align__(16) TcRecordB {
+    const void *b; // tensor map; condensed columns: the column list
+    int col0;      // first of 64 consecutive columns; condensed columns: -1 - item
+    int x;         // n0 (2-D boxes) or, with the top bit, the 64-column slab of n0 (3-D box)
+};
+
+// 16-byte unit u of an output row: alpha x 8 accumulators as FP16, or 4 as FP32.
+template <typename OutT> __device__ __forceinline__ uint4 pack_unit(const float *v, float alpha)
+{
+    uint4 u;
+    if constexpr (sizeof(OutT) == 2) {
+        __half2 *h = reinterpret_cast<__half2 *>(&u);
+#pragma unroll
+        for (int i = 0; i < 4; i++) h[i] = __floats2half2_rn(alpha * v[2 * i], alpha * v[2 * i + 1]);
+    } else {
+        u = make_uint4(__float_as_uint(alpha * v[0]), __float_as_uint(alpha * v[1]), __float_as_uint(alpha * v[2]),
+                       __float_as_uint(alpha * v[3]));
+    }
+    return u;
+}
+
+// The warp's 32 accumulator rows (lane = row, its row of C in out_row, -1:
+// none) times alpha, NT columns from n0 on, for beta = 0. Tensor memory gives
+// a lane its own row, but 32 lanes storing 16 bytes to 32 rows touch 32 lines
+// per instruction (measured: 3.5 us for a 128 x 256 FP16 tile). So groups of
+// four lanes transpose four 16-byte units among themselves by shuffles, and an
+// instruction stores 64 consecutive bytes of each of 8 rows.
+template <int NT, typename OutT, bool F8>
+__device__ __forceinline__ void store_rows(uint32_t acc, OutT *C, int ldc, int out_row, int n0, int N, float alpha,
+                                           float sa, const float *sb, int lane)
+{
+    constexpr int kUnit = 16 / (int)sizeof(OutT); // columns per unit
+    const int i = lane & 3;
+    int rows[4]; // rows of C that this lane stores to: those of its group
+#pragma unroll
+    for (int u = 0; u < 4; u++) rows[u] = __shfl_sync(0xffffffffu, out_row, (lane & ~3) + u);
+    for (int cb = 0; cb < NT / 32; cb++) {
+        if (n0 + cb * 32 >= N)
+            break; // uniform across the warp
+        uint32_t r[32];
+        tmem_ld32(acc + (uint32_t)(cb * 32), r);
+        float *f = reinterpret_cast<float *>(r);
+        if constexpr (F8) { // dequantise: row scale x column scale
+#pragma unroll
+            for (int q = 0; q < 32; q++) f[q] *= sa * sb[cb * 32 + q];
+        }
+#pragma unroll
+        for (int h = 0; h < 32 / (4 * kUnit); h++) {
+            uint4 v[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) v[u] = pack_unit<OutT>(f + (h * 4 + u) * kUnit, alpha);
+            // 4 x 4 transpose: afterwards v[u] is unit i of the group's row u
+#pragma unroll
+            for (int m = 1; m < 4; m <<= 1) {
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    if (u & m)
+                        continue;
+                    const bool hi = (lane & m) != 0;
+                    uint4 x = hi ? v[u] : v[u | m];
+                    x.x = __shfl_xor_sync(0xffffffffu, x.x, m);
+                    x.y = __shfl_xor_sync(0xffffffffu, x.y, m);
+                    x.z = __shfl_xor_sync(0xffffffffu, x.z, m);
+                    x.w = __shfl_xor_sync(0xffffffffu, x.w, m);
+                    if (hi) v[u] = x;
+                    else v[u | m] = x;
+                }
+            }
+            const int n = n0 + cb * 32 + (h * 4 + i) * kUnit;
+            if (n < N) {
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+                    if (rows[u] >= 0)
+                        *reinterpret_cast<uint4 *>(C + (size_t)rows[u] * ldc + n) = v[u];
+            }
+        }
+    }
+}
+
 // Persistent CTAs, one per SM: CTA b processes work items b, b + gridDim.x,
 // ... (at most kMaxCtaItems), as one continuous stream of total_chunks chunks
 // through the stage ring; every role runs over exactly those chunks. Roles
 // (kThreads threads):
-//   warps 4, 10, 11, 12 (loaders; loader l takes chunks g = l (mod kLoaders),
-//     so that four chunks are being issued at once -- one warp issuing every
-//     chunk in turn was measured to need ~0.9 us per chunk, three times the
-//     tensor-core time of an N = 256 chunk): per chunk, acquire the stage
-//     ("empty"), write the chunk's records (entries range and image for the
-//     scatter warps; first / last chunk of its item and accumulator buffer for
-//     the MMA lane), set the "full" transaction count and issue the dense A
-//     image (cp.async.bulk) or the sparse entries (cp.async.bulk into staging,
-//     completing on "staged"), then the B rows: tiled TMA boxes of 64
-//     contiguous rows for direct chunks, tile::gather4 for condensed ones.
-//     Chunk metadata (columns, image, entry range) is loaded into registers
-//     one chunk of the same loader ahead.
-//   warps 0-3 (scatter; two groups of two warps taking chunks in turn when
-//     the ring has an even number of stages, else one group of four): per
-//     chunk, wait "staged"; for a sparse chunk zero the A tile, scatter the
-//     staged entries, fence.proxy.async; arrive "full". With two groups, a
-//     group's previous use of a stage is its own (stage count even), so no
-//     group waits on a phase more than one ahead of an mbarrier.
-//   warp 5, lane 0 (MMA): per chunk wait "full"; on an item's first chunk
+//   warps 0 and 1 (loaders of B and of A): a TMA instruction takes its issuer
+//     about 0.1 us (a %clock trace), so each chunk's two go out from two
+//     warps. The chunk records -- tensor map and coordinates; image or entry
+//     range -- are made 32 at a time, one per lane, from loads issued 32
+//     chunks ahead, and kept in shared memory, so that one elected lane can
+//     walk the chunks alone: acquire the stage ("empty"), set its part of the
+//     "full" transaction count and issue. B: ONE 3-D box of 64 rows x NT
+//     columns for a direct chunk (64-column slabs as the third dimension; 2-D
+//     boxes of one slab each when N is not whole slabs), tile::gather4 for
+//     condensed ones (by all lanes). A: the dense image (cp.async.bulk), or
+//     the release of a sparse chunk to the scatter warps ("staged"), whose
+//     entries were sent for kAhead chunks before (cp.async.bulk into a
+//     staging slot, completing on its "staged").
+//   warp 2, one lane (MMA): per chunk wait "full"; on an item's first chunk
 //     wait until its TMEM accumulator buffer (item parity) is drained
 //     ("accum_empty"); 4 x tcgen05.mma (2 for E4M3); commit "empty"; on the
 //     item's last chunk commit "accum_full".
-//   warps 6-9 (epilogue): per item wait "accum_full", tcgen05.ld the rows
+//   warps 3-6 (scatter): per sparse chunk, once its entries are in and its
+//     stage is free ("staged"): zero the A tile, write the entries into the
+//     swizzled layout, arrive on "full" -- while the chunk's B rows are still
+//     on their way; image chunks pass them by. Sparse chunk q uses slot
+//     q % kSlots; it is filled when chunk g is issued, at most kAhead chunks
+//     before its own, so sparse chunk q - kSlots lies at least kStages chunks
+//     before g and is consumed.
+//   warps 7-10 (epilogue): per item wait "accum_full", tcgen05.ld the rows
 //     (warp w reads TMEM lanes 32 (w % 4) ..), alpha/beta, store to C[perm],
 //     arrive "accum_empty" -- overlapping the next item's main loop.
+// 64 registers a thread: two blocks of the CUDA-core kernel then fit beside
+// this one on an SM.
 template <int NT, typename OutT, bool F8, int CAP = kMaxJobs>
-__global__ void __launch_bounds__(kThreads, 1) spmm_tc_kernel(const __grid_constant__ TcBatchT<CAP> batch)
+__global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<CAP> batch)
 {
     using Cfg = TcCfg<NT, F8>;
     constexpr int S = Cfg::kStages;
@@ -225,26 +326,25 @@ __global__ void __launch_bounds__(kThreads, 1) spmm_tc_kernel(const __grid_const
     constexpr int kBoxes = NT / Cfg::kBoxCols; // 128-byte-wide boxes per B row slice
     constexpr int kGathers = 16 * kBoxes;      // gather4 instructions per condensed chunk
     extern __shared__ __align__(1024) uint8_t smem[];
-    int4 *pend = reinterpret_cast<int4 *>(smem + Cfg::kPendOff);
-    int4 *pend2 = reinterpret_cast<int4 *>(smem + Cfg::kPend2Off);
+    int2 *pend = reinterpret_cast<int2 *>(smem + Cfg::kPendOff);
+    TcRecordA *rec_a = reinterpret_cast<TcRecordA *>(smem + Cfg::kRecOff);
+    TcRecordB *rec_b = reinterpret_cast<TcRecordB *>(rec_a + kRecords);
     int4 *items = reinterpret_cast<int4 *>(smem + Cfg::kItemOff);
+    int *cum = reinterpret_cast<int *>(smem + Cfg::kCumOff);
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + Cfg::kBarOff);
     uint64_t *empty = full + S;
-    uint64_t *staged = empty + S;
-    uint64_t *acc_full = staged + S;  // [2]
-    uint64_t *acc_empty = acc_full + 2; // [2]
-    uint64_t *drain = acc_empty + 2;    // the MMA lane's last commit: every MMA it issued has completed
-    volatile int *flag = reinterpret_cast<volatile int *>(drain + 1); // 2 slots per scatter group
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(drain + 1) + 4;
-    constexpr int kScatterGroups = S % 2 == 0 ? 2 : 1; // two groups need an even ring (see the scatter role)
-    constexpr int kGroupThreads = kScatterThreads / kScatterGroups;
+    uint64_t *staged = empty + S;               // [kSlots]
+    uint64_t *acc_full = staged + Cfg::kSlots; // [2]
+    uint64_t *acc_empty = acc_full + 2;         // [2]
+    uint64_t *drain = acc_empty + 2;            // the MMA lane's last commit: every MMA it issued has completed
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(drain + 1);
 
     // A CUDA-core launch that follows on the stream as a programmatic
     // dependent may start as soon as every block of this grid is resident: it
     // reads nothing this kernel writes (the two paths own disjoint rows of C).
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int total = batch.item_start[batch.n_jobs];
     const int n_items = blockIdx.x < total ? min(kMaxCtaItems, (total - 1 - (int)blockIdx.x) / (int)gridDim.x + 1) : 0;
     if (smem_u32(smem) & 1023u) { // the swizzled tiles and TMA destinations need a 1024-byte aligned base
@@ -252,12 +352,65 @@ __global__ void __launch_bounds__(kThreads, 1) spmm_tc_kernel(const __grid_const
             atomicOr(batch.job[0].status, kStatusLayout);
         return;
     }
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < S; s++) {
-            mbar_init(&full[s], kGroupThreads);
-            mbar_init(&empty[s], 1);
-            mbar_init(&staged[s], 1);
+    // chunk g of the stream: its item (found from `k` on) and its place in the plan
+    auto locate = [&](int g, int &k) -> int {
+        while (k + 1 < n_items && cum[k + 1] <= g) k++;
+        const int4 it = items[k];
+        // windows of one problem start their chunk walks at different
+        // chunks, so that they do not read the same rows of B at once
+        int i = g - cum[k] + it.x % it.z;
+        if (i >= it.z) i -= it.z;
+        return it.y + i;
+    };
+    // a loader's chunk metadata from the plan, one chunk per lane: the columns
+    // of its ends (B), or its image and entry range (A)
+    int k = 0, c = 0, m0 = 0, m1 = 0, img = -1;
+    auto fetch = [&](int g, int k0) {
+        k = k0;
+        if (g < cum[n_items]) {
+            c = locate(g, k);
+            const TcJob &a = batch.job[items[k].w >> 16];
+            if (warp == kBLoaderWarp) {
+                m0 = __ldg(a.win_cols + (size_t)c * kChunkCols);
+                m1 = __ldg(a.win_cols + (size_t)c * kChunkCols + kChunkCols - 1);
+            } else {
+                img = __ldg(a.img_idx + c);
+                m0 = __ldg(a.tile_ptr + c);
+                m1 = __ldg(a.tile_ptr + c + 1);
+            }
         }
+    };
+    if (warp == kBLoaderWarp) {
+        // the item table and the first chunk of each item (a warp scan of the chunk counts)
+        int z = 0;
+        if (lane < n_items) {
+            const int4 it = decode_item(batch, blockIdx.x + lane * gridDim.x);
+            items[lane] = it;
+            z = it.z;
+        }
+        int sum = z;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, sum, o);
+            if (lane >= o) sum += v;
+        }
+        cum[lane + 1] = sum;
+        if (lane == 0) cum[0] = 0;
+        __syncwarp();
+        fetch(lane, 0); // the first records' loads, on their way during the rest of the set-up
+        if (lane < n_items)
+            prefetch_tensormap(&batch.job[items[lane].w >> 16].tmap_tile);
+    } else if (warp == kMmaWarp) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                     "r"(2 * NT)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    } else if (warp == kScatterWarp0 && lane == 0) {
+        for (int s = 0; s < S; s++) {
+            mbar_init(&full[s], 2); // both loaders' parts (of a sparse chunk: the scatter warps')
+            mbar_init(&empty[s], 1);
+        }
+        for (int s = 0; s < Cfg::kSlots; s++) mbar_init(&staged[s], 1);
         for (int b = 0; b < 2; b++) {
             mbar_init(&acc_full[b], 1);
             mbar_init(&acc_empty[b], kEpiThreads);
@@ -265,190 +418,210 @@ __global__ void __launch_bounds__(kThreads, 1) spmm_tc_kernel(const __grid_const
         mbar_init(drain, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if ((int)threadIdx.x < n_items)
-        items[threadIdx.x] = decode_item(batch, blockIdx.x + threadIdx.x * gridDim.x);
-    if (warp == kMmaWarp) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                     "r"(2 * NT)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     bool ok = true;
-    int total_chunks = 0; // of this CTA's items: every role runs over exactly these
-    for (int k = 0; k < n_items; k++) total_chunks += items[k].z;
+    const int total_chunks = cum[n_items]; // of this CTA's items: every role runs over exactly these
 
-    if (warp == kLoaderWarp || warp >= kLoaderWarp1) {
-        // ---------------- loaders ----------------
-        // Loader ld issues chunks g = ld, ld + kLoaders, ... of the CTA's chunk
-        // stream; (k, i) is the item and chunk-within-item of its next chunk.
-        const int ld = warp == kLoaderWarp ? 0 : warp - kLoaderWarp1 + 1;
-        auto advance = [&](int &k, int &i) {
-            while (k < n_items && i >= items[k].z) { i -= items[k].z; k++; }
-        };
-        // per-chunk metadata in registers: lanes 0-15 hold 4 columns each, every
-        // lane the image index and entry range; fetched one chunk of this loader ahead
-        struct Meta { int4 cols; int img, e0, e1; };
-        auto fetch = [&](int k, int i, Meta &m) {
-            m.cols = make_int4(-1, -1, -1, -1);
-            m.img = -1;
-            m.e0 = m.e1 = 0;
-            if (k < n_items) {
+    if (warp == kBLoaderWarp) {
+        // ---------------- loader of B ----------------
+        // records of chunks g0 .. g0 + 31 (fetched), and the loads of the next 32
+        auto make_records = [&](int g0) {
+            if (g0 + lane < total_chunks) {
                 const int4 it = items[k];
                 const TcJob &a = batch.job[it.w >> 16];
-                // windows of one problem start their chunk walks at different
-                // chunks, so that they do not read the same rows of B at once
-                const int c = it.y + (i + it.x % it.z) % it.z;
-                if (lane < 16)
-                    m.cols = __ldg(reinterpret_cast<const int4 *>(a.win_cols + (size_t)c * kChunkCols) + lane);
-                m.img = __ldg(a.img_idx + c);
-                m.e0 = __ldg(a.tile_ptr + c);
-                m.e1 = __ldg(a.tile_ptr + c + 1);
+                TcRecordB r;
+                const int n0 = (it.w & 0xffff) * NT;
+                const bool direct = m0 >= 0 && m1 == m0 + kChunkCols - 1;
+                r.b = direct ? (const void *)&a.tmap_tile : (const void *)(a.win_cols + (size_t)c * kChunkCols);
+                r.col0 = direct ? m0 : -1 - k;
+                r.x = a.tile3d ? (int)0x80000000 | (n0 / Cfg::kBoxCols) : n0;
+                rec_b[(g0 + lane) % kRecords] = r;
             }
+            fetch(g0 + 32 + lane, __shfl_sync(0xffffffffu, k, 31));
+            __syncwarp();
         };
-        int k = 0, i = ld;
-        advance(k, i);
-        int g = ld;
-        // One chunk: prefetch the metadata of this loader's next chunk into
-        // `nxt`, acquire the stage, issue the chunk described by `cur`. The
-        // loop below alternates the roles of two Meta variables (unrolled by
-        // two), so that no register copy waits for a prefetch still in flight.
-        auto step = [&](Meta &cur, Meta &nxt) -> bool {
-            if (g >= total_chunks || !ok)
-                return false;
-            int k2 = k, i2 = i + kLoaders;
-            advance(k2, i2);
-            fetch(k2, i2, nxt);
-            const int s = g % S;
-            uint32_t got = 1;
-            if (lane == 0 && g >= S)
-                got = mbar_wait(&empty[s], ((g / S) - 1) & 1) ? 1u : 0u;
-            got = __shfl_sync(0xffffffffu, got, 0);
-            if (!got) { ok = false; return false; }
-            const int4 it = items[k];
-            const TcJob &a = batch.job[it.w >> 16];
-            const int n0 = (it.w & 0xffff) * NT;
-            const uint32_t a_s = smem_u32(smem + s * Cfg::kStage), b_s = a_s + kATileBytes;
-            if (lane == 0) {
-                const int img = cur.img, e0 = cur.e0, e1 = cur.e1, e0a = e0 & ~3;
-                pend[s] = make_int4(img, e0, e0a, e1);
-                pend2[s] = make_int4((i == 0 ? 1 : 0) | (i == it.z - 1 ? 2 : 0), k & 1, k, 0);
-                mbar_expect_tx(&full[s], Cfg::kBTileBytes + (img >= 0 ? kATileBytes : 0));
-                if (img >= 0) {
-                    bulk_copy_g2s(a_s, a.images + (size_t)img * kATileBytes, kATileBytes, &full[s]);
-                    mbar_arrive(&staged[s]);
-                } else if (e1 > e0) {
-                    const uint32_t bytes = (uint32_t)(((e1 - e0a) * 4 + 15) & ~15);
-                    mbar_arrive_expect_tx(&staged[s], bytes);
-                    bulk_copy_g2s(smem_u32(smem + Cfg::kStagingOff + s * kStagingBytes), a.entries + e0a, bytes,
-                                  &staged[s]);
-                } else {
-                    mbar_arrive(&staged[s]);
-                }
-            }
-            __syncwarp(); // the transaction count is set before any B load is issued
-            const int col0 = __shfl_sync(0xffffffffu, cur.cols.x, 0);
-            const int col63 = __shfl_sync(0xffffffffu, cur.cols.w, 15);
-            if (col0 >= 0 && col63 == col0 + kChunkCols - 1) {
-                // 64 contiguous B rows (direct chunks): one 8 KB tiled box per 128-byte column slab
-                if (lane < kBoxes)
-                    tma_tile2d(b_s + lane * (kChunkCols * 128), &a.tmap_tile, n0 + lane * Cfg::kBoxCols, col0,
-                               &full[s]);
+        // a direct chunk's B rows into stage s
+        auto issue_boxes = [&](const TcRecordB &r, int s) {
+            const uint32_t b_s = smem_u32(smem + s * Cfg::kStage) + kATileBytes;
+            const CUtensorMap *map = static_cast<const CUtensorMap *>(r.b);
+            if (r.x < 0) {
+                tma_tile3d(b_s, map, 0, r.col0, r.x & 0x7fffffff, &full[s]);
             } else {
-                // condensed columns: gather q = lane, lane + 32, .. reads the 4 columns of lane q % 16
-                const int src = lane & 15;
-                const int y0 = __shfl_sync(0xffffffffu, cur.cols.x, src);
-                const int y1 = __shfl_sync(0xffffffffu, cur.cols.y, src);
-                const int y2 = __shfl_sync(0xffffffffu, cur.cols.z, src);
-                const int y3 = __shfl_sync(0xffffffffu, cur.cols.w, src);
-                for (int q = lane; q < kGathers; q += 32) {
-                    const int box = q >> 4;
-                    tma_gather4(b_s + box * (kChunkCols * 128) + src * 512, &a.tmap_b, n0 + box * Cfg::kBoxCols, y0,
-                                y1, y2, y3, &full[s]);
-                }
-            }
-            k = k2;
-            i = i2;
-            g += kLoaders;
-            return true;
-        };
-        Meta ma, mb;
-        fetch(k, i, ma);
-        while (step(ma, mb) && step(mb, ma)) {
-        }
-    } else if (warp < 4) {
-        // ---------------- scatter ----------------
-        // kScatterGroups groups of warps take the chunks in turn (group q:
-        // chunks g = q (mod kScatterGroups)), so that the scatter of one sparse
-        // chunk overlaps the next one's.
-        const int grp = kScatterGroups == 2 ? (warp >> 1) : 0;
-        const int sid = (int)threadIdx.x - grp * kGroupThreads;
-        int it = 0;
-        for (int g = grp; g < total_chunks; g += kScatterGroups, it++) {
-            const int s = g % S;
-            volatile int *fl = flag + grp * 2 + (it & 1);
-            if (sid == 0)
-                *fl = mbar_wait(&staged[s], (g / S) & 1) ? 1 : 0;
-            named_bar_sync(1 + grp, kGroupThreads); // also orders the staged data for every thread of the group
-            if (*fl == 0) { ok = false; break; } // uniform across the group
-            const int4 pd = pend[s];
-            if (pd.x == -1) {
-                uint8_t *At = smem + s * Cfg::kStage;
 #pragma unroll
-                for (int q = 0; q < kATileBytes / (16 * kGroupThreads); q++)
-                    reinterpret_cast<uint4 *>(At)[sid + q * kGroupThreads] = make_uint4(0, 0, 0, 0);
-                named_bar_sync(1 + grp, kGroupThreads);
-                const uint32_t *st = reinterpret_cast<const uint32_t *>(smem + Cfg::kStagingOff + s * kStagingBytes);
-                for (int e = pd.y + sid; e < pd.w; e += kGroupThreads) {
-                    const uint32_t v = st[e - pd.z];
-                    if constexpr (F8)
-                        At[swz64_offset(v >> 22, (v >> 16) & 63u)] = (uint8_t)(v & 0xffu);
-                    else
-                        *reinterpret_cast<uint16_t *>(At + swz128_offset(v >> 22, (v >> 16) & 63u)) =
-                            (uint16_t)(v & 0xffffu);
-                }
-                fence_proxy_async();
+                for (int bx = 0; bx < kBoxes; bx++)
+                    tma_tile2d(b_s + bx * (kChunkCols * 128), map, r.x + bx * Cfg::kBoxCols, r.col0, &full[s]);
             }
-            mbar_arrive(&full[s]);
+        };
+        int s = 0;
+        uint32_t phase = 1; // of "empty": the first pass over the ring finds every stage free
+        for (int g = 0; g < total_chunks;) {
+            make_records(g);
+            const int ge = min(total_chunks, g + 32);
+            int s1 = s;
+            uint32_t phase1 = phase;
+            if (__all_sync(0xffffffffu, g + lane >= ge || rec_b[(g + lane) % kRecords].col0 >= 0)) {
+                // direct chunks only: one lane alone
+                if (elect_one()) {
+                    TcRecordB r = rec_b[g % kRecords];
+                    for (int h = g; h < ge; h++) {
+                        const TcRecordB nxt = rec_b[(h + 1) % kRecords];
+                        if (!mbar_wait(&empty[s1], phase1)) { ok = false; break; }
+                        mbar_arrive_expect_tx(&full[s1], Cfg::kBTileBytes);
+                        issue_boxes(r, s1);
+                        if (++s1 == S) { s1 = 0; phase1 ^= 1; }
+                        r = nxt;
+                    }
+                }
+            } else {
+                int4 ncols = make_int4(-1, -1, -1, -1); // columns of the next chunk, when it is a condensed one
+                auto fetch_cols = [&](const TcRecordB &r) {
+                    if (r.col0 < 0 && lane < 16)
+                        ncols = __ldg(reinterpret_cast<const int4 *>(r.b) + lane);
+                };
+                fetch_cols(rec_b[g % kRecords]);
+                for (int h = g; h < ge; h++) {
+                    const TcRecordB r = rec_b[h % kRecords];
+                    if (elect_one()) {
+                        ok = mbar_wait(&empty[s1], phase1);
+                        if (ok) {
+                            mbar_arrive_expect_tx(&full[s1], Cfg::kBTileBytes);
+                            if (r.col0 >= 0)
+                                issue_boxes(r, s1);
+                        }
+                    }
+                    if (__any_sync(0xffffffffu, !ok)) break; // also: the transaction count is set
+                    if (r.col0 < 0) {
+                        // condensed columns: gather p = lane, lane + 32, .. reads the 4 columns of lane p % 16
+                        const int4 it = items[-1 - r.col0];
+                        const TcJob &a = batch.job[it.w >> 16];
+                        const uint32_t b_s = smem_u32(smem + s1 * Cfg::kStage) + kATileBytes;
+                        const int src = lane & 15, n0 = (it.w & 0xffff) * NT;
+                        const int y0 = __shfl_sync(0xffffffffu, ncols.x, src);
+                        const int y1 = __shfl_sync(0xffffffffu, ncols.y, src);
+                        const int y2 = __shfl_sync(0xffffffffu, ncols.z, src);
+                        const int y3 = __shfl_sync(0xffffffffu, ncols.w, src);
+                        for (int p = lane; p < kGathers; p += 32) {
+                            const int bx = p >> 4;
+                            tma_gather4(b_s + bx * (kChunkCols * 128) + src * 512, &a.tmap_b, n0 + bx * Cfg::kBoxCols,
+                                        y0, y1, y2, y3, &full[s1]);
+                        }
+                    }
+                    if (h + 1 < ge)
+                        fetch_cols(rec_b[(h + 1) % kRecords]);
+                    if (++s1 == S) { s1 = 0; phase1 ^= 1; }
+                }
+            }
+            if (__any_sync(0xffffffffu, !ok)) { ok = false; break; }
+            // the ring's place after this run of chunks (the elected lane may have walked it alone)
+            phase ^= (uint32_t)((s + ge - g) / S) & 1u;
+            s = (s + ge - g) % S;
+            g = ge;
+        }
+    } else if (warp == kALoaderWarp) {
+        // ---------------- loader of A ----------------
+        auto make_records = [&](int g0) {
+            if (g0 + lane < total_chunks) {
+                const TcJob &a = batch.job[items[k].w >> 16];
+                TcRecordA r;
+                r.src = img >= 0 ? (const void *)(a.images + (size_t)img * kATileBytes)
+                                 : (const void *)(a.entries + (m0 & ~3));
+                r.bytes = img >= 0 ? kATileBytes : m1 > m0 ? ((m1 - (m0 & ~3)) * 4 + 15) & ~15 : 0;
+                r.ent = ((m1 - m0) << 2) | (m0 & 3);
+                rec_a[(g0 + lane) % kRecords] = r;
+            }
+            fetch(g0 + 32 + lane, __shfl_sync(0xffffffffu, k, 31));
+            __syncwarp();
+        };
+        // send for the entries of chunk h if it is a sparse one
+        int pslot = 0, slot = 0, s = 0;
+        uint32_t phase = 1;
+        auto prefetch = [&](int h) {
+            if (h < total_chunks) {
+                const TcRecordA r = rec_a[h % kRecords];
+                if (r.bytes != kATileBytes) {
+                    if (r.bytes) {
+                        mbar_expect_tx(&staged[pslot], (uint32_t)r.bytes);
+                        bulk_copy_g2s(smem_u32(smem + Cfg::kStagingOff + pslot * kStagingBytes), r.src,
+                                      (uint32_t)r.bytes, &staged[pslot]);
+                    }
+                    if (++pslot == Cfg::kSlots) pslot = 0;
+                }
+            }
+        };
+        fetch(lane, 0);
+        make_records(0);
+        // one lane walks the chunks; every lane joins it to make the next records
+        const bool leader = elect_one();
+        if (leader)
+            for (int h = 0; h < kAhead; h++) prefetch(h);
+        for (int g = 0; g < total_chunks;) {
+            if (g > 0)
+                make_records(g + kAhead); // g + kAhead is a multiple of 32 here
+            const int ge = min(total_chunks, (g + kAhead) / 32 * 32 + 32 - kAhead);
+            if (leader) {
+                TcRecordA r = rec_a[g % kRecords];
+                for (int h = g; h < ge; h++) {
+                    const TcRecordA nxt = rec_a[(h + 1) % kRecords];
+                    if (!mbar_wait(&empty[s], phase)) { ok = false; break; }
+                    if (r.bytes == kATileBytes) {
+                        mbar_arrive_expect_tx(&full[s], kATileBytes);
+                        bulk_copy_g2s(smem_u32(smem + s * Cfg::kStage), r.src, kATileBytes, &full[s]);
+                    } else {
+                        pend[slot] = make_int2(s, r.ent);
+                        mbar_arrive(&staged[slot]); // the scatter warps arrive on "full"
+                        if (++slot == Cfg::kSlots) slot = 0;
+                    }
+                    prefetch(h + kAhead);
+                    if (++s == S) { s = 0; phase ^= 1; }
+                    r = nxt;
+                }
+            }
+            if (__any_sync(0xffffffffu, !ok)) { ok = false; break; }
+            g = ge;
         }
     } else if (warp == kMmaWarp) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc = idesc_f16(NT); // E4M3 has format code 0 in kind::f8f6f4 as FP16 in kind::f16
             // test hook: the CTA's last accumulator is never announced, so the
             // epilogue's bounded wait for it runs out (TCA_FLAG_TEST_WITHHOLD_ACCUM)
             const bool withhold = (batch.job[0].flags & TCA_FLAG_TEST_WITHHOLD_ACCUM) != 0;
-            for (int g = 0; g < total_chunks; g++) {
-                const int s = g % S;
-                if (!mbar_wait(&full[s], (g / S) & 1)) { ok = false; break; }
-                const int4 f = pend2[s];
-                const int b = f.y, k = f.z;
-                if ((f.x & 1) && k >= 2 && !mbar_wait(&acc_empty[b], ((k >> 1) - 1) & 1)) { ok = false; break; }
-                tc_fence_after();
-                const uint32_t a_s = smem_u32(smem + s * Cfg::kStage), b_s = a_s + kATileBytes;
+            int s = 0;
+            uint32_t phase = 0;
+            for (int k = 0; k < n_items && ok; k++) {
+                const int b = k & 1;
                 const uint32_t d = tmem + (uint32_t)(b * NT);
-                if constexpr (F8) {
-                    // 2 x K = 32: A rows of 64 bytes (64-byte swizzle, 8-row groups 512 bytes apart),
-                    // B k-rows of 128 bytes (128-byte swizzle, atoms along N 8 KB apart)
+                if (k >= 2 && !mbar_wait(&acc_empty[b], ((k >> 1) - 1) & 1)) { ok = false; break; }
+                uint32_t accum = 0;
+                for (int i = items[k].z; i > 0; i--) {
+                    if (!mbar_wait(&full[s], phase)) { ok = false; break; }
+                    tc_fence_after();
+                    const uint32_t a_s = smem_u32(smem + s * Cfg::kStage), b_s = a_s + kATileBytes;
+                    if constexpr (F8) {
+                        // 2 x K = 32: A rows of 64 bytes (64-byte swizzle, 8-row groups 512 bytes apart),
+                        // B k-rows of 128 bytes (128-byte swizzle, atoms along N 8 KB apart)
 #pragma unroll
-                    for (int kk = 0; kk < kChunkCols / 32; kk++) {
-                        const uint64_t ad = smem_desc(a_s + kk * 32, 16, 512, 4);
-                        const uint64_t bd = smem_desc(b_s + kk * 4096, kChunkCols * 128, 1024);
-                        umma_f8(d, ad, bd, idesc, ((f.x & 1) && kk == 0) ? 0u : 1u);
-                    }
-                } else {
+                        for (int kk = 0; kk < kChunkCols / 32; kk++) {
+                            const uint64_t ad = smem_desc(a_s + kk * 32, 16, 512, 4);
+                            const uint64_t bd = smem_desc(b_s + kk * 4096, kChunkCols * 128, 1024);
+                            umma_f8(d, ad, bd, idesc, kk == 0 ? accum : 1u);
+                        }
+                    } else {
 #pragma unroll
-                    for (int kk = 0; kk < kChunkCols / 16; kk++) {
-                        const uint64_t ad = smem_desc(a_s + kk * 32, 16, 1024);
-                        const uint64_t bd = smem_desc(b_s + kk * 2048, kChunkCols * 128, 1024);
-                        umma_f16(d, ad, bd, idesc, ((f.x & 1) && kk == 0) ? 0u : 1u);
+                        for (int kk = 0; kk < kChunkCols / 16; kk++) {
+                            const uint64_t ad = smem_desc(a_s + kk * 32, 16, 1024);
+                            const uint64_t bd = smem_desc(b_s + kk * 2048, kChunkCols * 128, 1024);
+                            umma_f16(d, ad, bd, idesc, kk == 0 ? accum : 1u);
+                        }
                     }
+                    accum = 1;
+                    umma_commit(&empty[s]);
+                    if (++s == S) { s = 0; phase ^= 1; }
                 }
-                umma_commit(&empty[s]);
-                if ((f.x & 2) && !(withhold && k == n_items - 1))
+                if (ok && !(withhold && k == n_items - 1))
                     umma_commit(&acc_full[b]);
             }
             // every MMA issued has completed before the tensor memory is
@@ -458,6 +631,49 @@ __global__ void __launch_bounds__(kThreads, 1) spmm_tc_kernel(const __grid_const
                 ok = false;
         }
         __syncwarp();
+    } else if (warp < kEpiWarp0) {
+        // ---------------- scatter ----------------
+        int n_sparse = 0, k = 0; // sparse chunks of this CTA
+        for (int g0 = 0; g0 < total_chunks; g0 += 32) {
+            bool sparse = false;
+            if (g0 + lane < total_chunks) {
+                const int c = locate(g0 + lane, k);
+                sparse = __ldg(batch.job[items[k].w >> 16].img_idx + c) < 0;
+            }
+            n_sparse += __popc(__ballot_sync(0xffffffffu, sparse));
+        }
+        const int sid = (int)threadIdx.x - kScatterWarp0 * 32;
+        constexpr int kScatterThreads = kScatterWarps * 32;
+        int slot = 0;
+        uint32_t phase = 0;
+        for (int q = 0; q < n_sparse; q++) {
+            const bool got = mbar_wait(&staged[slot], phase);
+            const int2 pd = got ? pend[slot] : make_int2(0, 0);
+            uint8_t *At = smem + pd.x * Cfg::kStage;
+            if (got) {
+#pragma unroll
+                for (int o = 0; o < kATileBytes / (16 * kScatterThreads); o++)
+                    reinterpret_cast<uint4 *>(At)[sid + o * kScatterThreads] = make_uint4(0, 0, 0, 0);
+            }
+            // the tile is zero; and the warps agree whether to go on
+            if (!named_bar_and(kScatterBar, kScatterThreads, got)) { ok = false; break; }
+            const uint32_t *st = reinterpret_cast<const uint32_t *>(smem + Cfg::kStagingOff + slot * kStagingBytes);
+            const int end = (pd.y >> 2) + (pd.y & 3);
+#pragma unroll 4
+            for (int e = (pd.y & 3) + sid; e < end; e += kScatterThreads) {
+                const uint32_t v = st[e];
+                if constexpr (F8)
+                    At[swz64_offset(v >> 22, (v >> 16) & 63u)] = (uint8_t)(v & 0xffu);
+                else
+                    *reinterpret_cast<uint16_t *>(At + swz128_offset(v >> 22, (v >> 16) & 63u)) =
+                        (uint16_t)(v & 0xffffu);
+            }
+            fence_proxy_async();
+            named_bar_sync(kScatterBar, kScatterThreads); // every warp's part is written
+            if (sid == 0)
+                mbar_arrive(&full[pd.x]);
+            if (++slot == Cfg::kSlots) { slot = 0; phase ^= 1; }
+        }
     } else {
         // ---------------- epilogue ----------------
         const int quarter = warp & 3;
@@ -489,15 +705,20 @@ __global__ void __launch_bounds__(kThreads, 1) spmm_tc_kernel(const __grid_const
             float sa = 1.f;
             if constexpr (F8)
                 sa = (i < a.M) ? a.row_scale[i] : 0.f;
-            for (int cb = 0; cb < NT / 16; cb++) {
+            const float *sb0 = reinterpret_cast<const float *>(smem + Cfg::kScaleOff) + b * NT;
+            const uint32_t acc = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * NT);
+            if (a.beta == 0.f)
+                store_rows<NT, OutT, F8>(acc, reinterpret_cast<OutT *>(a.C), a.ldc, out_row, n0, a.N, a.alpha, sa, sb0,
+                                         lane);
+            for (int cb = 0; a.beta != 0.f && cb < NT / 16; cb++) {
                 const int n = n0 + cb * 16;
                 if (n >= a.N)
                     break; // uniform across the warp
                 uint32_t r[16];
-                tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * NT + cb * 16), r);
+                tmem_ld16(acc + (uint32_t)(cb * 16), r);
                 if constexpr (F8) { // dequantise: row scale x column scale (staged above; the barrier orders it)
                     float *f = reinterpret_cast<float *>(r);
-                    const float *sb = reinterpret_cast<const float *>(smem + Cfg::kScaleOff) + b * NT + cb * 16;
+                    const float *sb = sb0 + cb * 16;
 #pragma unroll
                     for (int q = 0; q < 16; q++) f[q] *= sa * sb[q];
                 }
@@ -565,6 +786,16 @@ __global__ void __launch_bounds__(kThreads, 1) spmm_tc_kernel(const __grid_const
 // exit each CTA waits (bounded) until its partner has made its last access to
 // this CTA's shared memory. No load uses multicast.
 constexpr int kPairN = 256;
+// roles of the pair kernel
+namespace pair {
+constexpr int kScatterThreads = 128; // warps 0-3: sparse-entry scatter
+constexpr int kLoaderWarp = 4;       // TMA issue, chunks g = 0 (mod kLoaders)
+constexpr int kMmaWarp = 5;          // TMEM allocation, tcgen05.mma issue
+constexpr int kEpiWarp0 = 6;         // warps 6-9: epilogue
+constexpr int kLoaderWarp1 = 10;     // warps 10..: TMA issue, chunks g = 1, 2, .. (mod kLoaders)
+constexpr int kLoaders = 4;          // loader warps, each issuing every kLoaders-th chunk
+constexpr int kThreads = 320 + (kLoaders - 1) * 32;
+} // namespace pair
 
 template <bool F8> struct Tc2Cfg {
     static constexpr int kElem = F8 ? 1 : 2;
@@ -586,7 +817,7 @@ template <bool F8> struct Tc2Cfg {
     static_assert(kSmem <= 227 * 1024, "shared memory budget");
     static_assert(kStage % 1024 == 0 && kATileBytes % 1024 == 0, "swizzled tiles need 1024-byte alignment");
     static_assert(kPendOff % 16 == 0 && kItemOff % 16 == 0 && kBarOff % 16 == 0, "16-byte aligned regions");
-    static_assert(kStages % 2 == 0 && kLoaders <= kStages, "two scatter groups; loaders may not lap a stage");
+    static_assert(kStages % 2 == 0 && pair::kLoaders <= kStages, "two scatter groups; loaders may not lap a stage");
 };
 
 // kind::f16 / kind::f8f6f4 instruction descriptor for M = 256 across the pair
@@ -643,7 +874,7 @@ __device__ __forceinline__ void decode_pair_item(const TcBatch &batch, int item,
 }
 
 template <typename OutT, bool F8>
-__global__ void __launch_bounds__(kThreads, 1) spmm_tc_pair_kernel(const __grid_constant__ TcBatch batch)
+__global__ void __launch_bounds__(pair::kThreads, 1) spmm_tc_pair_kernel(const __grid_constant__ TcBatch batch)
 {
     using Cfg = Tc2Cfg<F8>;
     constexpr int S = Cfg::kStages;
@@ -663,7 +894,7 @@ __global__ void __launch_bounds__(kThreads, 1) spmm_tc_pair_kernel(const __grid_
     uint64_t *bye = drain + 1;           // the partner is done with this CTA's shared memory
     volatile int *flag = reinterpret_cast<volatile int *>(bye + 1);
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bye + 1) + 4;
-    constexpr int kGroupThreads = kScatterThreads / 2;
+    constexpr int kGroupThreads = pair::kScatterThreads / 2;
 
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
@@ -698,7 +929,7 @@ __global__ void __launch_bounds__(kThreads, 1) spmm_tc_pair_kernel(const __grid_
     if ((int)threadIdx.x < n_items)
         decode_pair_item(batch, pair_id + (int)threadIdx.x * n_pairs_grid, rank, &items[2 * threadIdx.x],
                          &items[2 * threadIdx.x + 1]);
-    if (warp == kMmaWarp) {
+    if (warp == pair::kMmaWarp) {
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
                      "r"(2 * kPairN)
                      : "memory");
@@ -712,9 +943,9 @@ __global__ void __launch_bounds__(kThreads, 1) spmm_tc_pair_kernel(const __grid_
     int total_chunks = 0;
     for (int k = 0; k < n_items; k++) total_chunks += items[2 * k].z;
 
-    if (warp == kLoaderWarp || warp >= kLoaderWarp1) {
+    if (warp == pair::kLoaderWarp || warp >= pair::kLoaderWarp1) {
         // ---------------- loaders (as in spmm_tc_kernel; B: this CTA's half of N) ----------------
-        const int ld = warp == kLoaderWarp ? 0 : warp - kLoaderWarp1 + 1;
+        const int ld = warp == pair::kLoaderWarp ? 0 : warp - pair::kLoaderWarp1 + 1;
         auto advance = [&](int &k, int &i) {
             while (k < n_items && i >= items[2 * k].z) { i -= items[2 * k].z; k++; }
         };
@@ -742,7 +973,7 @@ __global__ void __launch_bounds__(kThreads, 1) spmm_tc_pair_kernel(const __grid_
         auto step = [&](Meta &cur, Meta &nxt) -> bool {
             if (g >= total_chunks || !ok)
                 return false;
-            int k2 = k, i2 = i + kLoaders;
+            int k2 = k, i2 = i + pair::kLoaders;
             advance(k2, i2);
             fetch(k2, i2, nxt);
             const int s = g % S;
@@ -793,7 +1024,7 @@ __global__ void __launch_bounds__(kThreads, 1) spmm_tc_pair_kernel(const __grid_
             }
             k = k2;
             i = i2;
-            g += kLoaders;
+            g += pair::kLoaders;
             return true;
         };
         Meta ma, mb;
@@ -832,7 +1063,7 @@ __global__ void __launch_bounds__(kThreads, 1) spmm_tc_pair_kernel(const __grid_
             }
             mbar_arrive(&full[s]);
         }
-    } else if (warp == kMmaWarp) {
+    } else if (warp == pair::kMmaWarp) {
         if (lane == 0) {
             if (rank == 0) {
                 // ---------------- MMA issuer for the pair ----------------
@@ -931,7 +1162,7 @@ __global__ void __launch_bounds__(kThreads, 1) spmm_tc_pair_kernel(const __grid_
             }
             tc_fence_before();
             named_bar_sync(kEpiBar, kEpiThreads); // the four warps are done with buffer b
-            if (warp == kEpiWarp0 && lane == 0) {
+            if (warp == pair::kEpiWarp0 && lane == 0) {
                 if (rank == 0)
                     mbar_arrive(&acc_empty[b]);
                 else
@@ -960,7 +1191,7 @@ __global__ void __launch_bounds__(kThreads, 1) spmm_tc_pair_kernel(const __grid_
             atomicOr(batch.job[items[0].w >> 16].status, kStatusTimeout);
     }
     __syncthreads();
-    if (warp == kMmaWarp) {
+    if (warp == pair::kMmaWarp) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * kPairN) : "memory");
     }
@@ -982,24 +1213,41 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder()
 
 } // namespace
 
-int encode_tensor_map_2d(CUtensorMap *map, CUtensorMapDataType dtype, const void *base, uint64_t d0, uint64_t d1,
-                         uint64_t row_stride_bytes, uint32_t b0, uint32_t b1, CUtensorMapSwizzle swizzle)
+namespace {
+int encode_tiled(CUtensorMap *map, CUtensorMapDataType dtype, int rank, const void *base, const cuuint64_t *dims,
+                 const cuuint64_t *strides, const cuuint32_t *box, CUtensorMapSwizzle swizzle)
 {
     auto enc = tensor_map_encoder();
     if (!enc)
         return set_error(TCA_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
-    const cuuint64_t dims[2] = {(cuuint64_t)d0, (cuuint64_t)(d1 > 0 ? d1 : 1)};
-    const cuuint64_t strides[1] = {(cuuint64_t)row_stride_bytes};
-    const cuuint32_t box[2] = {b0, b1};
-    const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = enc(map, dtype, 2, const_cast<void *>(base), dims, strides, box, estr,
+    const cuuint32_t estr[3] = {1, 1, 1};
+    const CUresult r = enc(map, dtype, (cuuint32_t)rank, const_cast<void *>(base), dims, strides, box, estr,
                            CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS)
         return set_error(TCA_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d): dims {%llu, %llu}, stride %llu, box {%u, %u}",
-                         (int)r, (unsigned long long)d0, (unsigned long long)d1, (unsigned long long)row_stride_bytes,
-                         b0, b1);
+                         (int)r, (unsigned long long)dims[0], (unsigned long long)dims[1],
+                         (unsigned long long)strides[0], box[0], box[1]);
     return TCA_OK;
+}
+} // namespace
+
+int encode_tensor_map_2d(CUtensorMap *map, CUtensorMapDataType dtype, const void *base, uint64_t d0, uint64_t d1,
+                         uint64_t row_stride_bytes, uint32_t b0, uint32_t b1, CUtensorMapSwizzle swizzle)
+{
+    const cuuint64_t dims[2] = {(cuuint64_t)d0, (cuuint64_t)(d1 > 0 ? d1 : 1)};
+    const cuuint64_t strides[1] = {(cuuint64_t)row_stride_bytes};
+    const cuuint32_t box[2] = {b0, b1};
+    return encode_tiled(map, dtype, 2, base, dims, strides, box, swizzle);
+}
+
+int encode_tensor_map_slabs(CUtensorMap *map, CUtensorMapDataType dtype, int elem, const void *base, uint64_t slabs,
+                            uint64_t d1, uint64_t row_stride_bytes, uint32_t b1, uint32_t bslabs)
+{
+    const cuuint64_t dims[3] = {(cuuint64_t)(128 / elem), (cuuint64_t)(d1 > 0 ? d1 : 1), (cuuint64_t)slabs};
+    const cuuint64_t strides[2] = {(cuuint64_t)row_stride_bytes, 128};
+    const cuuint32_t box[3] = {(cuuint32_t)(128 / elem), b1, bslabs};
+    return encode_tiled(map, dtype, 3, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
 namespace {
@@ -1012,23 +1260,42 @@ int encode_b_map(const SpmmJob &sj, int K, int rows, CUtensorMap *map)
                                 (uint64_t)sj.ldb * 2, 64, (uint32_t)rows, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
+// NT: the slice width of the single-window kernel; 0: the pair kernel.
 int make_job(const SpmmJob &sj, float alpha, float beta, unsigned flags, int NT, TcJob *out)
 {
     const tca_plan *p = sj.p;
     TcJob &j = *out;
+    const int slab = sj.f8 ? 128 : 64; // columns of a 128-byte slab of B
+    // One box per chunk when N is whole slabs (load-only ring of 148 CTAs,
+    // 48 KB chunks: 0.38 us per chunk against 0.44 us with a 2-D box per slab);
+    // else the tensor map must know where a row ends inside a slab.
+    j.tile3d = NT > 0 && sj.N % slab == 0;
+    if (NT == 0)
+        NT = kPairN;
     if (sj.f8) {
         // E4M3 B (K x N bytes, row stride ldq): boxes of 128 columns
         TCA_TRY(encode_tensor_map_2d(&j.tmap_b, CU_TENSOR_MAP_DATA_TYPE_UINT8, sj.Bq, (uint64_t)sj.N, (uint64_t)p->K,
                                      (uint64_t)sj.ldq, 128, 1, CU_TENSOR_MAP_SWIZZLE_128B));
-        TCA_TRY(encode_tensor_map_2d(&j.tmap_tile, CU_TENSOR_MAP_DATA_TYPE_UINT8, sj.Bq, (uint64_t)sj.N,
-                                     (uint64_t)p->K, (uint64_t)sj.ldq, 128, kChunkCols, CU_TENSOR_MAP_SWIZZLE_128B));
+        if (j.tile3d)
+            TCA_TRY(encode_tensor_map_slabs(&j.tmap_tile, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, sj.Bq,
+                                            (uint64_t)(sj.N / slab), (uint64_t)p->K, (uint64_t)sj.ldq, kChunkCols,
+                                            (uint32_t)(NT / slab)));
+        else
+            TCA_TRY(encode_tensor_map_2d(&j.tmap_tile, CU_TENSOR_MAP_DATA_TYPE_UINT8, sj.Bq, (uint64_t)sj.N,
+                                         (uint64_t)p->K, (uint64_t)sj.ldq, 128, kChunkCols,
+                                         CU_TENSOR_MAP_SWIZZLE_128B));
         j.entries = p->tile_entries_f8;
         j.images = p->images_f8;
         j.row_scale = p->row_scale;
         j.col_scale = sj.col_scale;
     } else {
         TCA_TRY(encode_b_map(sj, p->K, 1, &j.tmap_b));
-        TCA_TRY(encode_b_map(sj, p->K, kChunkCols, &j.tmap_tile));
+        if (j.tile3d)
+            TCA_TRY(encode_tensor_map_slabs(&j.tmap_tile, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, sj.B,
+                                            (uint64_t)(sj.N / slab), (uint64_t)p->K, (uint64_t)sj.ldb * 2, kChunkCols,
+                                            (uint32_t)(NT / slab)));
+        else
+            TCA_TRY(encode_b_map(sj, p->K, kChunkCols, &j.tmap_tile));
         j.entries = p->tile_entries;
         j.images = reinterpret_cast<const uint8_t *>(p->images);
         j.row_scale = nullptr;
@@ -1119,7 +1386,7 @@ int launch_pair_group(const TcBatch &b, cudaStream_t s)
     attr[0].val.clusterDim.x = 2;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
-    cfg.blockDim = dim3(kThreads);
+    cfg.blockDim = dim3(pair::kThreads);
     cfg.dynamicSmemBytes = (size_t)smem;
     cfg.stream = s;
     cfg.attrs = attr;
@@ -1181,29 +1448,29 @@ int tc_block_regs(bool f8, int *regs)
             (const void *)spmm_tc_kernel<64, __half, false>, (const void *)spmm_tc_kernel<128, __half, false>,
             (const void *)spmm_tc_kernel<256, __half, false>, (const void *)spmm_tc_kernel<64, float, false>,
             (const void *)spmm_tc_kernel<128, float, false>, (const void *)spmm_tc_kernel<256, float, false>,
-            (const void *)spmm_tc_pair_kernel<__half, false>, (const void *)spmm_tc_pair_kernel<float, false>,
             (const void *)spmm_tc_kernel<64, __half, false, 1>, (const void *)spmm_tc_kernel<128, __half, false, 1>,
             (const void *)spmm_tc_kernel<256, __half, false, 1>, (const void *)spmm_tc_kernel<64, float, false, 1>,
             (const void *)spmm_tc_kernel<128, float, false, 1>, (const void *)spmm_tc_kernel<256, float, false, 1>};
         const void *f8_fns[] = {
             (const void *)spmm_tc_kernel<128, __half, true>, (const void *)spmm_tc_kernel<256, __half, true>,
             (const void *)spmm_tc_kernel<128, float, true>, (const void *)spmm_tc_kernel<256, float, true>,
-            (const void *)spmm_tc_pair_kernel<__half, true>, (const void *)spmm_tc_pair_kernel<float, true>,
             (const void *)spmm_tc_kernel<128, __half, true, 1>, (const void *)spmm_tc_kernel<256, __half, true, 1>,
             (const void *)spmm_tc_kernel<128, float, true, 1>, (const void *)spmm_tc_kernel<256, float, true, 1>};
+        const void *pair_fns[2][2] = {
+            {(const void *)spmm_tc_pair_kernel<__half, false>, (const void *)spmm_tc_pair_kernel<float, false>},
+            {(const void *)spmm_tc_pair_kernel<__half, true>, (const void *)spmm_tc_pair_kernel<float, true>}};
         int w = 0;
-        for (const void *f : f16_fns) {
-            if (f8) break;
+        auto widest = [&w](const void *f, int threads) -> int {
             int r = 0;
-            TCA_TRY(block_regs(f, kThreads, &r));
+            TCA_TRY(block_regs(f, threads, &r));
             w = std::max(w, r);
-        }
-        for (const void *f : f8_fns) {
-            if (!f8) break;
-            int r = 0;
-            TCA_TRY(block_regs(f, kThreads, &r));
-            w = std::max(w, r);
-        }
+            return TCA_OK;
+        };
+        if (f8)
+            for (const void *f : f8_fns) TCA_TRY(widest(f, kThreads));
+        else
+            for (const void *f : f16_fns) TCA_TRY(widest(f, kThreads));
+        for (const void *f : pair_fns[f8]) TCA_TRY(widest(f, pair::kThreads));
         worst[f8] = w;
     }
     *regs = worst[f8];
@@ -1247,7 +1514,7 @@ int launch_tc_jobs(const SpmmJob *jobs, int n_jobs, int c_dtype, float alpha, fl
                 const bool pair = pair_eligible(sj.p, sj.n_tile);
                 if (NT == 0 ? !pair : (pair || sj.n_tile != NT))
                     continue;
-                TCA_TRY(make_job(sj, alpha, beta, flags, NT == 0 ? kPairN : NT, &b.job[b.n_jobs]));
+                TCA_TRY(make_job(sj, alpha, beta, flags, NT, &b.job[b.n_jobs]));
                 const int units = NT == 0 ? sj.p->n_pairs : sj.p->n_tc;
                 b.item_start[b.n_jobs + 1] = b.item_start[b.n_jobs] + units * b.job[b.n_jobs].ntiles;
                 b.n_jobs++;
