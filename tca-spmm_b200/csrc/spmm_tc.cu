@@ -65,7 +65,6 @@ constexpr int kAhead = 4;        // chunks by which the entries of a sparse chun
 constexpr int kRecords = 64;     // chunk records kept: two batches of 32
 constexpr int kMaxCtaItems = 32;      // work items per persistent CTA
 constexpr int kEpiBar = 3;           // named barrier of the epilogue warps
-constexpr int kScatterBar = 1;       // named barrier of the scatter warps
 constexpr int kStagingBytes = ((kImageMinNnz + 3) * 4 + 15) & ~15; // entries of a sparse chunk, 16-byte rounded
 constexpr int kMaxJobs = 32;                                  // jobs per launch (kernel parameter space)
 
@@ -171,7 +170,8 @@ template <int NT, bool F8> struct TcCfg {
     static constexpr int kBTileBytes = kChunkCols * NT * kElem;
     static constexpr int kStage = kATileBytes + kBTileBytes;
     static constexpr int kStagingOff = kStages * kStage;
-    static constexpr int kSlots = kStages + kAhead;                       // entry staging slots (see the scatter role)
+    // entry staging slots: kStages + kAhead, rounded up to a multiple of the scatter warps (see the scatter role)
+    static constexpr int kSlots = (kStages + kAhead + kScatterWarps - 1) / kScatterWarps * kScatterWarps;
     static constexpr int kRecOff = kStagingOff + kSlots * kStagingBytes;  // TcRecordA, TcRecordB [kRecords]
     static constexpr int kItemOff = kRecOff + kRecords * 32;              // int4 [kMaxCtaItems]
     static constexpr int kPendOff = kItemOff + kMaxCtaItems * 16;         // int2 [kSlots]: stage, entries
@@ -305,13 +305,17 @@ __device__ __forceinline__ void store_rows(uint32_t acc, OutT *C, int ldc, int o
 //     wait until its TMEM accumulator buffer (item parity) is drained
 //     ("accum_empty"); 4 x tcgen05.mma (2 for E4M3); commit "empty"; on the
 //     item's last chunk commit "accum_full".
-//   warps 3-6 (scatter): per sparse chunk, once its entries are in and its
-//     stage is free ("staged"): zero the A tile, write the entries into the
-//     swizzled layout, arrive on "full" -- while the chunk's B rows are still
-//     on their way; image chunks pass them by. Sparse chunk q uses slot
-//     q % kSlots; it is filled when chunk g is issued, at most kAhead chunks
-//     before its own, so sparse chunk q - kSlots lies at least kStages chunks
-//     before g and is consumed.
+//   warps 3-6 (scatter): sparse chunk q belongs to warp q % 4, which, once
+//     the entries are in and the stage is free ("staged"), zeroes the A tile,
+//     writes the entries into the swizzled layout and arrives on "full" --
+//     while the chunk's B rows are still on their way; image chunks pass them
+//     by. (A warp per chunk and not all four per chunk: the steps of a chunk
+//     are a chain of ~0.6 us, and four chunks then run through it at once.)
+//     Sparse chunk q uses slot q % kSlots; it is filled when chunk g is
+//     issued, at most kAhead chunks before its own, so sparse chunk q -
+//     kSlots lies at least kStages chunks before g and is consumed; kSlots is
+//     a multiple of 4, so a slot always belongs to one warp and no wait is
+//     more than one phase behind its barrier.
 //   warps 7-10 (epilogue): per item wait "accum_full", tcgen05.ld the rows
 //     (warp w reads TMEM lanes 32 (w % 4) ..), alpha/beta, store to C[perm],
 //     arrive "accum_empty" -- overlapping the next item's main loop.
@@ -642,25 +646,19 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
             }
             n_sparse += __popc(__ballot_sync(0xffffffffu, sparse));
         }
-        const int sid = (int)threadIdx.x - kScatterWarp0 * 32;
-        constexpr int kScatterThreads = kScatterWarps * 32;
-        int slot = 0;
-        uint32_t phase = 0;
-        for (int q = 0; q < n_sparse; q++) {
-            const bool got = mbar_wait(&staged[slot], phase);
-            const int2 pd = got ? pend[slot] : make_int2(0, 0);
+        for (int q = warp - kScatterWarp0; q < n_sparse; q += kScatterWarps) {
+            const int slot = q % Cfg::kSlots;
+            if (!mbar_wait(&staged[slot], (uint32_t)(q / Cfg::kSlots) & 1u)) { ok = false; break; }
+            const int2 pd = pend[slot];
             uint8_t *At = smem + pd.x * Cfg::kStage;
-            if (got) {
-#pragma unroll
-                for (int o = 0; o < kATileBytes / (16 * kScatterThreads); o++)
-                    reinterpret_cast<uint4 *>(At)[sid + o * kScatterThreads] = make_uint4(0, 0, 0, 0);
-            }
-            // the tile is zero; and the warps agree whether to go on
-            if (!named_bar_and(kScatterBar, kScatterThreads, got)) { ok = false; break; }
+#pragma unroll 8
+            for (int o = 0; o < kATileBytes / (16 * 32); o++)
+                reinterpret_cast<uint4 *>(At)[lane + o * 32] = make_uint4(0, 0, 0, 0);
+            __syncwarp();
             const uint32_t *st = reinterpret_cast<const uint32_t *>(smem + Cfg::kStagingOff + slot * kStagingBytes);
             const int end = (pd.y >> 2) + (pd.y & 3);
 #pragma unroll 4
-            for (int e = (pd.y & 3) + sid; e < end; e += kScatterThreads) {
+            for (int e = (pd.y & 3) + lane; e < end; e += 32) {
                 const uint32_t v = st[e];
                 if constexpr (F8)
                     At[swz64_offset(v >> 22, (v >> 16) & 63u)] = (uint8_t)(v & 0xffu);
@@ -669,10 +667,9 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
                         (uint16_t)(v & 0xffffu);
             }
             fence_proxy_async();
-            named_bar_sync(kScatterBar, kScatterThreads); // every warp's part is written
-            if (sid == 0)
+            __syncwarp();
+            if (lane == 0)
                 mbar_arrive(&full[pd.x]);
-            if (++slot == Cfg::kSlots) { slot = 0; phase ^= 1; }
         }
     } else {
         // ---------------- epilogue ----------------
