@@ -3,20 +3,17 @@
 // C[r, :] = alpha * sum_j val_j * B[col_j, :] + beta * C[r, :], FP32 accumulation.
 // This restates the computation of kernel_our_spmm_balanced
 // (src/our_spmm.cu:290-346) without its host-built warp schedule and without
-// using mma.sync as a dot-product engine: a group of LPR lanes owns one row,
-// each lane owns 8 consecutive output columns (one 16-byte vector of B), and
-// the group walks the row's nonzeros, broadcasting (col, val) pairs by shuffle
-// so that every B access is a fully used, coalesced 16-byte load with 8 loads
-// in flight per lane.
+// using mma.sync as a dot-product engine.
 //
 // Kernels:
-//   * plan-free (tca_spmm_csr): group g computes caller row g straight from
-//     the CSR, 8 B loads in flight per lane;
+//   * spmm_rows_kernel: straight from a CSR, blocks of strided rows whose
+//     nonzeros are cut into equal runs -- the plan-free forward
+//     (tca_spmm_csr), and planned forwards whose dense operands are not
+//     16-byte aligned;
 //   * planned (tca_spmm / tca_spmm_batched): warps stream through work items
 //     of consecutive sorted rows of one or many plans (spmm_cc_stream_kernel,
-//     below; spmm_cc_items_kernel for operands that are not 16-byte aligned),
-//     or compute them as small mma.sync products (spmm_cc_mma_kernel, an
-//     autotuner candidate for FP16).
+//     below), or compute them as small mma.sync products (spmm_cc_mma_kernel,
+//     an autotuner candidate for FP16).
 //
 // Malformed CSR never faults: row ranges are clamped to [0, nnz] and
 // nonzeros whose column is outside [0, K) contribute nothing.
@@ -30,17 +27,6 @@
 
 namespace tca {
 namespace {
-
-__device__ __forceinline__ void fma8(float *acc, float a, const uint4 &b)
-{
-    const __half2 *h = reinterpret_cast<const __half2 *>(&b);
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        float2 f = __half22float2(h[i]);
-        acc[2 * i] = fmaf(a, f.x, acc[2 * i]);
-        acc[2 * i + 1] = fmaf(a, f.y, acc[2 * i + 1]);
-    }
-}
 
 __device__ __forceinline__ void load8(const __half *p, float *v)
 {
@@ -81,152 +67,301 @@ template <typename T> __device__ __forceinline__ T from_f(float x);
 template <> __device__ __forceinline__ __half from_f<__half>(float x) { return __float2half_rn(x); }
 template <> __device__ __forceinline__ float from_f<float>(float x) { return x; }
 
-// One row with LPR lanes, vectorised: N % 8 == 0, ldb % 8 == 0, 16-byte
-// aligned B and C rows. Every lane of the group must call it.
-template <typename OutT, int LPR>
-__device__ __forceinline__ void row_vec(int start, int end, int K, const int *__restrict__ col_idx,
-                                        const __half *__restrict__ vals, const __half *__restrict__ B, int ldb,
-                                        int N, OutT *__restrict__ Crow, float alpha, float beta, int sub,
-                                        unsigned gmask)
-{
-    constexpr int U = 8; // nonzeros in flight per lane
-    for (int nb = 0; nb < N; nb += LPR * 8) {
-        const int n0 = nb + sub * 8;
-        const bool active = n0 < N;
-        const __half *Bn = B + (active ? n0 : 0);
-        float acc[8];
-#pragma unroll
-        for (int i = 0; i < 8; i++) acc[i] = 0.f;
-
-        for (int base = start; base < end; base += LPR) {
-            const int j = base + sub;
-            int c = -1;
-            float a = 0.f;
-            if (j < end) {
-                c = __ldg(col_idx + j);
-                a = __half2float(vals[j]);
-                if (c < 0 || c >= K) { c = -1; a = 0.f; }
-            }
-            const int cnt = min(LPR, end - base);
-            int t = 0;
-            for (; t + U <= cnt; t += U) {
-                uint4 bv[U];
-                float av[U];
-#pragma unroll
-                for (int u = 0; u < U; u++) {
-                    const int cu = __shfl_sync(gmask, c, t + u, LPR);
-                    av[u] = __shfl_sync(gmask, a, t + u, LPR);
-                    bv[u] = make_uint4(0, 0, 0, 0);
-                    if (active && cu >= 0)
-                        bv[u] = __ldg(reinterpret_cast<const uint4 *>(Bn + (size_t)cu * ldb));
-                }
-#pragma unroll
-                for (int u = 0; u < U; u++) fma8(acc, av[u], bv[u]);
-            }
-            for (; t < cnt; t++) {
-                const int cu = __shfl_sync(gmask, c, t, LPR);
-                const float au = __shfl_sync(gmask, a, t, LPR);
-                if (active && cu >= 0)
-                    fma8(acc, au, __ldg(reinterpret_cast<const uint4 *>(Bn + (size_t)cu * ldb)));
-            }
-        }
-        if (active) {
-            OutT *cp = Crow + n0;
-            float out[8];
-            if (beta != 0.f) {
-                float old[8];
-                load8(cp, old);
-#pragma unroll
-                for (int i = 0; i < 8; i++) out[i] = fmaf(alpha, acc[i], beta * old[i]);
-            } else {
-#pragma unroll
-                for (int i = 0; i < 8; i++) out[i] = alpha * acc[i];
-            }
-            store8(cp, out);
-        }
-    }
-}
-
-// One row with a full warp, scalar: any N, leading dimension and alignment.
-template <typename OutT>
-__device__ __forceinline__ void row_scalar(int start, int end, int K, const int *__restrict__ col_idx,
-                                           const __half *__restrict__ vals, const __half *__restrict__ B,
-                                           int ldb, int N, OutT *__restrict__ Crow, float alpha, float beta,
-                                           int lane)
-{
-    for (int nb = 0; nb < N; nb += 32) {
-        const int n = nb + lane;
-        float acc = 0.f;
-        for (int base = start; base < end; base += 32) {
-            const int j = base + lane;
-            int c = -1;
-            float a = 0.f;
-            if (j < end) {
-                c = col_idx[j];
-                a = __half2float(vals[j]);
-                if (c < 0 || c >= K) { c = -1; a = 0.f; }
-            }
-            const int cnt = min(32, end - base);
-            for (int t = 0; t < cnt; t++) {
-                const int cu = __shfl_sync(0xffffffffu, c, t);
-                const float au = __shfl_sync(0xffffffffu, a, t);
-                if (n < N && cu >= 0)
-                    acc = fmaf(au, __half2float(B[(size_t)cu * ldb + n]), acc);
-            }
-        }
-        if (n < N) {
-            float o = alpha * acc;
-            if (beta != 0.f) o = fmaf(beta, to_f<OutT>(Crow[n]), o);
-            Crow[n] = from_f<OutT>(o);
-        }
-    }
-}
-
 __device__ __forceinline__ void clamp_range(int &start, int &end, int nnz)
 {
     start = max(0, min(start, nnz));
     end = max(start, min(end, nnz));
 }
 
-// Plan-free: group g of LPR lanes computes caller row g.
-template <typename OutT, int LPR>
-__global__ void __launch_bounds__(256)
-spmm_csr_vec_kernel(const int *__restrict__ row_ptr, const int *__restrict__ col_idx,
-                    const __half *__restrict__ vals, int M, int K, int nnz,
-                    const __half *__restrict__ B, int ldb, int N,
-                    OutT *__restrict__ C, int ldc, float alpha, float beta, unsigned flags)
-{
-    const int lane = threadIdx.x & 31;
-    const int sub = lane & (LPR - 1);
-    const long long group = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / LPR;
-    const unsigned gmask = (LPR == 32) ? 0xffffffffu : (((1u << LPR) - 1u) << (lane & ~(LPR - 1)));
-    if (group >= M)
-        return; // the whole group leaves together
-    const int r = (int)group;
-    int start = row_ptr[r], end = row_ptr[r + 1];
-    clamp_range(start, end, nnz);
-    if (start == end && (flags & TCA_FLAG_KEEP_EMPTY_ROWS))
-        return;
-    row_vec<OutT, LPR>(start, end, K, col_idx, vals, B, ldb, N, C + (size_t)r * ldc, alpha, beta, sub, gmask);
-}
+constexpr int kMaxCcJobs = 32;
 
-template <typename OutT>
-__global__ void __launch_bounds__(256)
-spmm_csr_scalar_kernel(const int *__restrict__ row_ptr, const int *__restrict__ col_idx,
-                       const __half *__restrict__ vals, int M, int K, int nnz,
-                       const __half *__restrict__ B, int ldb, int N,
-                       OutT *__restrict__ C, int ldc, float alpha, float beta, unsigned flags)
+// ---------------------------------------------------------------------------
+// Rows straight from a CSR: the caller's (plan-free) or a plan's re-ordered
+// one when the dense operands do not allow 16-byte accesses.
+//
+// A row of a skewed matrix can hold every column (one group of lanes walking
+// 1024 nonzeros took 120 us), so no row belongs to one group. Block b takes
+// the rows whose key row_ptr[r] + r lies in the b-th of equal parts (found by a
+// 32-way search: rows and nonzeros are both balanced, whatever the order of
+// the rows) and cuts their nonzeros, laid end to end, into equal runs, one per
+// group of LPR lanes. A group writes the rows that lie in its run; of a row
+// that began before its run it leaves the partial sum in shared memory, and
+// the group in which the row began adds those in run order (a fixed order) and
+// writes it. What bounds it is the gather of B rows from L2, U of them in
+// flight per lane.
+// Malformed CSR: rows are clamped to [0, nnz] one by one and indices are
+// checked, as everywhere in this file.
+// ---------------------------------------------------------------------------
+constexpr int kRowsThreads = 512;
+constexpr int kRowsMax = kRowsThreads; // rows in shared memory at a time: a thread each
+
+struct RowsJob {
+    const int *row_ptr, *col;
+    const int *perm; // row i of the CSR -> row of C; NULL: itself
+    const __half *val, *B;
+    void *C;
+    int M, K, nnz, N, ldb, ldc;
+    int n_blocks; // blocks per N-slice
+    float alpha, beta;
+    unsigned flags;
+};
+template <int CAP> struct RowsBatchT {
+    int n_jobs;
+    int block_start[CAP + 1];
+    RowsJob job[CAP];
+};
+
+// W output columns per lane of a group of LPR lanes. VEC: 8 consecutive ones,
+// in 16-byte accesses (N % 8 == 0, 16-byte aligned rows); else every LPR-th.
+template <typename OutT, int LPR, int W, bool VEC, int CAP>
+__global__ void __launch_bounds__(kRowsThreads, 2) spmm_rows_kernel(const __grid_constant__ RowsBatchT<CAP> batch)
 {
-    const int lane = threadIdx.x & 31;
-    const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (warp >= M)
-        return;
-    const int r = (int)warp;
-    int start = row_ptr[r], end = row_ptr[r + 1];
-    clamp_range(start, end, nnz);
-    if (start == end && (flags & TCA_FLAG_KEEP_EMPTY_ROWS))
-        return;
-    row_scalar<OutT>(start, end, K, col_idx, vals, B, ldb, N, C + (size_t)r * ldc, alpha, beta, lane);
+    static_assert(!VEC || W == 8, "16-byte accesses cover 8 columns");
+    constexpr int G = kRowsThreads / LPR;
+    constexpr int U = VEC ? 4 : W >= 8 ? 2 : W >= 4 ? 4 : 8; // nonzeros in flight per lane
+    __shared__ int s_start[kRowsMax], s_pre[kRowsMax + 1], s_warp[kRowsThreads / 32], s_range[2];
+    __shared__ __align__(16) float s_part[G * LPR * W];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = lane & (LPR - 1), g = (int)threadIdx.x / LPR;
+    const unsigned gmask = LPR == 32 ? 0xffffffffu : (((1u << LPR) - 1u) << (lane & ~(LPR - 1)));
+    int jb = 0;
+    while (jb + 1 < batch.n_jobs && batch.block_start[jb + 1] <= (int)blockIdx.x) jb++;
+    const RowsJob &a = batch.job[jb];
+    const int local = (int)blockIdx.x - batch.block_start[jb];
+    const int slice = local / a.n_blocks, b = local - slice * a.n_blocks;
+
+    // this block's rows: each half of the threads finds the first row whose
+    // key is at least its bound, kRowsThreads / 2 probes at a time
+    {
+        constexpr int kProbes = kRowsThreads / 2;
+        const int half = (int)threadIdx.x / kProbes, p = (int)threadIdx.x % kProbes, part = b + half;
+        const long long bound = ((long long)a.nnz + a.M) * part / a.n_blocks;
+        int lo = 0, len = part == 0 ? 0 : a.M; // the row is in [lo, lo + len]
+        if (part == a.n_blocks) {
+            lo = a.M;
+            len = 0;
+        }
+        while (__syncthreads_or(len > 0)) { // both halves take the same number of rounds
+            const int step = (len + kProbes - 1) / kProbes;
+            if (p == 0) s_range[half] = kProbes; // probe p is row lo + p * step
+            __syncthreads();
+            if (p * step < len) {
+                const int r = lo + p * step;
+                if ((long long)min(max(__ldg(a.row_ptr + r), 0), a.nnz) + r >= bound) atomicMin(&s_range[half], p);
+            }
+            __syncthreads();
+            const int first = s_range[half];
+            if (len > 0) { // the row lies after probe first - 1 and not after probe first
+                const int hi = lo + min(len, first * step);
+                if (first > 0) lo += (min(first, (len + step - 1) / step) - 1) * step + 1;
+                len = hi - lo;
+            }
+        }
+        if (p == 0) s_range[half] = lo;
+    }
+    __syncthreads();
+    const int row_end = s_range[1];
+    for (int row0 = s_range[0]; row0 < row_end; row0 += kRowsMax) {
+    const int n_rows = min(kRowsMax, row_end - row0);
+    { // the rows' starts and the prefix sums of their lengths
+        int len = 0;
+        if ((int)threadIdx.x < n_rows) {
+            int st = __ldg(a.row_ptr + row0 + threadIdx.x), en = __ldg(a.row_ptr + row0 + threadIdx.x + 1);
+            clamp_range(st, en, a.nnz);
+            len = en - st;
+            s_start[threadIdx.x] = st;
+        }
+        int sum = len;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, sum, o);
+            if (lane >= o) sum += v;
+        }
+        if (lane == 31) s_warp[warp] = sum;
+        __syncthreads();
+        int carry = 0;
+        for (int k = 0; k < warp; k++) carry += s_warp[k];
+        if ((int)threadIdx.x < n_rows) s_pre[threadIdx.x + 1] = carry + sum;
+        if (threadIdx.x == 0) s_pre[0] = 0;
+    }
+    __syncthreads();
+    const int total = s_pre[n_rows];
+    // a valid CSR's rows follow one another: position v is nonzero first + v
+    const int first = s_start[0];
+    const bool dense = __syncthreads_and((int)threadIdx.x >= n_rows ||
+                                         s_start[threadIdx.x] == first + s_pre[threadIdx.x]);
+    auto run_start = [&](int k) -> int { return (int)((long long)total * k / G); };
+    // the row that holds position v of the block's nonzeros: the last one starting at or before v
+    auto row_of = [&](int v) -> int {
+        int lo = 0, hi = n_rows - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (s_pre[mid] <= v) lo = mid;
+            else hi = mid - 1;
+        }
+        return lo;
+    };
+    const int n0 = slice * (LPR * W) + (VEC ? sub * W : sub);
+    auto col_ok = [&](int w) -> bool { return VEC ? n0 < a.N : n0 + w * LPR < a.N; };
+    auto write = [&](int i, const float *acc) {
+        const int r = row0 + i;
+        OutT *cp = reinterpret_cast<OutT *>(a.C) + (size_t)(a.perm ? __ldg(a.perm + r) : r) * a.ldc + n0;
+        if constexpr (VEC) {
+            if (!col_ok(0))
+                return;
+            float o[8];
+            if (a.beta != 0.f) {
+                float old[8];
+                load8(cp, old);
+#pragma unroll
+                for (int w = 0; w < 8; w++) o[w] = fmaf(a.alpha, acc[w], a.beta * old[w]);
+            } else {
+#pragma unroll
+                for (int w = 0; w < 8; w++) o[w] = a.alpha * acc[w];
+            }
+            store8(cp, o);
+        } else {
+#pragma unroll
+            for (int w = 0; w < W; w++) {
+                if (!col_ok(w))
+                    continue;
+                float o = a.alpha * acc[w];
+                if (a.beta != 0.f) o = fmaf(a.beta, to_f<OutT>(cp[w * LPR]), o);
+                cp[w * LPR] = from_f<OutT>(o);
+            }
+        }
+    };
+    float *part = s_part + (g * LPR + sub) * W;
+    auto leave = [&](const float *acc) {
+#pragma unroll
+        for (int w = 0; w < W; w++) part[w] = acc[w];
+    };
+
+    const int v0 = run_start(g), v1 = run_start(g + 1);
+    float acc[W];
+#pragma unroll
+    for (int w = 0; w < W; w++) acc[w] = 0.f;
+    int cr = 0, ce = 0;
+    bool before = false, tail = false; // row cr began in an earlier run; goes on in a later one
+    if (v0 < v1) {
+        cr = row_of(v0);
+        ce = s_pre[cr + 1];
+        before = s_pre[cr] < v0;
+        auto flush = [&](int v) { // row cr ends at v
+            if (before) leave(acc);
+            else write(cr, acc);
+            before = false;
+#pragma unroll
+            for (int w = 0; w < W; w++) acc[w] = 0.f;
+            do cr++; while (cr + 1 < n_rows && s_pre[cr + 1] <= v);
+            ce = cr < n_rows ? s_pre[cr + 1] : 0x7fffffff;
+        };
+        const __half *Bn = a.B + n0;
+        // nonzero of this lane in the LPR from `base` on
+        auto load_nz = [&](int base, int &c, unsigned short &x) {
+            c = -1;
+            x = 0;
+            const int v = base + sub;
+            if (v < v1) {
+                int j = first + v;
+                if (!dense) {
+                    const int i = row_of(v);
+                    j = s_start[i] + (v - s_pre[i]);
+                }
+                if (j >= 0 && j < a.nnz) {
+                    c = __ldg(a.col + j);
+                    x = __half_as_ushort(a.val[j]);
+                    if (c < 0 || c >= a.K) { c = -1; x = 0; } // adds 0 * 0
+                }
+            }
+        };
+        int c, cn;
+        unsigned short x, xn;
+        load_nz(v0, cn, xn);
+        for (int base = v0; base < v1; base += LPR) {
+            c = cn;
+            x = xn;
+            load_nz(base + LPR, cn, xn);
+            const int cnt = min(LPR, v1 - base);
+            for (int t = 0; t < cnt; t += U) {
+                int cu[U];
+                unsigned short xu[U];
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    cu[u] = __shfl_sync(gmask, c, (t + u) & (LPR - 1), LPR);
+                    xu[u] = (unsigned short)__shfl_sync(gmask, (int)x, (t + u) & (LPR - 1), LPR);
+                    if (t + u >= cnt) cu[u] = -1;
+                }
+                if constexpr (VEC) {
+                    uint4 bv[U];
+#pragma unroll
+                    for (int u = 0; u < U; u++) {
+                        bv[u] = make_uint4(0, 0, 0, 0);
+                        if (cu[u] >= 0 && col_ok(0))
+                            bv[u] = __ldg(reinterpret_cast<const uint4 *>(Bn + (size_t)cu[u] * a.ldb));
+                    }
+#pragma unroll
+                    for (int u = 0; u < U; u++) {
+                        if (t + u < cnt) {
+                            if (base + t + u >= ce) flush(base + t + u);
+                            const unsigned short *h = reinterpret_cast<const unsigned short *>(&bv[u]);
+#pragma unroll
+                            for (int w = 0; w < 8; w++) acc[w] = ptx::fma_f16_f32(xu[u], h[w], acc[w]);
+                        }
+                    }
+                } else {
+                    unsigned short bv[U][W];
+#pragma unroll
+                    for (int u = 0; u < U; u++) {
+                        const __half *br = Bn + (size_t)max(cu[u], 0) * a.ldb;
+#pragma unroll
+                        for (int w = 0; w < W; w++)
+                            bv[u][w] = cu[u] >= 0 && col_ok(w) ? __half_as_ushort(br[w * LPR]) : (unsigned short)0;
+                    }
+#pragma unroll
+                    for (int u = 0; u < U; u++) {
+                        if (t + u < cnt) {
+                            if (base + t + u >= ce) flush(base + t + u);
+#pragma unroll
+                            for (int w = 0; w < W; w++) acc[w] = ptx::fma_f16_f32(xu[u], bv[u][w], acc[w]);
+                        }
+                    }
+                }
+            }
+        }
+        // the run's last row
+        if (ce <= v1) {
+            if (before) leave(acc);
+            else write(cr, acc);
+        } else if (before) {
+            leave(acc);
+        } else {
+            tail = true;
+        }
+    } else {
+        leave(acc); // an empty run adds zero to a row that spans it
+    }
+    __syncthreads();
+    if (tail) { // the row goes on in the next runs: add their parts in run order
+        int k_end = g + 1;
+        while (k_end < G && run_start(k_end) < ce) k_end++;
+        const float *q = part;
+#pragma unroll 4
+        for (int k = g + 1; k < k_end; k++) {
+            q += LPR * W;
+#pragma unroll
+            for (int w = 0; w < W; w++) acc[w] += q[w];
+        }
+        write(cr, acc);
+    }
+    if (!(a.flags & TCA_FLAG_KEEP_EMPTY_ROWS)) {
+#pragma unroll
+        for (int w = 0; w < W; w++) acc[w] = 0.f;
+        for (int i = g; i < n_rows; i += G)
+            if (s_pre[i] == s_pre[i + 1])
+                write(i, acc);
+    }
+    __syncthreads(); // the next rows reuse shared memory
+    }
 }
 
 // Rows of plans, batched and streamed. Every job (one forward of one plan)
@@ -237,8 +372,6 @@ spmm_csr_scalar_kernel(const int *__restrict__ row_ptr, const int *__restrict__ 
 // accumulators to C[perm[row]] whenever the stream crosses a row end. Short
 // rows thus cost no dependent load chain per row, and a launch keeps
 // thousands of items in flight.
-constexpr int kMaxCcJobs = 32;
-
 struct CcJob {
     const int2 *items;
     const int *perm, *p_row_ptr, *p_col;
@@ -260,111 +393,10 @@ struct CcJob {
 template <int CAP>
 struct CcBatchT {
     int n_jobs;
-    int block_start[CAP + 1]; // first block of each job (spmm_cc_items_kernel)
-    int item_start[CAP + 1];  // first item of each job in the flattened list (spmm_cc_stream_kernel)
+    int item_start[CAP + 1]; // first item of each job in the flattened list
     CcJob job[CAP];
 };
 using CcBatch = CcBatchT<kMaxCcJobs>;
-
-template <typename OutT, int L, bool VEC>
-__global__ void __launch_bounds__(256) spmm_cc_items_kernel(const __grid_constant__ CcBatch b)
-{
-    constexpr int G = 256 / L;      // groups per block
-    constexpr int W = VEC ? 8 : 1;  // output columns per lane per pass
-    constexpr int U = 8;            // B loads in flight per lane
-    __shared__ int s_rs[G][kItemRows + 1];
-    __shared__ int s_out[G][kItemRows];
-    const int lane = threadIdx.x & 31;
-    const int sub = lane & (L - 1);
-    const int g = (int)threadIdx.x / L;
-    const unsigned gmask = (L == 32) ? 0xffffffffu : (((1u << L) - 1u) << (lane & ~(L - 1)));
-    int j = 0;
-    while (j + 1 < b.n_jobs && b.block_start[j + 1] <= (int)blockIdx.x) j++;
-    const CcJob &a = b.job[j];
-    const int item = ((int)blockIdx.x - b.block_start[j]) * G + g;
-    if (item >= a.n_items)
-        return; // whole group
-    const int2 it = a.items[item];
-    const int r0 = it.x, nrows = it.y - it.x;
-    for (int k = sub; k <= nrows; k += L) {
-        s_rs[g][k] = a.p_row_ptr[r0 + k];
-        if (k < nrows)
-            s_out[g][k] = a.perm[r0 + k];
-    }
-    __syncwarp(gmask);
-    const int j0 = s_rs[g][0], j1 = s_rs[g][nrows];
-    const bool keep = (a.flags & TCA_FLAG_KEEP_EMPTY_ROWS) != 0;
-
-    for (int nb = 0; nb < a.N; nb += L * W) {
-        const int n0 = nb + sub * W;
-        const bool active = n0 < a.N;
-        float acc[W];
-#pragma unroll
-        for (int i = 0; i < W; i++) acc[i] = 0.f;
-        int cr = 0;
-        int ce = s_rs[g][1];
-        auto flush = [&]() {
-            const bool empty_row = s_rs[g][cr] == ce;
-            if (active && !(keep && empty_row)) {
-                OutT *cp = reinterpret_cast<OutT *>(a.C) + (size_t)s_out[g][cr] * a.ldc + n0;
-                float out[W];
-                if (a.beta != 0.f) {
-                    float old[W];
-                    if constexpr (VEC) load8(cp, old); else old[0] = to_f<OutT>(*cp);
-#pragma unroll
-                    for (int i = 0; i < W; i++) out[i] = fmaf(a.alpha, acc[i], a.beta * old[i]);
-                } else {
-#pragma unroll
-                    for (int i = 0; i < W; i++) out[i] = a.alpha * acc[i];
-                }
-                if constexpr (VEC) store8(cp, out); else *cp = from_f<OutT>(out[0]);
-            }
-#pragma unroll
-            for (int i = 0; i < W; i++) acc[i] = 0.f;
-            cr++;
-            ce = (cr < nrows) ? s_rs[g][cr + 1] : 0x7fffffff;
-        };
-        const __half *Bn = a.B + (active ? n0 : 0);
-        for (int base = j0; base < j1; base += L) {
-            const int jj = base + sub;
-            int c = -1;
-            float v = 0.f;
-            if (jj < j1) {
-                c = __ldg(a.p_col + jj);
-                v = __half2float(a.p_val[jj]);
-            }
-            const int cnt = min(L, j1 - base);
-            for (int t = 0; t < cnt; t += U) {
-                uint4 bv[U];
-                float av[U];
-#pragma unroll
-                for (int u = 0; u < U; u++) {
-                    const int cu = __shfl_sync(gmask, c, (t + u) & (L - 1), L);
-                    av[u] = __shfl_sync(gmask, v, (t + u) & (L - 1), L);
-                    bv[u] = make_uint4(0, 0, 0, 0);
-                    if (active && t + u < cnt) {
-                        if constexpr (VEC)
-                            bv[u] = __ldg(reinterpret_cast<const uint4 *>(Bn + (size_t)cu * a.ldb));
-                        else
-                            bv[u].x = __half_as_ushort(Bn[(size_t)cu * a.ldb]);
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < U; u++) {
-                    if (t + u < cnt) { // uniform across the group
-                        while (base + t + u >= ce) flush();
-                        if constexpr (VEC) {
-                            fma8(acc, av[u], bv[u]);
-                        } else {
-                            acc[0] = fmaf(av[u], __half2float(__ushort_as_half((unsigned short)bv[u].x)), acc[0]);
-                        }
-                    }
-                }
-            }
-        }
-        while (cr < nrows) flush();
-    }
-}
 
 // ---------------------------------------------------------------------------
 // Vectorised item stream: one warp per stream of items, persistent.
@@ -704,29 +736,6 @@ __global__ void __launch_bounds__(256, 3) spmm_cc_stream_kernel(const __grid_con
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
-template <typename OutT, int LPR>
-void launch_vec(const int *rp, const int *ci, const __half *v, int M, int K, int nnz, const __half *B, int ldb,
-                int N, OutT *C, int ldc, float alpha, float beta, unsigned flags, cudaStream_t s)
-{
-    const long long threads = (long long)M * LPR;
-    const unsigned grid = (unsigned)((threads + 255) / 256);
-    spmm_csr_vec_kernel<OutT, LPR><<<grid, 256, 0, s>>>(rp, ci, v, M, K, nnz, B, ldb, N, C, ldc, alpha, beta, flags);
-}
-
-inline int pick_lpr(int N) { return N <= 32 ? 4 : N <= 64 ? 8 : N <= 128 ? 16 : 32; }
-
-template <typename OutT>
-void dispatch_vec(const int *rp, const int *ci, const __half *v, int M, int K, int nnz, const __half *B, int ldb,
-                  int N, OutT *C, int ldc, float alpha, float beta, unsigned flags, cudaStream_t s)
-{
-    switch (pick_lpr(N)) {
-    case 4: launch_vec<OutT, 4>(rp, ci, v, M, K, nnz, B, ldb, N, C, ldc, alpha, beta, flags, s); break;
-    case 8: launch_vec<OutT, 8>(rp, ci, v, M, K, nnz, B, ldb, N, C, ldc, alpha, beta, flags, s); break;
-    case 16: launch_vec<OutT, 16>(rp, ci, v, M, K, nnz, B, ldb, N, C, ldc, alpha, beta, flags, s); break;
-    default: launch_vec<OutT, 32>(rp, ci, v, M, K, nnz, B, ldb, N, C, ldc, alpha, beta, flags, s); break;
-    }
-}
-
 bool vec_ok(const void *B, int ldb, int N, const void *C, int ldc, int c_dtype)
 {
     const size_t c_elem = (c_dtype == TCA_DTYPE_F16) ? 2 : 4;
@@ -735,26 +744,92 @@ bool vec_ok(const void *B, int ldb, int N, const void *C, int ldc, int c_dtype)
 
 } // namespace
 
+namespace {
+
+// Lanes and blocks of a job of the rows kernel. A group covers N in one slice
+// up to 256 columns: narrower groups spend more instructions per byte gathered
+// (measured, 4096 x 4096 at 95 %, N = 512: 8 lanes a row 193 us, 32 lanes
+// 118 us). Blocks: about 64 nonzeros and rows per group, so that a
+// block's fixed cost (search, prefix sums, first dependent loads) is small
+// beside them, but at least two blocks per SM while a group keeps 8.
+struct RowsShape { int lpr, w; };
+RowsShape rows_shape(int N, bool vec)
+{
+    if (vec)
+        return {N <= 32 ? 4 : N <= 64 ? 8 : N <= 128 ? 16 : 32, 8};
+    return {32, N <= 32 ? 1 : N <= 64 ? 2 : N <= 128 ? 4 : 8};
+}
+int rows_blocks(const RowsJob &a, const RowsShape &sh, int slices) // per N-slice
+{
+    const long long groups = kRowsThreads / sh.lpr, keys = (long long)a.nnz + a.M;
+    const long long fill = std::min<long long>((2 * kSMs + slices - 1) / slices, (keys + groups * 8 - 1) / (groups * 8));
+    const long long n = std::max((keys + groups * 64 - 1) / (groups * 64), fill);
+    return (int)std::max<long long>(1, std::min<long long>(n, a.M));
+}
+
+template <typename OutT, int LPR, int W, bool VEC>
+int launch_rows(const RowsBatchT<kMaxCcJobs> &b, cudaStream_t s)
+{
+    const int grid = b.block_start[b.n_jobs];
+    if (b.n_jobs == 0 || grid == 0)
+        return TCA_OK;
+    if (b.n_jobs == 1) {
+        RowsBatchT<1> one;
+        one.n_jobs = 1;
+        one.block_start[0] = 0;
+        one.block_start[1] = grid;
+        one.job[0] = b.job[0];
+        spmm_rows_kernel<OutT, LPR, W, VEC, 1><<<grid, kRowsThreads, 0, s>>>(one);
+    } else {
+        spmm_rows_kernel<OutT, LPR, W, VEC, kMaxCcJobs><<<grid, kRowsThreads, 0, s>>>(b);
+    }
+    TCA_CUDA_TRY(cudaGetLastError());
+    return TCA_OK;
+}
+
+template <typename OutT>
+int launch_rows_shape(const RowsBatchT<kMaxCcJobs> &b, const RowsShape &sh, bool vec, cudaStream_t s)
+{
+    if (vec) {
+        switch (sh.lpr) {
+        case 4: return launch_rows<OutT, 4, 8, true>(b, s);
+        case 8: return launch_rows<OutT, 8, 8, true>(b, s);
+        case 16: return launch_rows<OutT, 16, 8, true>(b, s);
+        default: return launch_rows<OutT, 32, 8, true>(b, s);
+        }
+    }
+    switch (sh.w) {
+    case 1: return launch_rows<OutT, 32, 1, false>(b, s);
+    case 2: return launch_rows<OutT, 32, 2, false>(b, s);
+    case 4: return launch_rows<OutT, 32, 4, false>(b, s);
+    default: return launch_rows<OutT, 32, 8, false>(b, s);
+    }
+}
+
+void rows_add(RowsBatchT<kMaxCcJobs> &b, RowsJob &a, const RowsShape &sh)
+{
+    const int slices = (a.N + sh.lpr * sh.w - 1) / (sh.lpr * sh.w);
+    a.n_blocks = rows_blocks(a, sh, slices);
+    b.job[b.n_jobs] = a;
+    b.block_start[b.n_jobs + 1] = b.block_start[b.n_jobs] + a.n_blocks * slices;
+    b.n_jobs++;
+}
+
+} // namespace
+
 int launch_spmm_csr_cc(const int *row_ptr, const int *col_idx, const __half *vals, int M, int K, int nnz,
                        const __half *B, int ldb, int N, void *C, int ldc, int c_dtype,
                        float alpha, float beta, unsigned flags, cudaStream_t stream)
 {
-    if (vec_ok(B, ldb, N, C, ldc, c_dtype)) {
-        if (c_dtype == TCA_DTYPE_F16)
-            dispatch_vec<__half>(row_ptr, col_idx, vals, M, K, nnz, B, ldb, N, (__half *)C, ldc, alpha, beta, flags, stream);
-        else
-            dispatch_vec<float>(row_ptr, col_idx, vals, M, K, nnz, B, ldb, N, (float *)C, ldc, alpha, beta, flags, stream);
-    } else {
-        const unsigned grid = (unsigned)(((long long)M * 32 + 255) / 256);
-        if (c_dtype == TCA_DTYPE_F16)
-            spmm_csr_scalar_kernel<__half><<<grid, 256, 0, stream>>>(row_ptr, col_idx, vals, M, K, nnz, B, ldb, N,
-                                                                     (__half *)C, ldc, alpha, beta, flags);
-        else
-            spmm_csr_scalar_kernel<float><<<grid, 256, 0, stream>>>(row_ptr, col_idx, vals, M, K, nnz, B, ldb, N,
-                                                                    (float *)C, ldc, alpha, beta, flags);
-    }
-    TCA_CUDA_TRY(cudaGetLastError());
-    return TCA_OK;
+    const bool vec = vec_ok(B, ldb, N, C, ldc, c_dtype);
+    const RowsShape sh = rows_shape(N, vec);
+    RowsBatchT<kMaxCcJobs> b;
+    b.n_jobs = 0;
+    b.block_start[0] = 0;
+    RowsJob a{row_ptr, col_idx, nullptr, vals, B, C, M, K, nnz, N, ldb, ldc, 0, alpha, beta, flags};
+    rows_add(b, a, sh);
+    return c_dtype == TCA_DTYPE_F16 ? launch_rows_shape<__half>(b, sh, vec, stream)
+                                    : launch_rows_shape<float>(b, sh, vec, stream);
 }
 
 bool dense_operands_vec_ok(const void *B, int ldb, int N, const void *C, int ldc, int c_dtype)
@@ -763,16 +838,6 @@ bool dense_operands_vec_ok(const void *B, int ldb, int N, const void *C, int ldc
 }
 
 namespace {
-
-template <typename OutT, int LPR, bool VEC>
-int launch_cc_group(const CcBatch &b, cudaStream_t s)
-{
-    if (b.n_jobs == 0 || b.block_start[b.n_jobs] == 0)
-        return TCA_OK;
-    spmm_cc_items_kernel<OutT, LPR, VEC><<<b.block_start[b.n_jobs], 256, 0, s>>>(b);
-    TCA_CUDA_TRY(cudaGetLastError());
-    return TCA_OK;
-}
 
 // ---------------------------------------------------------------------------
 // Tensor-core item kernel (mma.sync, FP16): the CUDA-core windows' work items
@@ -1047,8 +1112,6 @@ int launch_stream_group(const CcBatch &b, int beside_regs, cudaStream_t s)
     if (b.n_jobs == 1) {
         CcBatchT<1> one;
         one.n_jobs = 1;
-        one.block_start[0] = b.block_start[0];
-        one.block_start[1] = b.block_start[1];
         one.item_start[0] = b.item_start[0];
         one.item_start[1] = b.item_start[1];
         one.job[0] = b.job[0];
@@ -1089,9 +1152,8 @@ int launch_stream_w(const CcBatch &b, int w, int beside_regs, cudaStream_t s)
 }
 
 template <typename OutT>
-int launch_cc_typed(const CcBatch &b, int w, bool vec, bool f8, int beside_regs, cudaStream_t s)
+int launch_cc_typed(const CcBatch &b, int w, bool f8, int beside_regs, cudaStream_t s)
 {
-    if (!vec) return launch_cc_group<OutT, 32, false>(b, s);
     if (w == kCcMma) return launch_mma_group<OutT>(b, s);
     return f8 ? launch_stream_w<OutT, true>(b, w, beside_regs, s) : launch_stream_w<OutT, false>(b, w, beside_regs, s);
 }
@@ -1101,22 +1163,61 @@ int launch_cc_typed(const CcBatch &b, int w, bool vec, bool f8, int beside_regs,
 int launch_cc_jobs(const SpmmJob *jobs, int n_jobs, int c_dtype, float alpha, float beta, unsigned flags,
                    cudaStream_t s, LaunchList *defer, int beside_regs)
 {
-    // groups: (columns per lane, vectorised, E4M3) -- stream kernel with 2/4/8 columns, scalar items
-    // and the FP16 tensor-core item kernel (kCcMma)
-    const int kinds[8][3] = {{2, 1, 0}, {4, 1, 0}, {8, 1, 0}, {kCcMma, 1, 0}, {32, 0, 0}, {2, 1, 1}, {4, 1, 1}, {8, 1, 1}};
+    // jobs whose operands do not allow 16-byte accesses (every window of the
+    // plan: the tensor-core kernel needs them too): the rows kernel
+    for (int w : {1, 2, 4, 8}) {
+        RowsBatchT<kMaxCcJobs> b;
+        b.n_jobs = 0;
+        b.block_start[0] = 0;
+        auto flush = [&]() -> int {
+            if (b.n_jobs == 0)
+                return TCA_OK;
+            auto run = [c_dtype, w](const RowsBatchT<kMaxCcJobs> &bb, cudaStream_t st) {
+                const RowsShape sh{32, w};
+                return c_dtype == TCA_DTYPE_F16 ? launch_rows_shape<__half>(bb, sh, false, st)
+                                                : launch_rows_shape<float>(bb, sh, false, st);
+            };
+            int status = TCA_OK;
+            if (defer) {
+                auto held = std::make_shared<RowsBatchT<kMaxCcJobs>>(b);
+                defer->push_back([held, run](cudaStream_t st) { return run(*held, st); });
+            } else {
+                status = run(b, s);
+            }
+            b.n_jobs = 0;
+            return status;
+        };
+        for (int i = 0; i < n_jobs; i++) {
+            const SpmmJob &sj = jobs[i];
+            const tca_plan *p = sj.p;
+            if (sj.f8 || sj.N <= 0 || p->M == 0 || vec_ok(sj.B, sj.ldb, sj.N, sj.C, sj.ldc, c_dtype))
+                continue;
+            const RowsShape sh = rows_shape(sj.N, false);
+            if (sh.w != w)
+                continue;
+            RowsJob a{p->p_row_ptr, p->p_col, p->perm, p->p_val, sj.B, sj.C, p->M, p->K, p->nnz, sj.N, sj.ldb, sj.ldc,
+                      0, alpha, beta, flags};
+            rows_add(b, a, sh);
+            if (b.n_jobs == kMaxCcJobs)
+                TCA_TRY(flush());
+        }
+        TCA_TRY(flush());
+    }
+    // groups: (columns per lane, E4M3) -- stream kernel with 2/4/8 columns and
+    // the FP16 tensor-core item kernel (kCcMma)
+    const int kinds[7][2] = {{2, 0}, {4, 0}, {8, 0}, {kCcMma, 0}, {2, 1}, {4, 1}, {8, 1}};
     for (const auto &kd : kinds) {
         CcBatch b;
         b.n_jobs = 0;
-        b.block_start[0] = 0;
         b.item_start[0] = 0;
         auto flush = [&]() -> int {
             if (b.n_jobs == 0)
                 return TCA_OK;
             const int w = kd[0];
-            const bool vec = kd[1] != 0, f8 = kd[2] != 0;
-            auto run = [c_dtype, w, vec, f8, beside_regs](const CcBatch &bb, cudaStream_t st) {
-                return (c_dtype == TCA_DTYPE_F16) ? launch_cc_typed<__half>(bb, w, vec, f8, beside_regs, st)
-                                                  : launch_cc_typed<float>(bb, w, vec, f8, beside_regs, st);
+            const bool f8 = kd[1] != 0;
+            auto run = [c_dtype, w, f8, beside_regs](const CcBatch &bb, cudaStream_t st) {
+                return (c_dtype == TCA_DTYPE_F16) ? launch_cc_typed<__half>(bb, w, f8, beside_regs, st)
+                                                  : launch_cc_typed<float>(bb, w, f8, beside_regs, st);
             };
             int status = TCA_OK;
             if (defer) {
@@ -1135,14 +1236,12 @@ int launch_cc_jobs(const SpmmJob *jobs, int n_jobs, int c_dtype, float alpha, fl
             if (n_items == 0 || sj.N <= 0)
                 continue;
             // E4M3 jobs always qualify (B is the library's own aligned copy; C was checked)
-            const bool vec = sj.f8 || vec_ok(sj.B, sj.ldb, sj.N, sj.C, sj.ldc, c_dtype);
-            int lpr = 32;
-            if (vec) {
-                lpr = (sj.cc_w == 2 || sj.cc_w == 4 || sj.cc_w == 8) ? sj.cc_w : pick_w(sj.N);
-                if (sj.cc_w == kCcMma && !sj.f8)
-                    lpr = kCcMma;
-            }
-            if (lpr != kd[0] || (vec ? 1 : 0) != kd[1] || (sj.f8 ? 1 : 0) != kd[2])
+            if (!sj.f8 && !vec_ok(sj.B, sj.ldb, sj.N, sj.C, sj.ldc, c_dtype))
+                continue;
+            int w = (sj.cc_w == 2 || sj.cc_w == 4 || sj.cc_w == 8) ? sj.cc_w : pick_w(sj.N);
+            if (sj.cc_w == kCcMma && !sj.f8)
+                w = kCcMma;
+            if (w != kd[0] || (sj.f8 ? 1 : 0) != kd[1])
                 continue;
             CcJob &a = b.job[b.n_jobs];
             a.items = sj.tc ? p->cc_items : p->all_items;
@@ -1166,8 +1265,6 @@ int launch_cc_jobs(const SpmmJob *jobs, int n_jobs, int c_dtype, float alpha, fl
             a.alpha = alpha;
             a.beta = beta;
             a.flags = flags;
-            const int per_block = vec ? 8 : 256 / lpr;
-            b.block_start[b.n_jobs + 1] = b.block_start[b.n_jobs] + (a.n_items + per_block - 1) / per_block;
             b.item_start[b.n_jobs + 1] = b.item_start[b.n_jobs] + a.n_items;
             b.n_jobs++;
             if (b.n_jobs == kMaxCcJobs)
