@@ -64,14 +64,6 @@ __global__ void k_scatter_half(const int *__restrict__ idx, const __half *__rest
         dst[idx[i]] = src[i];
 }
 
-__global__ void k_gather_half(const int *__restrict__ idx, const __half *__restrict__ src, __half *__restrict__ dst,
-                              int n)
-{
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n)
-        dst[i] = src[idx[i]];
-}
-
 // Sorted row of warp w: w itself, or with a window list (the CUDA-core
 // windows) row w % 128 of window windows[w / 128]; -1 past the rows.
 __device__ __forceinline__ long long sddmm_row(long long w, const int *windows, long long n_rows, int M)
@@ -185,8 +177,8 @@ int build_transpose(tca_plan *p, cudaStream_t s)
     if (p->tplan)
         return TCA_OK;
     const int M = p->M, K = p->K, nnz = p->nnz;
-    Tmp tk, tk2, tv, tv2, tcount, trp, tcol, tcub;
-    for (Tmp *t : {&tk, &tk2, &tv, &tv2, &tcount, &trp, &tcol, &tcub}) t->s = s;
+    Tmp tk, tk2, tv, tv2, tcount, trp, tcol, tval, tcub;
+    for (Tmp *t : {&tk, &tk2, &tv, &tv2, &tcount, &trp, &tcol, &tval, &tcub}) t->s = s;
     unsigned long long *keys = nullptr, *keys2 = nullptr;
     int *order = nullptr, *order2 = nullptr, *count = nullptr, *t_rp = nullptr, *t_col = nullptr;
     const size_t n1 = nnz > 0 ? nnz : 1;
@@ -198,7 +190,8 @@ int build_transpose(tca_plan *p, cudaStream_t s)
     TCA_TRY(dev_malloc((void **)&t_rp, sizeof(int) * (size_t)(K + 1), s)); trp.p = t_rp;
     TCA_TRY(dev_malloc((void **)&t_col, sizeof(int) * n1, s)); tcol.p = t_col;
     TCA_TRY(dev_malloc((void **)&p->t_src, sizeof(int) * n1, s));
-    TCA_TRY(dev_malloc((void **)&p->t_vals, sizeof(__half) * n1, s));
+    __half *t_val = nullptr; // only for the build: the plan keeps its own copy
+    TCA_TRY(dev_malloc((void **)&t_val, sizeof(__half) * n1, s)); tval.p = t_val;
     TCA_CUDA_TRY(cudaMemsetAsync(count, 0, sizeof(int) * (size_t)(K + 1), s));
     if (M > 0)
         k_transpose_keys<<<blocks_of((long long)M * 32, 256), 256, 0, s>>>(p->perm, p->p_row_ptr, p->p_col, p->src,
@@ -218,7 +211,7 @@ int build_transpose(tca_plan *p, cudaStream_t s)
         // (src is a permutation, so the scatter has no conflicts)
         k_scatter_half<<<blocks_of(nnz, 256), 256, 0, s>>>(p->src, p->p_val, vals_caller, nnz);
         k_transpose_fill<<<blocks_of(nnz, 256), 256, 0, s>>>(keys2, order2, vals_caller, nnz, count, t_col,
-                                                            p->t_vals, p->t_src);
+                                                            t_val, p->t_src);
         TCA_CUDA_TRY(cudaGetLastError());
         TCA_CUDA_TRY(cudaStreamSynchronize(s)); // vals_caller freed at scope exit
     }
@@ -233,7 +226,7 @@ int build_transpose(tca_plan *p, cudaStream_t s)
         TCA_CUDA_TRY(cudaStreamSynchronize(s));
     }
     tca_plan_t tp = nullptr;
-    TCA_TRY(tca_plan_create(t_rp, t_col, p->t_vals, K, M, nnz, &p->opts, (tca_stream_t)s, &tp));
+    TCA_TRY(tca_plan_create(t_rp, t_col, t_val, K, M, nnz, &p->opts, (tca_stream_t)s, &tp));
     p->tplan = tp;
     return TCA_OK;
 }
@@ -313,23 +306,12 @@ int tca_sddmm(tca_plan_t plan, const void *d_dY_f16, int ldy, const void *d_B_f1
 } // extern "C"
 
 namespace tca {
-// Called by tca_plan_update_values / tca_plan_destroy (plan.cu).
-int transpose_update_values(tca_plan *p, const __half *vals, cudaStream_t s)
-{
-    if (!p->tplan || p->nnz == 0)
-        return TCA_OK;
-    k_gather_half<<<blocks_of(p->nnz, 256), 256, 0, s>>>(p->t_src, vals, p->t_vals, p->nnz);
-    TCA_CUDA_TRY(cudaGetLastError());
-    return tca_plan_update_values(p->tplan, p->t_vals, (tca_stream_t)s);
-}
-
+// Called by tca_plan_destroy (plan.cu).
 void transpose_free(tca_plan *p)
 {
     if (p->tplan) tca_plan_destroy(p->tplan);
     if (p->t_src) dev_free(p->t_src, nullptr);
-    if (p->t_vals) dev_free(p->t_vals, nullptr);
     p->tplan = nullptr;
     p->t_src = nullptr;
-    p->t_vals = nullptr;
 }
 } // namespace tca

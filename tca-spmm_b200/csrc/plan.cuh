@@ -25,6 +25,7 @@
 //                      swizzled K-major layout the tensor cores read from
 //                      shared memory; img_idx is -1 for the other chunks
 #pragma once
+#include <atomic>
 #include <functional>
 #include <vector>
 #include "tca_internal.cuh"
@@ -75,12 +76,13 @@ struct tca_plan {
     // all_items, images).
     void *arena[3] = {nullptr, nullptr, nullptr};
     size_t bytes = 0;
+    // counts tca_plan_update_values calls
+    std::atomic<unsigned long long> values_version{0};
     // A^T as a plan of its own (built on first use by tca_spmm_t or by
     // tca_plan_build_transpose), with t_src mapping each of its entries to the
-    // caller's nonzero index and t_vals the values in that order.
+    // caller's nonzero index.
     struct tca_plan *tplan = nullptr;
     int *t_src = nullptr;
-    __half *t_vals = nullptr;
     // FP8-E4M3 representation of A (tca_plan_quantize_fp8): per sorted row an
     // FP32 scale (row absmax / 448), the quantized values in sorted order, the
     // tile entries with E4M3 bits in their low byte, and 8 KB dense images
@@ -204,8 +206,7 @@ int sddmm_tc(const tca_plan *p, const __half *dY, int ldy, const __half *B, int 
 int plan_requantize_fp8(tca_plan *p, cudaStream_t s);
 void plan_free_fp8(tca_plan *p);
 
-// The plan of A^T (adjoint.cu): propagate new caller-order values; release.
-int transpose_update_values(tca_plan *p, const __half *vals, cudaStream_t s);
+// The plan of A^T (adjoint.cu): release.
 void transpose_free(tca_plan *p);
 
 // Whether B/C of a forward allow the vectorised and tensor-core kernels.

@@ -1218,9 +1218,18 @@ int encode_tiled(CUtensorMap *map, CUtensorMapDataType dtype, int rank, const vo
     if (!enc)
         return set_error(TCA_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
     const cuuint32_t estr[3] = {1, 1, 1};
-    const CUresult r = enc(map, dtype, (cuuint32_t)rank, const_cast<void *>(base), dims, strides, box, estr,
-                           CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    auto encode = [&] {
+        return enc(map, dtype, (cuuint32_t)rank, const_cast<void *>(base), dims, strides, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    };
+    CUresult r = encode();
+    if (r == CUDA_ERROR_INVALID_CONTEXT) { // a host thread's first CUDA call: make the device's context current
+        int dev = 0;
+        TCA_CUDA_TRY(cudaGetDevice(&dev));
+        TCA_CUDA_TRY(cudaSetDevice(dev));
+        r = encode();
+    }
     if (r != CUDA_SUCCESS)
         return set_error(TCA_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d): dims {%llu, %llu}, stride %llu, box {%u, %u}",
                          (int)r, (unsigned long long)dims[0], (unsigned long long)dims[1],

@@ -85,6 +85,7 @@ _SIGS = {
     "tca_plan_opts_default": ([ctypes.POINTER(PlanOpts)], None),
     "tca_plan_create": ([_P, _P, _P, _I, _I, _I, ctypes.POINTER(PlanOpts), _VP, ctypes.POINTER(_VP)], _I),
     "tca_plan_update_values": ([_VP, _P, _VP], _I),
+    "tca_plan_values_version": ([_VP, ctypes.POINTER(ctypes.c_ulonglong)], _I),
     "tca_plan_info": ([_VP, ctypes.POINTER(PlanInfo)], _I),
     "tca_plan_export": ([_VP, _I, _P, ctypes.c_size_t, ctypes.POINTER(ctypes.c_size_t)], _I),
     "tca_plan_status": ([_VP], _I),
@@ -272,6 +273,12 @@ class Plan:
 
     def update_values(self, vals, stream=None):
         _check(self._lib.tca_plan_update_values(self._h, _ptr(vals), _stream_handle(stream)))
+
+    def values_version(self) -> int:
+        """How many times the plan's values have been replaced (tca_plan_values_version)."""
+        v = ctypes.c_ulonglong()
+        _check(self._lib.tca_plan_values_version(self._h, ctypes.byref(v)))
+        return v.value
 
     def status(self):
         _check(self._lib.tca_plan_status(self._h))

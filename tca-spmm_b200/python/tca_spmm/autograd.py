@@ -20,6 +20,7 @@ class SpMMFunction(torch.autograd.Function):
         v16 = vals.detach().to(torch.float16).contiguous()
         B16 = B.detach().to(torch.float16).contiguous()
         plan.update_values(v16)
+        ctx.values_version = plan.values_version()
         Y = plan.spmm(B16, out_dtype=out_dtype)
         ctx.plan = plan
         ctx.save_for_backward(v16, B16)
@@ -32,12 +33,17 @@ class SpMMFunction(torch.autograd.Function):
         plan = ctx.plan
         dY16 = dY.to(torch.float16).contiguous()
         d_vals = d_B = None
-        if ctx.needs_input_grad[0] or ctx.needs_input_grad[1]:
-            plan.update_values(v16)  # the pattern's values as they were in forward
+        # the pattern's values as they were in forward: another forward may have replaced them
+        if ctx.needs_input_grad[1] and plan.values_version() != ctx.values_version:
+            plan.update_values(v16)
+        # gradients in the inputs' types: FP32 sums, rounded once by the kernel that forms them
+        direct = (torch.float16, torch.float32)
         if ctx.needs_input_grad[0]:
-            d_vals = plan.sddmm(dY16, B16, out_dtype=torch.float32).to(ctx.vals_dtype)
+            out = ctx.vals_dtype if ctx.vals_dtype in direct else torch.float32
+            d_vals = plan.sddmm(dY16, B16, out_dtype=out).to(ctx.vals_dtype)
         if ctx.needs_input_grad[1]:
-            d_B = plan.spmm_t(dY16, out_dtype=torch.float32).to(ctx.B_dtype)
+            out = ctx.B_dtype if ctx.B_dtype in direct else torch.float32
+            d_B = plan.spmm_t(dY16, out_dtype=out).to(ctx.B_dtype)
         return d_vals, d_B, None, None
 
 
