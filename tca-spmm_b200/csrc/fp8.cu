@@ -16,7 +16,9 @@
 #include <mutex>
 #include <vector>
 #include "tca_internal.cuh"
+#include <cuda.h>
 #include "plan.cuh"
+#include "ptx.cuh"
 
 namespace tca {
 namespace {
@@ -101,249 +103,11 @@ struct QBatch {
     QJob job[kMaxQJobs];
 };
 
-__global__ void k_col_zero(const __grid_constant__ QBatch b)
-{
-    const QJob &q = b.job[blockIdx.z];
-    for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < q.N; n += gridDim.x * blockDim.x) q.colmax[n] = 0u;
-}
-
 // B rows load 8 halves (16 bytes) at a time when B and its rows are 16-byte
 // aligned; otherwise one half at a time.
 __device__ __forceinline__ bool vec8_ok(const QJob &q)
 {
     return (reinterpret_cast<uintptr_t>(q.B) & 15u) == 0 && (q.ldb & 7) == 0;
-}
-
-__device__ __forceinline__ void load8h(const QJob &q, int k, int n, bool vec, float *v)
-{
-    const __half *row = q.B + (size_t)k * q.ldb;
-    if (vec && n + 8 <= q.N) {
-        const uint4 u = __ldg(reinterpret_cast<const uint4 *>(row + n));
-        const __half2 *h = reinterpret_cast<const __half2 *>(&u);
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const float2 f = __half22float2(h[i]);
-            v[2 * i] = f.x;
-            v[2 * i + 1] = f.y;
-        }
-    } else {
-#pragma unroll
-        for (int i = 0; i < 8; i++) v[i] = n + i < q.N ? __half2float(row[n + i]) : 0.f;
-    }
-}
-
-// The two B passes tile B into blocks of 64 rows x 256 columns: thread
-// (x, y) of a 32 x 8 block takes the 8 consecutive columns (one 16-byte
-// vector) 8 x of the block's columns in the 8 consecutive rows 8 y .. of its
-// rows, so that a warp reads whole 512-byte row segments; all 8 loads of a
-// thread are issued before the first is used (blockIdx.z = matrix).
-constexpr int kQTileRows = 64, kQTileCols = 256, kQRows = kQTileRows / 8;
-
-struct QTile {
-    int n, k0, k1;
-    bool fast; // full 16-byte vectors and all kQRows rows in range
-};
-
-__device__ __forceinline__ QTile q_tile(const QJob &q)
-{
-    QTile t;
-    t.n = blockIdx.x * kQTileCols + threadIdx.x * 8;
-    t.k0 = blockIdx.y * kQTileRows + threadIdx.y * kQRows;
-    t.k1 = min(q.K, t.k0 + kQRows);
-    t.fast = vec8_ok(q) && t.n + 8 <= q.N && t.k0 + kQRows <= q.K;
-    return t;
-}
-
-__device__ __forceinline__ void load_rows8(const QJob &q, const QTile &t, uint4 *r)
-{
-#pragma unroll
-    for (int j = 0; j < kQRows; j++)
-        r[j] = __ldg(reinterpret_cast<const uint4 *>(q.B + (size_t)(t.k0 + j) * q.ldb + t.n));
-    asm volatile("" ::: "memory"); // every load issued before the first use
-}
-
-// Column absolute maxima (FP32 bit patterns order like the non-negative
-// values): per thread the maxima of its rows, per block the maxima over its
-// 8 row slices (shared memory), then one atomicMax per column and block.
-__global__ void __launch_bounds__(256) k_col_absmax(const __grid_constant__ QBatch b)
-{
-    const QJob &q = b.job[blockIdx.z];
-    if ((int)blockIdx.x * kQTileCols >= q.N || (int)blockIdx.y * kQTileRows >= q.K)
-        return; // whole block
-    __shared__ float s_m[8][8][32]; // [row slice][column in vector][vector]
-    const QTile t = q_tile(q);
-    float m[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    if (t.fast) {
-        uint4 r[kQRows];
-        load_rows8(q, t, r);
-#pragma unroll
-        for (int j = 0; j < kQRows; j++) {
-            const __half2 *h = reinterpret_cast<const __half2 *>(&r[j]);
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const float2 f = __half22float2(h[i]);
-                m[2 * i] = fmaxf(m[2 * i], fabsf(f.x));
-                m[2 * i + 1] = fmaxf(m[2 * i + 1], fabsf(f.y));
-            }
-        }
-    } else if (t.n < q.N) {
-        const bool vec = vec8_ok(q);
-        for (int k = t.k0; k < t.k1; k++) {
-            float v[8];
-            load8h(q, k, t.n, vec, v);
-#pragma unroll
-            for (int i = 0; i < 8; i++) m[i] = fmaxf(m[i], fabsf(v[i]));
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < 8; i++) s_m[threadIdx.y][i][threadIdx.x] = m[i];
-    __syncthreads();
-    const int c = threadIdx.y * 32 + threadIdx.x; // column of the block: vector c / 8, element c % 8
-    float v = 0.f;
-#pragma unroll
-    for (int y = 0; y < 8; y++) v = fmaxf(v, s_m[y][c & 7][c >> 3]);
-    const int col = blockIdx.x * kQTileCols + c;
-    if (col < q.N && v > 0.f) // the maxima start at 0
-        atomicMax(q.colmax + col, __float_as_uint(v));
-}
-
-// Bq[k, n] = E4M3(B[k, n] / s[n]) over the thread's rows and columns.
-__global__ void __launch_bounds__(256) k_quant_cols(const __grid_constant__ QBatch b)
-{
-    const QJob &q = b.job[blockIdx.z];
-    const QTile t = q_tile(q);
-    if (t.n >= q.N || t.k0 >= q.K)
-        return;
-    float s[8]; // reciprocals of the column scales (B is multiplied by them)
-#pragma unroll
-    for (int i = 0; i < 8; i++) s[i] = 1.f / (t.n + i < q.N ? scale_of(__uint_as_float(q.colmax[t.n + i])) : 1.f);
-    const bool st8 = (q.ldq & 7) == 0 && (reinterpret_cast<uintptr_t>(q.Bq) & 7u) == 0;
-    if (t.fast && st8) {
-        uint4 r[kQRows];
-        load_rows8(q, t, r);
-#pragma unroll
-        for (int j = 0; j < kQRows; j++) {
-            const __half2 *h = reinterpret_cast<const __half2 *>(&r[j]);
-            uint32_t w[2];
-#pragma unroll
-            for (int p = 0; p < 2; p++) {
-                const float2 f0 = __half22float2(h[2 * p]), f1 = __half22float2(h[2 * p + 1]);
-                const uint32_t q0 = __nv_cvt_float2_to_fp8x2(make_float2(f0.x * s[4 * p], f0.y * s[4 * p + 1]),
-                                                             __NV_SATFINITE, __NV_E4M3);
-                const uint32_t q1 = __nv_cvt_float2_to_fp8x2(make_float2(f1.x * s[4 * p + 2], f1.y * s[4 * p + 3]),
-                                                             __NV_SATFINITE, __NV_E4M3);
-                w[p] = (q0 & 0xffffu) | (q1 << 16);
-            }
-            *reinterpret_cast<uint2 *>(q.Bq + (size_t)(t.k0 + j) * q.ldq + t.n) = make_uint2(w[0], w[1]);
-        }
-        return;
-    }
-    const bool vec = vec8_ok(q);
-    for (int k = t.k0; k < t.k1; k++) {
-        float v[8];
-        load8h(q, k, t.n, vec, v);
-        uint32_t lo = 0, hi = 0;
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            lo |= (uint32_t)to_e4m3(v[i] * s[i]) << (8 * i);
-            hi |= (uint32_t)to_e4m3(v[4 + i] * s[4 + i]) << (8 * i);
-        }
-        uint8_t *dst = q.Bq + (size_t)k * q.ldq + t.n;
-        if (t.n + 8 <= q.N && (reinterpret_cast<uintptr_t>(dst) & 7u) == 0) {
-            *reinterpret_cast<uint2 *>(dst) = make_uint2(lo, hi);
-        } else {
-            for (int i = 0; t.n + i < q.N && i < 8; i++) dst[i] = (uint8_t)((i < 4 ? lo : hi) >> (8 * (i & 3)));
-        }
-    }
-}
-
-// The whole quantization of B in one launch: one block per (matrix, strip of
-// SW columns) reads the strip's K rows for the column maxima, reduces them
-// (warp shuffles, then the block's 8 warps), writes the scales and reads the
-// strip again (now from L2) to quantize it. Nothing is cleared beforehand
-// and no block depends on another. A thread takes 8 consecutive columns
-// (16 bytes) of every RPP-th row, four rows' loads in flight.
-template <int SW>
-__global__ void __launch_bounds__(256) k_quant_b_strip(const __grid_constant__ QBatch b)
-{
-    constexpr int TPR = SW / 8;    // threads per row
-    constexpr int RPP = 256 / TPR; // rows per pass
-    const QJob &q = b.job[blockIdx.y];
-    const int n0 = blockIdx.x * SW;
-    if (n0 >= q.N)
-        return; // whole block
-    __shared__ float s_m[8][SW];
-    __shared__ float s_scale[SW];
-    const int tx = threadIdx.x % TPR, ty = threadIdx.x / TPR;
-    const int n = n0 + tx * 8;
-    const bool vec = vec8_ok(q);
-    float m[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    if (n < q.N) {
-        for (int k = ty; k < q.K; k += 4 * RPP) {
-            float v[4][8];
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-                if (k + u * RPP < q.K)
-                    load8h(q, k + u * RPP, n, vec, v[u]);
-                else
-#pragma unroll
-                    for (int i = 0; i < 8; i++) v[u][i] = 0.f;
-            }
-#pragma unroll
-            for (int u = 0; u < 4; u++)
-#pragma unroll
-                for (int i = 0; i < 8; i++) m[i] = fmaxf(m[i], fabsf(v[u][i]));
-        }
-    }
-    // lanes of a warp with the same columns differ by multiples of TPR
-#pragma unroll
-    for (int o = TPR; o < 32; o <<= 1)
-#pragma unroll
-        for (int i = 0; i < 8; i++) m[i] = fmaxf(m[i], __shfl_xor_sync(0xffffffffu, m[i], o));
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (lane < TPR)
-#pragma unroll
-        for (int i = 0; i < 8; i++) s_m[warp][lane * 8 + i] = m[i];
-    __syncthreads();
-    if ((int)threadIdx.x < SW) {
-        float v = 0.f;
-#pragma unroll
-        for (int w = 0; w < 8; w++) v = fmaxf(v, s_m[w][threadIdx.x]);
-        const float sc = scale_of(v);
-        s_scale[threadIdx.x] = sc;
-        if (n0 + (int)threadIdx.x < q.N)
-            q.colmax[n0 + threadIdx.x] = __float_as_uint(sc);
-    }
-    __syncthreads();
-    if (n >= q.N)
-        return;
-    float sc[8]; // reciprocals of the column scales (B is multiplied by them)
-#pragma unroll
-    for (int i = 0; i < 8; i++) sc[i] = 1.f / s_scale[tx * 8 + i];
-    const bool st8 = n + 8 <= q.N && (q.ldq & 7) == 0 && (reinterpret_cast<uintptr_t>(q.Bq) & 7u) == 0;
-    for (int k = ty; k < q.K; k += 4 * RPP) {
-        float v[4][8];
-#pragma unroll
-        for (int u = 0; u < 4; u++)
-            if (k + u * RPP < q.K)
-                load8h(q, k + u * RPP, n, vec, v[u]);
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-            if (k + u * RPP >= q.K)
-                break;
-            uint32_t lo = 0, hi = 0;
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                lo |= (uint32_t)to_e4m3(v[u][i] * sc[i]) << (8 * i);
-                hi |= (uint32_t)to_e4m3(v[u][4 + i] * sc[4 + i]) << (8 * i);
-            }
-            uint8_t *dst = q.Bq + (size_t)(k + u * RPP) * q.ldq + n;
-            if (st8)
-                *reinterpret_cast<uint2 *>(dst) = make_uint2(lo, hi);
-            else
-                for (int i = 0; n + i < q.N && i < 8; i++) dst[i] = (uint8_t)((i < 4 ? lo : hi) >> (8 * (i & 3)));
-        }
-    }
 }
 
 // 8 halves of B row k from column n as raw FP16 bits (zeros past N).
@@ -359,44 +123,59 @@ __device__ __forceinline__ uint4 load8raw(const QJob &q, int k, int n, bool vec)
                       h[6] | (unsigned)h[7] << 16);
 }
 
-// k_quant_b_strip with the strip kept in shared memory (K x SW halves, when
-// that fits): every row of the strip is read from HBM once, with all of a
-// thread's loads (K / RPP of them, at most kQStripLoads) in flight together,
-// written to shared memory on arrival and folded into the column maxima; the
-// quantization then reads shared memory. One HBM round trip per block instead
-// of two passes of dependent loads (measured on the headline batch: 23 us for
-// the two-pass kernel under the profiler).
-constexpr int kQStripLoads = 8;             // rows a thread loads before the first use
-constexpr size_t kQStripSmem = 96 * 1024;     // largest strip kept in shared memory (two blocks per SM)
+// The quantization of B in one launch: a cluster of blocks per (matrix, strip
+// of 64 columns, or 16 or 8), the strip's K rows cut among the cluster's blocks. A block
+// reads its rows once (whole 128-byte lines, 8 of a thread's loads in flight),
+// keeps them in shared memory and folds them into column maxima; the cluster's
+// blocks read each other's maxima (distributed shared memory) and every block
+// quantizes its own rows from shared memory. HBM-bound in the limit (2 bytes
+// read and 1 written per element); at these sizes it is two dependent trips to
+// memory and a cluster barrier. It replaces four launches (clear, maxima with
+// atomics, quantize, scales; 4096 x 1024, issued one by one: 24 us from the
+// first to the last, now 7.7; as a graph 8.0, now 7.6) and, for batches, a
+// block per strip of 16 columns (32 matrices of 1024 x 256: 11.6 -> 10.0 us;
+// 1024 x 256 alone 6.7 -> 4.6). KEEP = false: the rows do not fit shared
+// memory (K > 100,000 for few columns) and are read again, from L2 for the
+// most part.
+constexpr int kQLoads = 8;                // rows a thread loads before the first use
+constexpr int kQMaxCluster = 8;
+constexpr size_t kQSmemTwo = 96 * 1024;   // two blocks per SM
+constexpr size_t kQSmemMax = 200 * 1024;
 
-template <int SW>
-__global__ void __launch_bounds__(256) k_quant_b_smem(const __grid_constant__ QBatch b)
+template <int kQCols, bool KEEP> // kQCols: columns per strip
+__global__ void __launch_bounds__(256, 4) k_quant_b(const __grid_constant__ QBatch b, int cluster)
 {
-    constexpr int TPR = SW / 8;
-    constexpr int RPP = 256 / TPR;
-    extern __shared__ uint4 s_strip[]; // [K][TPR]
-    __shared__ float s_m[8][SW];
-    __shared__ float s_scale[SW];
+    constexpr int kQRowThreads = kQCols / 8; // threads per row (8 columns each)
+    constexpr int kQRowsPerPass = 256 / kQRowThreads;
+    extern __shared__ uint4 s_rows[]; // KEEP: [rows of the block][kQRowThreads]
+    __shared__ float s_m[8][kQCols];
+    __shared__ float s_max[kQCols]; // this block's maxima, read by the cluster
+    __shared__ float s_scale[kQCols];
+    // the forward that follows may take its place on SMs that are done here;
+    // it waits for this grid's end before it reads anything
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const QJob &q = b.job[blockIdx.y];
-    const int n0 = blockIdx.x * SW;
+    const int strip = (int)blockIdx.x / cluster, rank = (int)blockIdx.x - strip * cluster;
+    const int n0 = strip * kQCols;
     if (n0 >= q.N)
-        return; // whole block
-    const int tx = threadIdx.x % TPR, ty = threadIdx.x / TPR;
+        return; // the whole cluster
+    const int k_begin = (int)((long long)q.K * rank / cluster), k_end = (int)((long long)q.K * (rank + 1) / cluster);
+    const int tx = threadIdx.x % kQRowThreads, ty = threadIdx.x / kQRowThreads;
     const int n = n0 + tx * 8;
     const bool vec = vec8_ok(q);
     float m[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int k0 = ty; k0 < q.K; k0 += kQStripLoads * RPP) {
-        uint4 r[kQStripLoads];
+    for (int k0 = k_begin + ty; k0 < k_end; k0 += kQLoads * kQRowsPerPass) {
+        uint4 r[kQLoads];
 #pragma unroll
-        for (int u = 0; u < kQStripLoads; u++) {
-            const int k = k0 + u * RPP;
-            r[u] = (k < q.K && n < q.N) ? load8raw(q, k, n, vec) : make_uint4(0, 0, 0, 0);
+        for (int u = 0; u < kQLoads; u++) {
+            const int k = k0 + u * kQRowsPerPass;
+            r[u] = (k < k_end && n < q.N) ? load8raw(q, k, n, vec) : make_uint4(0, 0, 0, 0);
         }
 #pragma unroll
-        for (int u = 0; u < kQStripLoads; u++) {
-            const int k = k0 + u * RPP;
-            if (k < q.K)
-                s_strip[k * TPR + tx] = r[u];
+        for (int u = 0; u < kQLoads; u++) {
+            const int k = k0 + u * kQRowsPerPass;
+            if (KEEP && k < k_end)
+                s_rows[(k - k_begin) * kQRowThreads + tx] = r[u];
             const __half2 *h = reinterpret_cast<const __half2 *>(&r[u]);
 #pragma unroll
             for (int i = 0; i < 4; i++) {
@@ -406,33 +185,42 @@ __global__ void __launch_bounds__(256) k_quant_b_smem(const __grid_constant__ QB
             }
         }
     }
+    // lanes of a warp with the same columns differ by multiples of kQRowThreads
 #pragma unroll
-    for (int o = TPR; o < 32; o <<= 1)
+    for (int o = kQRowThreads; o < 32; o <<= 1)
 #pragma unroll
         for (int i = 0; i < 8; i++) m[i] = fmaxf(m[i], __shfl_xor_sync(0xffffffffu, m[i], o));
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (lane < TPR)
+    if (lane < kQRowThreads)
 #pragma unroll
         for (int i = 0; i < 8; i++) s_m[warp][lane * 8 + i] = m[i];
-    __syncthreads(); // also: the whole strip is in shared memory
-    if ((int)threadIdx.x < SW) {
+    __syncthreads();
+    if ((int)threadIdx.x < kQCols) {
         float v = 0.f;
 #pragma unroll
         for (int w = 0; w < 8; w++) v = fmaxf(v, s_m[w][threadIdx.x]);
+        s_max[threadIdx.x] = v;
+    }
+    ptx::cluster_sync_all(); // (a cluster of one: a block barrier)
+    if ((int)threadIdx.x < kQCols) {
+        float v = 0.f;
+        for (int r = 0; r < cluster; r++)
+            v = fmaxf(v, ptx::ld_cluster_f32(ptx::cluster_map(ptx::smem_u32(&s_max[threadIdx.x]), (uint32_t)r)));
         const float sc = scale_of(v);
         s_scale[threadIdx.x] = sc;
-        if (n0 + (int)threadIdx.x < q.N)
+        if (rank == 0 && n0 + (int)threadIdx.x < q.N)
             q.colmax[n0 + threadIdx.x] = __float_as_uint(sc);
     }
-    __syncthreads();
+    ptx::cluster_sync_all(); // the scales are there; no block of the cluster reads another's maxima any more
     if (n >= q.N)
         return;
     float sc[8]; // reciprocals of the column scales (B is multiplied by them)
 #pragma unroll
     for (int i = 0; i < 8; i++) sc[i] = 1.f / s_scale[tx * 8 + i];
     const bool st8 = n + 8 <= q.N && (q.ldq & 7) == 0 && (reinterpret_cast<uintptr_t>(q.Bq) & 7u) == 0;
-    for (int k = ty; k < q.K; k += RPP) {
-        const uint4 r = s_strip[k * TPR + tx];
+#pragma unroll 4
+    for (int k = k_begin + ty; k < k_end; k += kQRowsPerPass) {
+        const uint4 r = KEEP ? s_rows[(k - k_begin) * kQRowThreads + tx] : load8raw(q, k, n, vec);
         const __half2 *h = reinterpret_cast<const __half2 *>(&r);
         uint32_t w[2];
 #pragma unroll
@@ -452,14 +240,6 @@ __global__ void __launch_bounds__(256) k_quant_b_smem(const __grid_constant__ QB
     }
 }
 
-// column maxima -> scales, in place
-__global__ void k_col_scale(const __grid_constant__ QBatch b)
-{
-    const QJob &q = b.job[blockIdx.z];
-    for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < q.N; n += gridDim.x * blockDim.x)
-        q.colmax[n] = __float_as_uint(scale_of(__uint_as_float(q.colmax[n])));
-}
-
 unsigned blocks(long long n, int per) { return (unsigned)((n + per - 1) / per); }
 
 int quantize_b_batch(const QBatch &b, cudaStream_t s)
@@ -471,47 +251,41 @@ int quantize_b_batch(const QBatch &b, cudaStream_t s)
     }
     if (b.n == 0 || maxK == 0 || maxN == 0)
         return TCA_OK;
-    const unsigned z = (unsigned)b.n;
-    // One launch, a block per column strip (k_quant_b_strip), when the strips
-    // give about two blocks per SM; else (few, wide matrices) the column
-    // maxima of 64-row tiles with one atomic per column and block, then the
-    // quantization and the scales, in four launches.
-    auto strips = [&](int sw) { return (long long)b.n * blocks(maxN, sw); };
-    if (strips(8) >= kSMs) {
-        const int sw = strips(64) >= 2 * kSMs ? 64 : strips(32) >= 2 * kSMs ? 32 : strips(16) >= 2 * kSMs ? 16 : 8;
-        const dim3 grid(blocks(maxN, sw), z);
-        const size_t strip_bytes = (size_t)maxK * sw * 2;
-        if (strip_bytes <= kQStripSmem) {
-            auto launch = [&](auto kernel) -> int {
-                TCA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kQStripSmem));
-                kernel<<<grid, 256, strip_bytes, s>>>(b);
-                TCA_CUDA_TRY(cudaGetLastError());
-                return TCA_OK;
-            };
-            switch (sw) {
-            case 64: return launch(k_quant_b_smem<64>);
-            case 32: return launch(k_quant_b_smem<32>);
-            case 16: return launch(k_quant_b_smem<16>);
-            default: return launch(k_quant_b_smem<8>);
-            }
-        }
-        switch (sw) {
-        case 64: k_quant_b_strip<64><<<grid, 256, 0, s>>>(b); break;
-        case 32: k_quant_b_strip<32><<<grid, 256, 0, s>>>(b); break;
-        case 16: k_quant_b_strip<16><<<grid, 256, 0, s>>>(b); break;
-        default: k_quant_b_strip<8><<<grid, 256, 0, s>>>(b); break;
-        }
-        TCA_CUDA_TRY(cudaGetLastError());
-        return TCA_OK;
-    }
-    const dim3 tiles(blocks(maxN, kQTileCols), blocks(maxK, kQTileRows), z), tile_threads(32, 8);
-    if (tiles.y > 65535u)
+    if (b.n * blocks(maxN, 8) < (unsigned)kSMs && blocks(maxK, 64) > 65535u)
         return set_error(TCA_ERR_INVALID_ARG, "B has too many rows to quantize (K=%d)", maxK);
-    k_col_zero<<<dim3(blocks(maxN, 256), 1, z), 256, 0, s>>>(b);
-    k_col_absmax<<<tiles, tile_threads, 0, s>>>(b);
-    k_quant_cols<<<tiles, tile_threads, 0, s>>>(b);
-    k_col_scale<<<dim3(blocks(maxN, 256), 1, z), 256, 0, s>>>(b);
-    TCA_CUDA_TRY(cudaGetLastError());
+    // Blocks per strip: doubled while there are fewer than two blocks per SM
+    // and each keeps 64 rows, and until two blocks' rows fit an SM.
+    // Narrower strips where full clusters of wider ones leave half of the SMs
+    // without a block and each has more than 512 rows (20,000 x 128: 31 us with
+    // 64 columns, 9.0 with 16, 12.7 with 8; 60,000 x 64: 26.9 with 16, 13.9 with 8).
+    int cols = 64;
+    if (2LL * b.n * blocks(maxN, 64) * kQMaxCluster <= kSMs && maxK > 512 * kQMaxCluster)
+        cols = 4LL * b.n * blocks(maxN, 16) * kQMaxCluster > kSMs ? 16 : 8;
+    const long long strips = (long long)b.n * blocks(maxN, cols);
+    auto bytes = [&](int c) { return (size_t)((maxK + c - 1) / c) * cols * sizeof(__half); };
+    int cluster = 1;
+    while (cluster < kQMaxCluster &&
+           ((strips * cluster < 2 * kSMs && maxK / (2 * cluster) >= 64) || bytes(cluster) > kQSmemTwo))
+        cluster *= 2;
+    const bool keep = bytes(cluster) <= kQSmemMax;
+    auto kernel = cols == 64 ? (keep ? k_quant_b<64, true> : k_quant_b<64, false>)
+                : cols == 16 ? (keep ? k_quant_b<16, true> : k_quant_b<16, false>)
+                             : (keep ? k_quant_b<8, true> : k_quant_b<8, false>);
+    if (keep)
+        TCA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kQSmemMax));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks(maxN, cols) * (unsigned)cluster, (unsigned)b.n);
+    cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = keep ? bytes(cluster) : 0;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)cluster;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    TCA_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, b, cluster));
     return TCA_OK;
 }
 

@@ -583,8 +583,8 @@ __global__ void k_update_p_val(const int *__restrict__ src, const __half *__rest
 // (whose zeros stay where they are). It was seven launches (values, entries,
 // images of both plans, the transpose's gather) of 2-3 us each, the images
 // re-rendered; what bounds it now is the chain of index loads per value.
-// 2048 x 512 at 90 % with its transpose 13.9 -> UPD_A us, 4096 x 4096 at 90 %
-// 61.5 -> UPD_B us.
+// 2048 x 512 at 90 % with its transpose 13.9 -> 5.3 us, 4096 x 4096 at 90 %
+// 61.5 -> 43 us.
 struct ValueJob {
     const int *src;  // position in sorted order -> nonzero (of the transpose: entry of t_src)
     const int *via;  // the transpose: entry -> caller's nonzero; NULL: src is that already
@@ -1130,7 +1130,7 @@ int run_jobs_with_events(const SpmmJob *jobs, int n_jobs, int c_dtype, float alp
     // programmatic dependents and run beside it; with events (which time each
     // path alone) the two run one after the other.
     LaunchList tc, cc;
-    TCA_TRY(launch_tc_jobs(jobs, n_jobs, c_dtype, alpha, beta, flags, s, &tc));
+    TCA_TRY(launch_tc_jobs(jobs, n_jobs, c_dtype, alpha, beta, flags, s, &tc, !events));
     int beside = 0;
     for (int i = 0; !events && !tc.empty() && i < n_jobs; i++) {
         int r = 0;

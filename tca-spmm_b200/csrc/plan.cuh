@@ -160,9 +160,11 @@ using LaunchList = std::vector<std::function<int(cudaStream_t)>>;
 
 // Tensor-core (tcgen05) forward over the tensor-core windows of every job
 // (jobs with tc set), in as few launches as the N-slice widths allow. With
-// `defer` the prepared launches are appended to it instead of issued.
+// `defer` the prepared launches are appended to it instead of issued. With
+// `dependent` the E4M3 launches are programmatic dependents of the kernel
+// before them on the stream (B's quantization): their set-up runs while it ends.
 int launch_tc_jobs(const SpmmJob *jobs, int n_jobs, int c_dtype, float alpha, float beta, unsigned flags,
-                   cudaStream_t s, LaunchList *defer = nullptr);
+                   cudaStream_t s, LaunchList *defer = nullptr, bool dependent = false);
 
 // Registers that one block of the tensor-core kernel holds on an SM (the
 // largest over its FP16 or its E4M3 instantiations).

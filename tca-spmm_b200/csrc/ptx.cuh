@@ -94,6 +94,12 @@ __device__ __forceinline__ uint32_t cluster_map(uint32_t local, uint32_t rank)
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"(rank));
     return r;
 }
+__device__ __forceinline__ float ld_cluster_f32(uint32_t cluster_addr)
+{
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(cluster_addr) : "memory");
+    return v;
+}
 // Arrive (count 1) on an mbarrier of a CTA in the cluster, releasing this
 // thread's prior writes at cluster scope.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr)

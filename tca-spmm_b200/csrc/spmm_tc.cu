@@ -346,7 +346,10 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
     // A CUDA-core launch that follows on the stream as a programmatic
     // dependent may start as soon as every block of this grid is resident: it
     // reads nothing this kernel writes (the two paths own disjoint rows of C).
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // E4M3: both read what the quantization before them writes, so the trigger
+    // comes after this grid's own wait for it, below.
+    if constexpr (!F8)
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int total = batch.item_start[batch.n_jobs];
@@ -426,6 +429,10 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    if constexpr (F8) {
+        asm volatile("griddepcontrol.wait;" ::: "memory"); // B is quantized
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    }
     bool ok = true;
     const int total_chunks = cum[n_items]; // of this CTA's items: every role runs over exactly these
 
@@ -1329,7 +1336,7 @@ int make_job(const SpmmJob &sj, float alpha, float beta, unsigned flags, int NT,
 }
 
 template <int NT, typename OutT, bool F8, int CAP>
-int launch_group_cap(const TcBatchT<CAP> &b, cudaStream_t s)
+int launch_group_cap(const TcBatchT<CAP> &b, bool dependent, cudaStream_t s)
 {
     const int smem = TcCfg<NT, F8>::kSmem;
     TCA_CUDA_TRY(cudaFuncSetAttribute(spmm_tc_kernel<NT, OutT, F8, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1344,13 +1351,22 @@ int launch_group_cap(const TcBatchT<CAP> &b, cudaStream_t s)
                                       (int)cudaSharedmemCarveoutMaxShared));
     const int total = b.item_start[b.n_jobs];
     const int grid = std::min(total, std::max(kSMs, (total + kMaxCtaItems - 1) / kMaxCtaItems));
-    spmm_tc_kernel<NT, OutT, F8, CAP><<<grid, kThreads, smem, s>>>(b);
-    TCA_CUDA_TRY(cudaGetLastError());
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = F8 && dependent ? 1 : 0;
+    TCA_CUDA_TRY(cudaLaunchKernelEx(&cfg, spmm_tc_kernel<NT, OutT, F8, CAP>, b));
     return TCA_OK;
 }
 
 template <int NT, typename OutT, bool F8>
-int launch_group(const TcBatch &b, cudaStream_t s)
+int launch_group(const TcBatch &b, bool dependent, cudaStream_t s)
 {
     if (b.n_jobs == 1) {
         TcBatchT<1> one;
@@ -1358,20 +1374,20 @@ int launch_group(const TcBatch &b, cudaStream_t s)
         one.item_start[0] = b.item_start[0];
         one.item_start[1] = b.item_start[1];
         one.job[0] = b.job[0];
-        return launch_group_cap<NT, OutT, F8, 1>(one, s);
+        return launch_group_cap<NT, OutT, F8, 1>(one, dependent, s);
     }
-    return launch_group_cap<NT, OutT, F8, kMaxJobs>(b, s);
+    return launch_group_cap<NT, OutT, F8, kMaxJobs>(b, dependent, s);
 }
 
 template <typename OutT>
-int launch_group_out(const TcBatch &b, int NT, bool f8, cudaStream_t s)
+int launch_group_out(const TcBatch &b, int NT, bool f8, bool dependent, cudaStream_t s)
 {
     if (f8)
-        return NT == 128 ? launch_group<128, OutT, true>(b, s) : launch_group<256, OutT, true>(b, s);
+        return NT == 128 ? launch_group<128, OutT, true>(b, dependent, s) : launch_group<256, OutT, true>(b, dependent, s);
     switch (NT) {
-    case 64: return launch_group<64, OutT, false>(b, s);
-    case 128: return launch_group<128, OutT, false>(b, s);
-    default: return launch_group<256, OutT, false>(b, s);
+    case 64: return launch_group<64, OutT, false>(b, dependent, s);
+    case 128: return launch_group<128, OutT, false>(b, dependent, s);
+    default: return launch_group<256, OutT, false>(b, dependent, s);
     }
 }
 
@@ -1422,11 +1438,12 @@ int launch_pair_typed(const TcBatch &b, bool f8, int c_dtype, cudaStream_t s)
     return f8 ? launch_pair_group<float, true>(b, s) : launch_pair_group<float, false>(b, s);
 }
 
-int launch_group_typed(const TcBatch &b, int NT, bool f8, int c_dtype, cudaStream_t s)
+int launch_group_typed(const TcBatch &b, int NT, bool f8, int c_dtype, bool dependent, cudaStream_t s)
 {
     if (b.n_jobs == 0 || b.item_start[b.n_jobs] == 0)
         return TCA_OK;
-    return c_dtype == TCA_DTYPE_F16 ? launch_group_out<__half>(b, NT, f8, s) : launch_group_out<float>(b, NT, f8, s);
+    return c_dtype == TCA_DTYPE_F16 ? launch_group_out<__half>(b, NT, f8, dependent, s)
+                                    : launch_group_out<float>(b, NT, f8, dependent, s);
 }
 
 } // namespace
@@ -1492,15 +1509,16 @@ bool pair_eligible(const tca_plan *p, int NT)
 }
 
 int launch_tc_jobs(const SpmmJob *jobs, int n_jobs, int c_dtype, float alpha, float beta, unsigned flags,
-                   cudaStream_t s, LaunchList *defer)
+                   cudaStream_t s, LaunchList *defer, bool dependent)
 {
     // widths of the single-window kernel, then (0) the pair kernel for N-slices of 256
     const int widths[4] = {64, 128, 256, 0};
     auto emit = [&](const TcBatch &b, int NT, bool f8) -> int {
         if (b.n_jobs == 0 || b.item_start[b.n_jobs] == 0)
             return TCA_OK;
-        auto run = [NT, f8, c_dtype](const TcBatch &bb, cudaStream_t st) {
-            return NT == 0 ? launch_pair_typed(bb, f8, c_dtype, st) : launch_group_typed(bb, NT, f8, c_dtype, st);
+        auto run = [NT, f8, c_dtype, dependent](const TcBatch &bb, cudaStream_t st) {
+            return NT == 0 ? launch_pair_typed(bb, f8, c_dtype, st)
+                           : launch_group_typed(bb, NT, f8, c_dtype, dependent, st);
         };
         if (!defer)
             return run(b, s);
