@@ -191,11 +191,16 @@ template <int NT, bool F8> struct TcCfg {
 template <typename Batch>
 __device__ __forceinline__ int4 decode_item(const Batch &batch, int item)
 {
-    int j = 0;
-    while (j + 1 < batch.n_jobs && batch.item_start[j + 1] <= item) j++;
+    int j = 0, hi = batch.n_jobs - 1; // the last job whose first item is <= item
+    while (j < hi) {
+        const int mid = (j + hi + 1) >> 1;
+        if (batch.item_start[mid] <= item) j = mid;
+        else hi = mid - 1;
+    }
     const TcJob &a = batch.job[j];
+    prefetch_tensormap(&a.tmap_tile);
     const int local = item - batch.item_start[j];
-    const int4 wi = a.win_info[local / a.ntiles];
+    const int4 wi = __ldg(a.win_info + local / a.ntiles);
     return make_int4(wi.x, wi.y, wi.z, (j << 16) | (local % a.ntiles));
 }
 
@@ -387,8 +392,12 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
             }
         }
     };
-    if (warp == kBLoaderWarp) {
-        // the item table and the first chunk of each item (a warp scan of the chunk counts)
+    if (warp == kBLoaderWarp || warp == kALoaderWarp) {
+        // The item table and the first chunk of each item (a warp scan of the
+        // chunk counts), by both loaders alike -- the same values to the same
+        // places --, so that each can go on to its first records' loads, on
+        // their way during the rest of the set-up (a chain of cold misses:
+        // parameters, window list, chunk lists, then the data).
         int z = 0;
         if (lane < n_items) {
             const int4 it = decode_item(batch, blockIdx.x + lane * gridDim.x);
@@ -404,9 +413,7 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
         cum[lane + 1] = sum;
         if (lane == 0) cum[0] = 0;
         __syncwarp();
-        fetch(lane, 0); // the first records' loads, on their way during the rest of the set-up
-        if (lane < n_items)
-            prefetch_tensormap(&batch.job[items[lane].w >> 16].tmap_tile);
+        fetch(lane, 0);
     } else if (warp == kMmaWarp) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
                      "r"(2 * NT)
@@ -562,7 +569,6 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
                 }
             }
         };
-        fetch(lane, 0);
         make_records(0);
         // one lane walks the chunks; every lane joins it to make the next records
         const bool leader = elect_one();
@@ -664,14 +670,23 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
             __syncwarp();
             const uint32_t *st = reinterpret_cast<const uint32_t *>(smem + Cfg::kStagingOff + slot * kStagingBytes);
             const int end = (pd.y >> 2) + (pd.y & 3);
-#pragma unroll 4
-            for (int e = (pd.y & 3) + lane; e < end; e += 32) {
-                const uint32_t v = st[e];
-                if constexpr (F8)
-                    At[swz64_offset(v >> 22, (v >> 16) & 63u)] = (uint8_t)(v & 0xffu);
-                else
-                    *reinterpret_cast<uint16_t *>(At + swz128_offset(v >> 22, (v >> 16) & 63u)) =
-                        (uint16_t)(v & 0xffffu);
+            // eight loads before the first store: the compiler may not move a
+            // shared load over a shared store, and one entry at a time is a
+            // chain of ~100 cycles
+            for (int e = (pd.y & 3) + lane; e < end; e += 8 * 32) {
+                uint32_t v[8];
+#pragma unroll
+                for (int u = 0; u < 8; u++) v[u] = e + u * 32 < end ? st[e + u * 32] : 0xffffffffu; // row 1023: none
+#pragma unroll
+                for (int u = 0; u < 8; u++) {
+                    if (v[u] == 0xffffffffu)
+                        continue;
+                    if constexpr (F8)
+                        At[swz64_offset(v[u] >> 22, (v[u] >> 16) & 63u)] = (uint8_t)(v[u] & 0xffu);
+                    else
+                        *reinterpret_cast<uint16_t *>(At + swz128_offset(v[u] >> 22, (v[u] >> 16) & 63u)) =
+                            (uint16_t)(v[u] & 0xffffu);
+                }
             }
             fence_proxy_async();
             __syncwarp();
