@@ -46,6 +46,7 @@
 #include <algorithm>
 #include <memory>
 #include <mutex>
+#include <vector>
 #include "tca_internal.cuh"
 #include "plan.cuh"
 #include "ptx.cuh"
@@ -82,6 +83,7 @@ struct TcJob {
     void *C;
     int *status;
     int M, N, ldb, ldc, ntiles;
+    int nt;                  // width of its N-slices, at most the kernel's
     int tile3d;              // tmap_tile covers the whole NT-wide slice in one box
     float alpha, beta;
     unsigned flags;
@@ -210,10 +212,12 @@ struct __align__(16) TcRecordA {
     int bytes;       // of src: kATileBytes for an image, fewer for entries
     int ent;         // entries: count << 2 | entries before the first one
 };
+constexpr int kSlabBits = 26;
+constexpr uint32_t kSlabMask = (1u << kSlabBits) - 1u;
 struct __align__(16) TcRecordB {
     const void *b; // tensor map; condensed columns: the column list
     int col0;      // first of 64 consecutive columns; condensed columns: -1 - item
-    int x;         // n0 (2-D boxes) or, with the top bit, the 64-column slab of n0 (3-D box)
+    uint32_t x;    // 128-byte slab of n0 | slabs of the slice << kSlabBits | top bit: one 3-D box
 };
 
 // 16-byte unit u of an output row: alpha x 8 accumulators as FP16, or 4 as FP32.
@@ -306,6 +310,8 @@ __device__ __forceinline__ void store_rows(uint32_t acc, OutT *C, int ldc, int o
 //     the release of a sparse chunk to the scatter warps ("staged"), whose
 //     entries were sent for kAhead chunks before (cp.async.bulk into a
 //     staging slot, completing on its "staged").
+//     Jobs of narrower N-slices than the kernel's run in the same launch
+//     (smaller boxes, narrower MMAs).
 //   warp 2, one lane (MMA): per chunk wait "full"; on an item's first chunk
 //     wait until its TMEM accumulator buffer (item parity) is drained
 //     ("accum_empty"); 4 x tcgen05.mma (2 for E4M3); commit "empty"; on the
@@ -332,8 +338,6 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
     using Cfg = TcCfg<NT, F8>;
     constexpr int S = Cfg::kStages;
     constexpr int kATileBytes = Cfg::kATileBytes;
-    constexpr int kBoxes = NT / Cfg::kBoxCols; // 128-byte-wide boxes per B row slice
-    constexpr int kGathers = 16 * kBoxes;      // gather4 instructions per condensed chunk
     extern __shared__ __align__(1024) uint8_t smem[];
     int2 *pend = reinterpret_cast<int2 *>(smem + Cfg::kPendOff);
     TcRecordA *rec_a = reinterpret_cast<TcRecordA *>(smem + Cfg::kRecOff);
@@ -359,6 +363,8 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int total = batch.item_start[batch.n_jobs];
     const int n_items = blockIdx.x < total ? min(kMaxCtaItems, (total - 1 - (int)blockIdx.x) / (int)gridDim.x + 1) : 0;
+    // a job's N-slice width: a single forward runs in the kernel of its own width
+    auto width = [](const TcJob &a) { return CAP == 1 ? NT : a.nt; };
     if (smem_u32(smem) & 1023u) { // the swizzled tiles and TMA destinations need a 1024-byte aligned base
         if (threadIdx.x == 0 && n_items > 0)
             atomicOr(batch.job[0].status, kStatusLayout);
@@ -451,26 +457,28 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
                 const int4 it = items[k];
                 const TcJob &a = batch.job[it.w >> 16];
                 TcRecordB r;
-                const int n0 = (it.w & 0xffff) * NT;
+                const int n0 = (it.w & 0xffff) * width(a);
                 const bool direct = m0 >= 0 && m1 == m0 + kChunkCols - 1;
                 r.b = direct ? (const void *)&a.tmap_tile : (const void *)(a.win_cols + (size_t)c * kChunkCols);
                 r.col0 = direct ? m0 : -1 - k;
-                r.x = a.tile3d ? (int)0x80000000 | (n0 / Cfg::kBoxCols) : n0;
+                r.x = (uint32_t)(n0 / Cfg::kBoxCols) | (uint32_t)(width(a) / Cfg::kBoxCols) << kSlabBits |
+                      (a.tile3d ? 0x80000000u : 0u);
                 rec_b[(g0 + lane) % kRecords] = r;
             }
             fetch(g0 + 32 + lane, __shfl_sync(0xffffffffu, k, 31));
             __syncwarp();
         };
+        auto boxes = [](const TcRecordB &r) { return CAP == 1 ? NT / Cfg::kBoxCols : (int)(r.x >> kSlabBits & 7u); }; // 128-byte-wide ones of its slice
         // a direct chunk's B rows into stage s
         auto issue_boxes = [&](const TcRecordB &r, int s) {
             const uint32_t b_s = smem_u32(smem + s * Cfg::kStage) + kATileBytes;
             const CUtensorMap *map = static_cast<const CUtensorMap *>(r.b);
-            if (r.x < 0) {
-                tma_tile3d(b_s, map, 0, r.col0, r.x & 0x7fffffff, &full[s]);
+            const int slab = (int)(r.x & kSlabMask);
+            if (r.x >> 31) {
+                tma_tile3d(b_s, map, 0, r.col0, slab, &full[s]);
             } else {
-#pragma unroll
-                for (int bx = 0; bx < kBoxes; bx++)
-                    tma_tile2d(b_s + bx * (kChunkCols * 128), map, r.x + bx * Cfg::kBoxCols, r.col0, &full[s]);
+                for (int bx = 0; bx < boxes(r); bx++)
+                    tma_tile2d(b_s + bx * (kChunkCols * 128), map, (slab + bx) * Cfg::kBoxCols, r.col0, &full[s]);
             }
         };
         int s = 0;
@@ -487,7 +495,7 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
                     for (int h = g; h < ge; h++) {
                         const TcRecordB nxt = rec_b[(h + 1) % kRecords];
                         if (!mbar_wait(&empty[s1], phase1)) { ok = false; break; }
-                        mbar_arrive_expect_tx(&full[s1], Cfg::kBTileBytes);
+                        mbar_arrive_expect_tx(&full[s1], (uint32_t)boxes(r) * (kChunkCols * 128));
                         issue_boxes(r, s1);
                         if (++s1 == S) { s1 = 0; phase1 ^= 1; }
                         r = nxt;
@@ -505,7 +513,7 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
                     if (elect_one()) {
                         ok = mbar_wait(&empty[s1], phase1);
                         if (ok) {
-                            mbar_arrive_expect_tx(&full[s1], Cfg::kBTileBytes);
+                            mbar_arrive_expect_tx(&full[s1], (uint32_t)boxes(r) * (kChunkCols * 128));
                             if (r.col0 >= 0)
                                 issue_boxes(r, s1);
                         }
@@ -516,12 +524,12 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
                         const int4 it = items[-1 - r.col0];
                         const TcJob &a = batch.job[it.w >> 16];
                         const uint32_t b_s = smem_u32(smem + s1 * Cfg::kStage) + kATileBytes;
-                        const int src = lane & 15, n0 = (it.w & 0xffff) * NT;
+                        const int src = lane & 15, n0 = (int)(r.x & kSlabMask) * Cfg::kBoxCols;
                         const int y0 = __shfl_sync(0xffffffffu, ncols.x, src);
                         const int y1 = __shfl_sync(0xffffffffu, ncols.y, src);
                         const int y2 = __shfl_sync(0xffffffffu, ncols.z, src);
                         const int y3 = __shfl_sync(0xffffffffu, ncols.w, src);
-                        for (int p = lane; p < kGathers; p += 32) {
+                        for (int p = lane; p < 16 * boxes(r); p += 32) {
                             const int bx = p >> 4;
                             tma_gather4(b_s + bx * (kChunkCols * 128) + src * 512, &a.tmap_b, n0 + bx * Cfg::kBoxCols,
                                         y0, y1, y2, y3, &full[s1]);
@@ -602,8 +610,7 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
     } else if (warp == kMmaWarp) {
         // ---------------- MMA issuer ----------------
         if (elect_one()) {
-            constexpr uint32_t idesc = idesc_f16(NT); // E4M3 has format code 0 in kind::f8f6f4 as FP16 in kind::f16
-            // test hook: the CTA's last accumulator is never announced, so the
+                        // test hook: the CTA's last accumulator is never announced, so the
             // epilogue's bounded wait for it runs out (TCA_FLAG_TEST_WITHHOLD_ACCUM)
             const bool withhold = (batch.job[0].flags & TCA_FLAG_TEST_WITHHOLD_ACCUM) != 0;
             int s = 0;
@@ -611,6 +618,8 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
             for (int k = 0; k < n_items && ok; k++) {
                 const int b = k & 1;
                 const uint32_t d = tmem + (uint32_t)(b * NT);
+                // E4M3 has format code 0 in kind::f8f6f4 as FP16 in kind::f16
+                const uint32_t idesc = idesc_f16(width(batch.job[items[k].w >> 16]));
                 if (k >= 2 && !mbar_wait(&acc_empty[b], ((k >> 1) - 1) & 1)) { ok = false; break; }
                 uint32_t accum = 0;
                 for (int i = items[k].z; i > 0; i--) {
@@ -699,7 +708,7 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
         for (int k = 0; k < n_items; k++) {
             const int4 it = items[k];
             const TcJob &a = batch.job[it.w >> 16];
-            const int n0 = (it.w & 0xffff) * NT;
+            const int nt = width(a), n0 = (it.w & 0xffff) * nt, n_end = min(a.N, n0 + nt);
             const int i = it.x * kWindowRows + quarter * 32 + lane;
             int out_row = -1;
             if (i < a.M && !((a.flags & TCA_FLAG_KEEP_EMPTY_ROWS) && a.p_row_ptr[i + 1] == a.p_row_ptr[i]))
@@ -710,7 +719,7 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
                 // was last read for item k - 2, which every epilogue thread
                 // finished before the barrier of item k - 1)
                 float *sc = reinterpret_cast<float *>(smem + Cfg::kScaleOff) + b * NT;
-                for (int c = quarter * 32 + lane; c < NT; c += kEpiThreads)
+                for (int c = quarter * 32 + lane; c < nt; c += kEpiThreads)
                     sc[c] = n0 + c < a.N ? __ldg(a.col_scale + n0 + c) : 0.f;
             }
             uint32_t got = 0;
@@ -727,11 +736,11 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
             const float *sb0 = reinterpret_cast<const float *>(smem + Cfg::kScaleOff) + b * NT;
             const uint32_t acc = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * NT);
             if (a.beta == 0.f)
-                store_rows<NT, OutT, F8>(acc, reinterpret_cast<OutT *>(a.C), a.ldc, out_row, n0, a.N, a.alpha, sa, sb0,
+                store_rows<NT, OutT, F8>(acc, reinterpret_cast<OutT *>(a.C), a.ldc, out_row, n0, n_end, a.alpha, sa, sb0,
                                          lane);
             for (int cb = 0; a.beta != 0.f && cb < NT / 16; cb++) {
                 const int n = n0 + cb * 16;
-                if (n >= a.N)
+                if (n >= n_end)
                     break; // uniform across the warp
                 uint32_t r[16];
                 tmem_ld16(acc + (uint32_t)(cb * 16), r);
@@ -743,7 +752,7 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
                 }
                 if (Crow) {
                     store8_out(Crow + n, reinterpret_cast<const float *>(r), a.alpha, a.beta);
-                    if (n + 8 < a.N)
+                    if (n + 8 < n_end)
                         store8_out(Crow + n + 8, reinterpret_cast<const float *>(r) + 8, a.alpha, a.beta);
                 }
             }
@@ -1343,6 +1352,7 @@ int make_job(const SpmmJob &sj, float alpha, float beta, unsigned flags, int NT,
     j.N = sj.N;
     j.ldb = sj.ldb;
     j.ldc = sj.ldc;
+    j.nt = NT;
     j.ntiles = (sj.N + NT - 1) / NT;
     j.alpha = alpha;
     j.beta = beta;
@@ -1526,8 +1536,6 @@ bool pair_eligible(const tca_plan *p, int NT)
 int launch_tc_jobs(const SpmmJob *jobs, int n_jobs, int c_dtype, float alpha, float beta, unsigned flags,
                    cudaStream_t s, LaunchList *defer, bool dependent)
 {
-    // widths of the single-window kernel, then (0) the pair kernel for N-slices of 256
-    const int widths[4] = {64, 128, 256, 0};
     auto emit = [&](const TcBatch &b, int NT, bool f8) -> int {
         if (b.n_jobs == 0 || b.item_start[b.n_jobs] == 0)
             return TCA_OK;
@@ -1541,28 +1549,39 @@ int launch_tc_jobs(const SpmmJob *jobs, int n_jobs, int c_dtype, float alpha, fl
         defer->push_back([held, run](cudaStream_t st) { return run(*held, st); });
         return TCA_OK;
     };
+    // All jobs of a precision in one launch, as wide as their widest N-slice:
+    // launches run one after the other, each with its own set-up and its own
+    // partly filled last round (24 layers with N of 64 to 1024: three launches
+    // 73.9 us, one 43.5 us). Jobs with more chunks per item first: rounds of
+    // equal items, the short ones last, to fill the CTAs evenly.
+    auto cost = [](const SpmmJob &j) { // of one item: chunks, weighted by the width of the slice
+        return (long long)(j.p->n_tc_chunks / std::max(1, j.p->n_tc)) * (j.n_tile + 128);
+    };
     for (bool f8 : {false, true}) {
-        for (int NT : widths) {
-            TcBatch b;
-            b.n_jobs = 0;
-            b.item_start[0] = 0;
+        for (bool pair : {false, true}) {
+            std::vector<const SpmmJob *> sel;
             for (int i = 0; i < n_jobs; i++) {
                 const SpmmJob &sj = jobs[i];
-                if (!sj.tc || sj.f8 != f8 || sj.p->n_tc == 0 || sj.N <= 0)
-                    continue;
-                const bool pair = pair_eligible(sj.p, sj.n_tile);
-                if (NT == 0 ? !pair : (pair || sj.n_tile != NT))
-                    continue;
-                TCA_TRY(make_job(sj, alpha, beta, flags, NT, &b.job[b.n_jobs]));
-                const int units = NT == 0 ? sj.p->n_pairs : sj.p->n_tc;
-                b.item_start[b.n_jobs + 1] = b.item_start[b.n_jobs] + units * b.job[b.n_jobs].ntiles;
-                b.n_jobs++;
-                if (b.n_jobs == kMaxJobs) {
-                    TCA_TRY(emit(b, NT, f8));
-                    b.n_jobs = 0;
-                }
+                if (sj.tc && sj.f8 == f8 && sj.p->n_tc > 0 && sj.N > 0 && pair_eligible(sj.p, sj.n_tile) == pair)
+                    sel.push_back(&sj);
             }
-            TCA_TRY(emit(b, NT, f8));
+            std::stable_sort(sel.begin(), sel.end(),
+                             [&](const SpmmJob *x, const SpmmJob *y) { return cost(*x) > cost(*y); });
+            for (size_t i0 = 0; i0 < sel.size(); i0 += kMaxJobs) {
+                TcBatch b;
+                b.n_jobs = 0;
+                b.item_start[0] = 0;
+                int NT = 0;
+                for (size_t i = i0; i < std::min(sel.size(), i0 + kMaxJobs); i++) {
+                    const SpmmJob &sj = *sel[i];
+                    TCA_TRY(make_job(sj, alpha, beta, flags, pair ? 0 : sj.n_tile, &b.job[b.n_jobs]));
+                    const int units = pair ? sj.p->n_pairs : sj.p->n_tc;
+                    b.item_start[b.n_jobs + 1] = b.item_start[b.n_jobs] + units * b.job[b.n_jobs].ntiles;
+                    b.n_jobs++;
+                    if (!pair) NT = std::max(NT, sj.n_tile);
+                }
+                TCA_TRY(emit(b, NT, f8));
+            }
         }
     }
     return TCA_OK;

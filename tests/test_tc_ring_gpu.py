@@ -82,3 +82,27 @@ def test_ring_e4m3(cuda, chunks, N, out):
     # the quantized operands' magnitudes exceed the FP16 ones by at most 2^-4 each
     check(C, ref, c, out == "f16", extra=2.0 ** -21, vals=np.abs(c["vals"]) * np.float16(1.0625),
           B=np.abs(c["B"]) * np.float16(1.0625))
+
+
+@pytest.mark.parametrize("precision", ["f16", "e4m3"])
+@pytest.mark.parametrize("n_tile", [0, 128])
+def test_mixed_widths_one_launch(cuda, precision, n_tile):
+    """Jobs of different N-slice widths, chunk counts and N (whole slabs and
+    not) in one launch; more jobs than one launch holds."""
+    specs = [(3, 64), (17, 8), (1, 256), (9, 136), (5, 520), (33, 200), (2, 128)] * 5
+    cs = [matrix(ch, N, 7 * i + N) for i, (ch, N) in enumerate(specs)]
+    plans, Bs, outs = [], [], []
+    for c in cs:
+        rp, ci, v, B = (torch.from_numpy(c[k]).to(cuda) for k in ("row_ptr", "col", "vals", "B"))
+        plans.append(tca_spmm.Plan(rp, ci, v, c["K"], path="tensor_core"))
+        Bs.append(B)
+        outs.append(torch.full((c["M"], c["N"]), 5.0, dtype=torch.float32, device=cuda))
+    f8 = precision == "e4m3"
+    (tca_spmm.spmm_fp8_batched if f8 else tca_spmm.spmm_batched)(plans, Bs, outs, n_tile=n_tile)
+    for p, C, c in zip(plans, outs, cs):
+        p.status()
+        if f8:
+            check(C, oracle.spmm_fp8_f64(c["row_ptr"], c["col"], c["vals"], c["B"]), c, False, extra=2.0 ** -21,
+                  vals=np.abs(c["vals"]) * np.float16(1.0625), B=np.abs(c["B"]) * np.float16(1.0625))
+        else:
+            check(C, oracle.spmm_f64(c["row_ptr"], c["col"], c["vals"], c["B"]), c, False)
