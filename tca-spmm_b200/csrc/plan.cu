@@ -793,7 +793,7 @@ void build_items(const std::vector<int> &windows, const std::vector<int> &row_pt
 // only where they are first read (the tile entries), so that steps 1-5 run
 // while they are still on their way.
 int build_plan(tca_plan *p, const int *row_ptr, const int *col, const __half *val, cudaStream_t s,
-               cudaEvent_t vals_ready = nullptr, bool sync_end = true)
+               cudaEvent_t vals_ready = nullptr, bool sync_end = true, const std::function<int()> &meanwhile = {})
 {
     BuildStream build_stream(s);
     const int M = p->M, K = p->K, nnz = p->nnz;
@@ -924,6 +924,8 @@ int build_plan(tca_plan *p, const int *row_ptr, const int *col, const __half *va
     } else if (W > 0) {
         TCA_TRY(zero_async(d_stage, sizeof(int) * 4 * (size_t)W, s));
     }
+    if (meanwhile)
+        TCA_TRY(meanwhile());
     std::vector<int> h_stage(n_stage);
     TCA_CUDA_TRY(cudaMemcpyAsync(h_stage.data(), d_stage, sizeof(int) * n_stage, cudaMemcpyDeviceToHost, s));
     TCA_CUDA_TRY(cudaStreamSynchronize(s));
@@ -973,6 +975,7 @@ int build_plan(tca_plan *p, const int *row_ptr, const int *col, const __half *va
     std::vector<int4> h_wi((size_t)n_tc);
     for (int t = 0; t < n_tc; t++)
         h_wi[t] = make_int4(tc_list[t], h_first[t], h_first[t + 1] - h_first[t], h_direct[t]);
+    p->has_gathers = K % kChunkCols != 0 || std::count(h_direct.begin(), h_direct.end(), 1) != n_tc;
     // window pairs for the pair kernel: greedily, consecutive windows whose
     // chunks are all 64-column blocks of K (identical columns)
     std::vector<int2> h_pairs;
@@ -1161,7 +1164,7 @@ int run_jobs_with_events(const SpmmJob *jobs, int n_jobs, int c_dtype, float alp
 namespace tca {
 int plan_create(const int *d_row_ptr, const int *d_col_idx, const void *d_vals_f16, int M, int K, int nnz,
                 const tca_plan_opts_t *opts, cudaStream_t stream, cudaEvent_t vals_ready, bool sync_end,
-                tca_plan_t *plan)
+                tca_plan_t *plan, const std::function<int()> &meanwhile)
 {
     clear_error();
     if (!plan)
@@ -1182,7 +1185,7 @@ int plan_create(const int *d_row_ptr, const int *d_col_idx, const void *d_vals_f
     p->M = M; p->K = K; p->nnz = nnz; p->opts = o;
     int st = TCA_OK;
     if (M > 0)
-        st = build_plan(p, d_row_ptr, d_col_idx, (const __half *)d_vals_f16, stream, vals_ready, sync_end);
+        st = build_plan(p, d_row_ptr, d_col_idx, (const __half *)d_vals_f16, stream, vals_ready, sync_end, meanwhile);
     if (st != TCA_OK) {
         free_plan(p);
         return st;

@@ -50,6 +50,9 @@ struct tca_plan {
     // chunk columns and pair up; any other window is alone (second -1)
     int2 *tc_pairs = nullptr;
     int n_pairs = 0, n_full_pairs = 0;
+    // some chunk's B rows are gathered: a condensed window, or the last block
+    // of a K that is not whole 64-column blocks
+    bool has_gathers = false;
     int *win_cols = nullptr;
     int *tile_ptr = nullptr;
     uint32_t *tile_entries = nullptr;
@@ -191,9 +194,11 @@ int run_jobs_with_events(const SpmmJob *jobs, int n_jobs, int c_dtype, float alp
 // tca_plan_create with two extra controls for the host-buffer forward:
 // vals_ready (an event after which the values may be read; NULL: at once)
 // and sync_end (false: the build is only ordered on `stream`, not waited for).
+// `meanwhile` (may be empty) runs on the host before the build first waits for
+// the device, with the first kernels already issued.
 int plan_create(const int *d_row_ptr, const int *d_col_idx, const void *d_vals_f16, int M, int K, int nnz,
                 const tca_plan_opts_t *opts, cudaStream_t stream, cudaEvent_t vals_ready, bool sync_end,
-                tca_plan_t *plan);
+                tca_plan_t *plan, const std::function<int()> &meanwhile = {});
 
 // The N-slice width a single forward of this plan uses.
 int pick_tc_tile(const tca_plan *p, int N, bool batched, bool f8 = false);

@@ -1163,6 +1163,11 @@ int launch_cc_typed(const CcBatch &b, int w, bool f8, int beside_regs, cudaStrea
 int launch_cc_jobs(const SpmmJob *jobs, int n_jobs, int c_dtype, float alpha, float beta, unsigned flags,
                    cudaStream_t s, LaunchList *defer, int beside_regs)
 {
+    bool any = false; // rows left for this path
+    for (int i = 0; i < n_jobs && !any; i++)
+        any = jobs[i].N > 0 && (!jobs[i].tc || jobs[i].p->n_cc_items > 0);
+    if (!any)
+        return TCA_OK;
     // jobs whose operands do not allow 16-byte accesses (every window of the
     // plan: the tensor-core kernel needs them too): the rows kernel
     for (int w : {1, 2, 4, 8}) {

@@ -1311,8 +1311,9 @@ int make_job(const SpmmJob &sj, float alpha, float beta, unsigned flags, int NT,
         NT = kPairN;
     if (sj.f8) {
         // E4M3 B (K x N bytes, row stride ldq): boxes of 128 columns
-        TCA_TRY(encode_tensor_map_2d(&j.tmap_b, CU_TENSOR_MAP_DATA_TYPE_UINT8, sj.Bq, (uint64_t)sj.N, (uint64_t)p->K,
-                                     (uint64_t)sj.ldq, 128, 1, CU_TENSOR_MAP_SWIZZLE_128B));
+        if (p->has_gathers)
+            TCA_TRY(encode_tensor_map_2d(&j.tmap_b, CU_TENSOR_MAP_DATA_TYPE_UINT8, sj.Bq, (uint64_t)sj.N, (uint64_t)p->K,
+                                         (uint64_t)sj.ldq, 128, 1, CU_TENSOR_MAP_SWIZZLE_128B));
         if (j.tile3d)
             TCA_TRY(encode_tensor_map_slabs(&j.tmap_tile, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, sj.Bq,
                                             (uint64_t)(sj.N / slab), (uint64_t)p->K, (uint64_t)sj.ldq, kChunkCols,
@@ -1326,7 +1327,8 @@ int make_job(const SpmmJob &sj, float alpha, float beta, unsigned flags, int NT,
         j.row_scale = p->row_scale;
         j.col_scale = sj.col_scale;
     } else {
-        TCA_TRY(encode_b_map(sj, p->K, 1, &j.tmap_b));
+        if (p->has_gathers) // nothing else reads it
+            TCA_TRY(encode_b_map(sj, p->K, 1, &j.tmap_b));
         if (j.tile3d)
             TCA_TRY(encode_tensor_map_slabs(&j.tmap_tile, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, sj.B,
                                             (uint64_t)(sj.N / slab), (uint64_t)p->K, (uint64_t)sj.ldb * 2, kChunkCols,
@@ -1390,30 +1392,24 @@ int launch_group_cap(const TcBatchT<CAP> &b, bool dependent, cudaStream_t s)
     return TCA_OK;
 }
 
-template <int NT, typename OutT, bool F8>
-int launch_group(const TcBatch &b, bool dependent, cudaStream_t s)
-{
-    if (b.n_jobs == 1) {
-        TcBatchT<1> one;
-        one.n_jobs = 1;
-        one.item_start[0] = b.item_start[0];
-        one.item_start[1] = b.item_start[1];
-        one.job[0] = b.job[0];
-        return launch_group_cap<NT, OutT, F8, 1>(one, dependent, s);
-    }
-    return launch_group_cap<NT, OutT, F8, kMaxJobs>(b, dependent, s);
-}
-
-template <typename OutT>
-int launch_group_out(const TcBatch &b, int NT, bool f8, bool dependent, cudaStream_t s)
+template <typename OutT, int CAP>
+int launch_group_out(const TcBatchT<CAP> &b, int NT, bool f8, bool dependent, cudaStream_t s)
 {
     if (f8)
-        return NT == 128 ? launch_group<128, OutT, true>(b, dependent, s) : launch_group<256, OutT, true>(b, dependent, s);
+        return NT == 128 ? launch_group_cap<128, OutT, true>(b, dependent, s)
+                         : launch_group_cap<256, OutT, true>(b, dependent, s);
     switch (NT) {
-    case 64: return launch_group<64, OutT, false>(b, dependent, s);
-    case 128: return launch_group<128, OutT, false>(b, dependent, s);
-    default: return launch_group<256, OutT, false>(b, dependent, s);
+    case 64: return launch_group_cap<64, OutT, false>(b, dependent, s);
+    case 128: return launch_group_cap<128, OutT, false>(b, dependent, s);
+    default: return launch_group_cap<256, OutT, false>(b, dependent, s);
     }
+}
+
+template <int CAP>
+int launch_typed(const TcBatchT<CAP> &b, int NT, bool f8, int c_dtype, bool dependent, cudaStream_t s)
+{
+    return c_dtype == TCA_DTYPE_F16 ? launch_group_out<__half>(b, NT, f8, dependent, s)
+                                    : launch_group_out<float>(b, NT, f8, dependent, s);
 }
 
 // Pair kernel: clusters of two CTAs (one per SM), persistent over the pair
@@ -1467,8 +1463,15 @@ int launch_group_typed(const TcBatch &b, int NT, bool f8, int c_dtype, bool depe
 {
     if (b.n_jobs == 0 || b.item_start[b.n_jobs] == 0)
         return TCA_OK;
-    return c_dtype == TCA_DTYPE_F16 ? launch_group_out<__half>(b, NT, f8, dependent, s)
-                                    : launch_group_out<float>(b, NT, f8, dependent, s);
+    if (b.n_jobs == 1 && b.job[0].nt == NT) {
+        TcBatchT<1> one;
+        one.n_jobs = 1;
+        one.item_start[0] = b.item_start[0];
+        one.item_start[1] = b.item_start[1];
+        one.job[0] = b.job[0];
+        return launch_typed(one, NT, f8, c_dtype, dependent, s);
+    }
+    return launch_typed(b, NT, f8, c_dtype, dependent, s);
 }
 
 } // namespace
@@ -1536,6 +1539,25 @@ bool pair_eligible(const tca_plan *p, int NT)
 int launch_tc_jobs(const SpmmJob *jobs, int n_jobs, int c_dtype, float alpha, float beta, unsigned flags,
                    cudaStream_t s, LaunchList *defer, bool dependent)
 {
+    if (n_jobs == 1 && !pair_eligible(jobs[0].p, jobs[0].n_tile)) {
+        // a single forward: no batch of job slots to fill and copy
+        const SpmmJob &sj = jobs[0];
+        if (!sj.tc || sj.p->n_tc == 0 || sj.N <= 0)
+            return TCA_OK;
+        TcBatchT<1> one;
+        one.n_jobs = 1;
+        TCA_TRY(make_job(sj, alpha, beta, flags, sj.n_tile, &one.job[0]));
+        one.item_start[0] = 0;
+        one.item_start[1] = sj.p->n_tc * one.job[0].ntiles;
+        const int NT = sj.n_tile;
+        const bool f8 = sj.f8;
+        if (!defer)
+            return launch_typed(one, NT, f8, c_dtype, dependent, s);
+        defer->push_back([one, NT, f8, c_dtype, dependent](cudaStream_t st) {
+            return launch_typed(one, NT, f8, c_dtype, dependent, st);
+        });
+        return TCA_OK;
+    }
     auto emit = [&](const TcBatch &b, int NT, bool f8) -> int {
         if (b.n_jobs == 0 || b.item_start[b.n_jobs] == 0)
             return TCA_OK;
