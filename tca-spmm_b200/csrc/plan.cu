@@ -84,8 +84,12 @@ __global__ void k_row_check(const int *__restrict__ row_ptr, const int *__restri
 // offsets), and copies of the offsets and of the check verdict into the
 // array the host reads after step 3. Global loads and stores are striped
 // (coalesced), exchanged through shared memory with the sort's blocked order.
-constexpr int kOrderThreads = 1024, kOrderItems = 8, kOrderRows = kOrderThreads * kOrderItems;
+// The work of a pass is that of kOrderItems rows per thread whether there are
+// that many or not, so up to 2048 and 4096 rows take their own sizes (2048
+// rows: 9.7 -> 6.5 us).
+constexpr int kOrderThreads = 1024, kOrderRows = kOrderThreads * 8;
 
+template <int kOrderItems>
 __global__ void __launch_bounds__(kOrderThreads)
 k_order_small(const int *__restrict__ row_nnz, const int *__restrict__ row_sorted, int M, int sort,
               const int *__restrict__ err, int *__restrict__ perm, int *__restrict__ p_row_ptr,
@@ -116,7 +120,7 @@ k_order_small(const int *__restrict__ row_nnz, const int *__restrict__ row_sorte
     __syncthreads();
     Xchg(tmp.xchg).StripedToBlocked(val, val);
 #pragma unroll
-    for (int u = 0; u < kOrderItems; u++) // blocked: item u of thread t is row t * 8 + u
+    for (int u = 0; u < kOrderItems; u++) // blocked: item u of thread t is row t * kOrderItems + u
         val[u] = ((unsigned)(t * kOrderItems + u) << 1) | (val[u] & 1u);
     if (sort) {
         mx = __reduce_max_sync(0xffffffffu, mx);
@@ -157,23 +161,22 @@ k_order_small(const int *__restrict__ row_nnz, const int *__restrict__ row_sorte
     }
 }
 
-// Exclusive prefix sum of n values into out[0, n] (out[n] = the total), in
-// one block: the tile offsets of up to kScanSmallMax chunks.
+// Exclusive prefix sum of n values into out[0, n] (out[n] = the total), by one
+// block: the tile offsets of up to kScanSmallMax chunks.
 constexpr int kScanThreads = 1024, kScanItems = 8, kScanSmallMax = 8 * kScanThreads * kScanItems;
+using SmallScan = cub::BlockScan<int, kScanThreads>;
 
-__global__ void __launch_bounds__(kScanThreads) k_scan_small(const int *__restrict__ in, int n, int *__restrict__ out)
+__device__ void scan_small(const int *in, int n, int *out, typename SmallScan::TempStorage &tmp)
 {
-    using Scan = cub::BlockScan<int, kScanThreads>;
-    __shared__ typename Scan::TempStorage tmp;
     int carry = 0;
     for (int base = 0; base < n; base += kScanThreads * kScanItems) {
         int v[kScanItems], o[kScanItems], agg;
 #pragma unroll
         for (int u = 0; u < kScanItems; u++) {
             const int i = base + (int)threadIdx.x * kScanItems + u;
-            v[u] = i < n ? in[i] : 0;
+            v[u] = i < n ? __ldcg(in + i) : 0;
         }
-        Scan(tmp).ExclusiveSum(v, o, agg);
+        SmallScan(tmp).ExclusiveSum(v, o, agg);
 #pragma unroll
         for (int u = 0; u < kScanItems; u++) {
             const int i = base + (int)threadIdx.x * kScanItems + u;
@@ -392,7 +395,8 @@ __device__ int block_exclusive_scan(int v, int *total, int *scratch)
 // window) and writes its columns, ascending, 64 per chunk, -1 padding.
 __global__ void __launch_bounds__(1024)
 k_tile_cols(const int4 *__restrict__ win_info, const int *__restrict__ p_row_ptr, const int *__restrict__ p_col,
-            int M, int K, const uint32_t *__restrict__ bitmaps, int *__restrict__ win_cols)
+            int M, int K, const uint32_t *__restrict__ bitmaps, int *__restrict__ win_cols, int *__restrict__ chunk_nnz,
+            int n_chunks, int *__restrict__ done, uint32_t *__restrict__ pad)
 {
     extern __shared__ uint32_t sm[];
     __shared__ int scratch[33];
@@ -404,6 +408,16 @@ k_tile_cols(const int4 *__restrict__ win_info, const int *__restrict__ p_row_ptr
     const int r0 = w * kWindowRows, r1 = min(M, r0 + kWindowRows);
     const int lo = p_row_ptr[r0], hi = p_row_ptr[r1];
 
+    // cleared for k_tile_count: the chunk counters and its block counter; and
+    // the entries' padding
+    for (int i = threadIdx.x; i < nch; i += blockDim.x) chunk_nnz[c0 + i] = 0;
+    if (blockIdx.x == 0 && threadIdx.x < kEntryPad) {
+        pad[threadIdx.x] = 0u;
+        if (threadIdx.x == 0) {
+            chunk_nnz[n_chunks] = 0;
+            *done = 0;
+        }
+    }
     if (bitmaps) { // the window's column bitmap, as k_window_stats built it
         for (int i = threadIdx.x; i < nwords; i += blockDim.x) bm[i] = bitmaps[(size_t)w * nwords + i];
     } else {
@@ -478,9 +492,11 @@ constexpr int kTileBlocksPerChunk = kWindowRows / 32;
 __global__ void __launch_bounds__(1024)
 k_tile_count(const int2 *__restrict__ chunk_win, const int4 *__restrict__ win_info,
              const int *__restrict__ p_row_ptr, const int *__restrict__ p_col, const int *__restrict__ win_cols,
-             int M, int *__restrict__ chunk_nnz, int2 *__restrict__ row_range)
+             int M, int *chunk_nnz, int2 *__restrict__ row_range, int n_chunks, int *done, int *__restrict__ tile_ptr)
 {
-    __shared__ int s_sum;
+    static_assert(kScanThreads == 1024, "the block that scans has k_tile_count's threads");
+    __shared__ typename SmallScan::TempStorage s_scan;
+    __shared__ int s_sum, s_last;
     const int chunk = blockIdx.x / kTileBlocksPerChunk;
     const int lane = threadIdx.x & 31, lr = (blockIdx.x % kTileBlocksPerChunk) * 32 + (threadIdx.x >> 5);
     if (threadIdx.x == 0)
@@ -507,8 +523,21 @@ k_tile_count(const int2 *__restrict__ chunk_win, const int4 *__restrict__ win_in
             atomicAdd(&s_sum, hi - lo);
     }
     __syncthreads();
-    if (threadIdx.x == 0 && s_sum > 0)
-        atomicAdd(&chunk_nnz[chunk], s_sum); // integer sums: order-independent
+    if (threadIdx.x == 0) {
+        if (s_sum > 0)
+            atomicAdd(&chunk_nnz[chunk], s_sum); // integer sums: order-independent
+        if (tile_ptr) {
+            __threadfence();
+            s_last = atomicAdd(done, 1) == (int)gridDim.x - 1;
+        }
+    }
+    if (!tile_ptr)
+        return;
+    __syncthreads();
+    if (s_last) { // every block's counts are in: this one turns them into the tile offsets
+        __threadfence();
+        scan_small(chunk_nnz, n_chunks, tile_ptr, s_scan);
+    }
 }
 
 // 5c. Entries of each chunk, ordered by (row, column): a warp per row writes
@@ -737,6 +766,42 @@ struct Carve {
     }
 };
 
+// Page-locked memory for what the host reads during a build, one buffer per
+// host thread (a build uses it for one copy at a time and waits for that copy
+// before the next): a copy to pageable memory goes through the driver's own
+// staging and back (3.5 us on the device and ~25 us until the host goes on,
+// against ~8). At most kPinnedMax bytes, freed with the thread; NULL: use
+// pageable memory.
+constexpr size_t kPinnedMax = 4u << 20;
+struct PinnedBuffer {
+    void *p = nullptr;
+    size_t bytes = 0;
+    ~PinnedBuffer() { if (p) cudaFreeHost(p); }
+};
+void *pinned_staging(size_t bytes)
+{
+    thread_local PinnedBuffer b;
+    if (bytes > kPinnedMax)
+        return nullptr;
+    if (bytes > b.bytes) {
+        size_t n = 64 * 1024;
+        while (n < bytes) n *= 2;
+        void *q = nullptr;
+        if (cudaHostAlloc(&q, n, cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        if (b.p) cudaFreeHost(b.p);
+        b.p = q;
+        b.bytes = n;
+    }
+    return b.p;
+}
+struct EventGuard {
+    cudaEvent_t e = nullptr;
+    ~EventGuard() { if (e) cudaEventDestroy(e); }
+};
+
 template <typename T>
 T *at(void *base, size_t off)
 {
@@ -872,8 +937,9 @@ int build_plan(tca_plan *p, const int *row_ptr, const int *col, const __half *va
 
     // 2. row order
     if (small) {
-        k_order_small<<<1, kOrderThreads, 0, s>>>(row_nnz, row_sorted, M, p->opts.sort_rows ? 1 : 0, err, p->perm,
-                                                  p->p_row_ptr, p_sorted, d_stage + 4 * W, d_stage + 4 * W + 1);
+        auto order = M <= 2 * kOrderThreads ? k_order_small<2> : M <= 4 * kOrderThreads ? k_order_small<4> : k_order_small<8>;
+        order<<<1, kOrderThreads, 0, s>>>(row_nnz, row_sorted, M, p->opts.sort_rows ? 1 : 0, err, p->perm,
+                                          p->p_row_ptr, p_sorted, d_stage + 4 * W, d_stage + 4 * W + 1);
     } else {
         int *iota = at<int>(tb, o_iota), *keys_out = at<int>(tb, o_keys), *scan_in = at<int>(tb, o_scan_in);
         k_iota<<<blocks_for(M, 256), 256, 0, s>>>(iota, M);
@@ -927,8 +993,11 @@ int build_plan(tca_plan *p, const int *row_ptr, const int *col, const __half *va
     if (meanwhile)
         TCA_TRY(meanwhile());
     std::vector<int> h_stage(n_stage);
-    TCA_CUDA_TRY(cudaMemcpyAsync(h_stage.data(), d_stage, sizeof(int) * n_stage, cudaMemcpyDeviceToHost, s));
+    void *pin = pinned_staging(sizeof(int) * n_stage);
+    TCA_CUDA_TRY(cudaMemcpyAsync(pin ? pin : h_stage.data(), d_stage, sizeof(int) * n_stage, cudaMemcpyDeviceToHost, s));
     TCA_CUDA_TRY(cudaStreamSynchronize(s));
+    if (pin)
+        std::memcpy(h_stage.data(), pin, sizeof(int) * n_stage);
     const int h_err = h_stage[4 * (size_t)W];
     if (h_err & kErrRowPtr)
         return set_error(TCA_ERR_FORMAT, "row_ptr is not a valid CSR offset array (must start at 0, be non-decreasing and end at nnz=%d)", nnz);
@@ -1030,18 +1099,21 @@ int build_plan(tca_plan *p, const int *row_ptr, const int *col, const __half *va
         // pageable: the copy returns once its source is staged
         TCA_CUDA_TRY(cudaMemcpyAsync(a, h_part.data(), host_part, cudaMemcpyHostToDevice, s));
     }
-    TCA_TRY(zero_async(p->tile_entries + p->tc_nnz, sizeof(uint32_t) * kEntryPad, s));
 
     // 5. tiles
     DevBuf t_step5;
     std::vector<int> h_ptr((size_t)n_ch + 1, 0);
+    EventGuard ptr_read;
+    pin = pinned_staging(sizeof(int) * h_ptr.size());
+    if (pin && cudaEventCreateWithFlags(&ptr_read.e, cudaEventDisableTiming) != cudaSuccess)
+        pin = nullptr;
     if (n_tc > 0) {
         const bool small_scan = n_ch <= kScanSmallMax;
         size_t tmp = 0;
         if (!small_scan)
             TCA_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tmp, (const int *)nullptr, (int *)nullptr, n_ch + 1, s));
         Carve c;
-        const size_t o_cn = c.take<int>((size_t)n_ch + 1), o_rr = c.take<int2>((size_t)n_ch * kWindowRows),
+        const size_t o_cn = c.take<int>((size_t)n_ch + 2), o_rr = c.take<int2>((size_t)n_ch * kWindowRows),
                      o_tmp = c.take<char>(tmp);
         char *tb5;
         TCA_TRY(dev_alloc(&tb5, c.size, nullptr));
@@ -1050,14 +1122,19 @@ int build_plan(tca_plan *p, const int *row_ptr, const int *col, const __half *va
         int2 *d_rr = at<int2>(tb5, o_rr);
         const size_t smem = 2 * sizeof(uint32_t) * ((K + 31) / 32);
         TCA_CUDA_TRY(cudaFuncSetAttribute(k_tile_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k_tile_cols<<<n_tc, 1024, smem, s>>>(p->tc_win_info, p->p_row_ptr, p->p_col, M, K, d_bm, p->win_cols);
-        TCA_TRY(zero_async(d_cn, sizeof(int) * ((size_t)n_ch + 1), s));
-        k_tile_count<<<(unsigned)n_ch * kTileBlocksPerChunk, 1024, 0, s>>>(d_cw, p->tc_win_info, p->p_row_ptr,
-                                                                           p->p_col, p->win_cols, M, d_cn, d_rr);
-        if (small_scan) {
-            k_scan_small<<<1, kScanThreads, 0, s>>>(d_cn, n_ch, p->tile_ptr);
-        } else {
+        int *d_done5 = d_cn + n_ch + 1;
+        k_tile_cols<<<n_tc, 1024, smem, s>>>(p->tc_win_info, p->p_row_ptr, p->p_col, M, K, d_bm, p->win_cols, d_cn, n_ch,
+                                             d_done5, p->tile_entries + p->tc_nnz);
+        k_tile_count<<<(unsigned)n_ch * kTileBlocksPerChunk, 1024, 0, s>>>(
+            d_cw, p->tc_win_info, p->p_row_ptr, p->p_col, p->win_cols, M, d_cn, d_rr, n_ch, d_done5,
+            small_scan ? p->tile_ptr : nullptr);
+        if (!small_scan) {
             TCA_CUDA_TRY(cub::DeviceScan::ExclusiveSum(at<char>(tb5, o_tmp), tmp, d_cn, p->tile_ptr, n_ch + 1, s));
+        }
+        // the host reads the tile offsets while the device writes the tiles
+        if (pin) {
+            TCA_CUDA_TRY(cudaMemcpyAsync(pin, p->tile_ptr, sizeof(int) * h_ptr.size(), cudaMemcpyDeviceToHost, s));
+            TCA_CUDA_TRY(cudaEventRecord(ptr_read.e, s));
         }
         TCA_TRY(gather_vals());
         k_tile_write<<<(unsigned)n_ch * kTileBlocksPerChunk, 1024, 0, s>>>(d_cw, p->tc_win_info, p->p_col, p->p_val,
@@ -1066,6 +1143,7 @@ int build_plan(tca_plan *p, const int *row_ptr, const int *col, const __half *va
         TCA_CUDA_TRY(cudaGetLastError());
     } else {
         TCA_TRY(zero_async(p->tile_ptr, sizeof(int), s));
+        TCA_TRY(zero_async(p->tile_entries, sizeof(uint32_t) * kEntryPad, s));
     }
 
     // 7 (while the device writes the tiles). CUDA-core work items.
@@ -1079,8 +1157,13 @@ int build_plan(tca_plan *p, const int *row_ptr, const int *col, const __half *va
 
     // 6. dense tile images for chunks holding at least kImageMinNnz nonzeros
     if (n_ch > 0) {
-        TCA_CUDA_TRY(cudaMemcpyAsync(h_ptr.data(), p->tile_ptr, sizeof(int) * h_ptr.size(), cudaMemcpyDeviceToHost, s));
-        TCA_CUDA_TRY(cudaStreamSynchronize(s));
+        if (pin) {
+            TCA_CUDA_TRY(cudaEventSynchronize(ptr_read.e));
+            std::memcpy(h_ptr.data(), pin, sizeof(int) * h_ptr.size());
+        } else {
+            TCA_CUDA_TRY(cudaMemcpyAsync(h_ptr.data(), p->tile_ptr, sizeof(int) * h_ptr.size(), cudaMemcpyDeviceToHost, s));
+            TCA_CUDA_TRY(cudaStreamSynchronize(s));
+        }
     }
     std::vector<int> h_img((size_t)n_ch, -1), h_img_chunk;
     for (int c = 0; c < n_ch; c++)
