@@ -1428,6 +1428,12 @@ static int spmm_impl(tca_plan_t p, const void *d_B_f16, int ldb, int N, void *d_
     SpmmJob job;
     TCA_TRY(make_job(p, d_B_f16, ldb, N, d_C, ldc, c_dtype, false, &job));
     if (p->M == 0 || N == 0) return TCA_OK;
+    if (!ev && !dense_operands_vec_ok(d_B_f16, ldb, N, d_C, ldc, c_dtype)) {
+        bool done = false;
+        TCA_TRY(spmm_padded(&job, p->p_row_ptr, p->p_col, p->p_val, p->M, p->K, p->nnz, job.B, ldb, N, d_C, ldc, c_dtype,
+                            alpha, beta, flags, s, &done));
+        if (done) return TCA_OK;
+    }
     return run_jobs_with_events(&job, 1, c_dtype, alpha, beta, flags, s, ev);
 }
 

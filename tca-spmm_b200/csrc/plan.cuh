@@ -200,6 +200,13 @@ int plan_create(const int *d_row_ptr, const int *d_col_idx, const void *d_vals_f
                 const tca_plan_opts_t *opts, cudaStream_t stream, cudaEvent_t vals_ready, bool sync_end,
                 tca_plan_t *plan, const std::function<int()> &meanwhile = {});
 
+// A forward whose operands do not allow 16-byte accesses, through an aligned
+// copy of B when that pays (*done; spmm_csr_cc.cu): of a plan (`sj`; row_ptr,
+// col, val its re-ordered CSR) or straight from a CSR (sj NULL).
+int spmm_padded(const SpmmJob *sj, const int *row_ptr, const int *col, const __half *val, int M, int K, int nnz,
+                const __half *B, int ldb, int N, void *C, int ldc, int c_dtype, float alpha, float beta, unsigned flags,
+                cudaStream_t s, bool *done);
+
 // The N-slice width a single forward of this plan uses.
 int pick_tc_tile(const tca_plan *p, int N, bool batched, bool f8 = false);
 

@@ -112,8 +112,10 @@ template <int CAP> struct RowsBatchT {
 };
 
 // W output columns per lane of a group of LPR lanes. VEC: 8 consecutive ones,
-// in 16-byte accesses (N % 8 == 0, 16-byte aligned rows); else every LPR-th.
-template <typename OutT, int LPR, int W, bool VEC, int CAP>
+// B read in 16-byte accesses (16-byte aligned rows of at least N rounded up to
+// 8 columns), C written so too with VC (N % 8 == 0, 16-byte aligned rows);
+// else every LPR-th column.
+template <typename OutT, int LPR, int W, bool VEC, bool VC, int CAP>
 __global__ void __launch_bounds__(kRowsThreads, 2) spmm_rows_kernel(const __grid_constant__ RowsBatchT<CAP> batch)
 {
     static_assert(!VEC || W == 8, "16-byte accesses cover 8 columns");
@@ -205,7 +207,16 @@ __global__ void __launch_bounds__(kRowsThreads, 2) spmm_rows_kernel(const __grid
     auto write = [&](int i, const float *acc) {
         const int r = row0 + i;
         OutT *cp = reinterpret_cast<OutT *>(a.C) + (size_t)(a.perm ? __ldg(a.perm + r) : r) * a.ldc + n0;
-        if constexpr (VEC) {
+        if constexpr (VEC && !VC) {
+#pragma unroll
+            for (int w = 0; w < 8; w++) {
+                if (n0 + w >= a.N)
+                    continue;
+                float o = a.alpha * acc[w];
+                if (a.beta != 0.f) o = fmaf(a.beta, to_f<OutT>(cp[w]), o);
+                cp[w] = from_f<OutT>(o);
+            }
+        } else if constexpr (VEC) {
             if (!col_ok(0))
                 return;
             float o[8];
@@ -751,7 +762,7 @@ namespace {
 // (measured, 4096 x 4096 at 95 %, N = 512: 8 lanes a row 193 us, 32 lanes
 // 118 us). Blocks: about 64 nonzeros and rows per group, so that a
 // block's fixed cost (search, prefix sums, first dependent loads) is small
-// beside them, but at least two blocks per SM while a group keeps 8.
+// beside them, in whole waves of two blocks per SM, while a group keeps 8.
 struct RowsShape { int lpr, w; };
 RowsShape rows_shape(int N, bool vec)
 {
@@ -762,8 +773,10 @@ RowsShape rows_shape(int N, bool vec)
 int rows_blocks(const RowsJob &a, const RowsShape &sh, int slices) // per N-slice
 {
     const long long groups = kRowsThreads / sh.lpr, keys = (long long)a.nnz + a.M;
-    const long long fill = std::min<long long>((2 * kSMs + slices - 1) / slices, (keys + groups * 8 - 1) / (groups * 8));
-    const long long n = std::max((keys + groups * 64 - 1) / (groups * 64), fill);
+    const long long wave = 2 * kSMs; // resident blocks
+    // whole waves over all slices (3001 x 1777 at 92 %, N = 203: 419 blocks, 1.4 waves, 41.6 us; 296 34.5 us)
+    const long long waves = std::max(1LL, (keys * slices / (groups * 64) + wave / 2) / wave);
+    const long long n = std::min((waves * wave + slices - 1) / slices, (keys + groups * 8 - 1) / (groups * 8));
     return (int)std::max<long long>(1, std::min<long long>(n, a.M));
 }
 
@@ -779,9 +792,9 @@ int launch_rows(const RowsBatchT<kMaxCcJobs> &b, cudaStream_t s)
         one.block_start[0] = 0;
         one.block_start[1] = grid;
         one.job[0] = b.job[0];
-        spmm_rows_kernel<OutT, LPR, W, VEC, 1><<<grid, kRowsThreads, 0, s>>>(one);
+        spmm_rows_kernel<OutT, LPR, W, VEC, VEC, 1><<<grid, kRowsThreads, 0, s>>>(one);
     } else {
-        spmm_rows_kernel<OutT, LPR, W, VEC, kMaxCcJobs><<<grid, kRowsThreads, 0, s>>>(b);
+        spmm_rows_kernel<OutT, LPR, W, VEC, VEC, kMaxCcJobs><<<grid, kRowsThreads, 0, s>>>(b);
     }
     TCA_CUDA_TRY(cudaGetLastError());
     return TCA_OK;
@@ -817,11 +830,171 @@ void rows_add(RowsBatchT<kMaxCcJobs> &b, RowsJob &a, const RowsShape &sh)
 
 } // namespace
 
+namespace {
+
+// Copies rows of N halves to rows of ldp (a multiple of 8, at least N), zeros
+// after them: a warp per 256 columns of a row, every access coalesced.
+__global__ void __launch_bounds__(256) k_pad_rows(const __half *__restrict__ src, int rows, int N, int ld,
+                                                  __half *__restrict__ dst, int ldp)
+{
+    const int slices = (ldp + 255) / 256, lane = threadIdx.x & 31;
+    const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (w >= (long long)rows * slices)
+        return;
+    const long long r = w / slices;
+    const int n0 = (int)(w - r * slices) * 256 + lane;
+    unsigned short v[8];
+#pragma unroll
+    for (int u = 0; u < 8; u++)
+        v[u] = n0 + u * 32 < N ? __ldg(reinterpret_cast<const unsigned short *>(src) + r * ld + n0 + u * 32) : (unsigned short)0;
+#pragma unroll
+    for (int u = 0; u < 8; u++)
+        if (n0 + u * 32 < ldp)
+            reinterpret_cast<unsigned short *>(dst)[r * ldp + n0 + u * 32] = v[u];
+}
+
+// C = alpha * S + beta * C from FP32 sums S (rows of lds), FP16 C of any
+// alignment; rows without nonzeros are skipped with KEEP_EMPTY_ROWS. A warp
+// per 256 columns of a sorted row.
+__global__ void __launch_bounds__(256)
+k_unpad_rows(const float *__restrict__ sums, int lds, const int *__restrict__ perm, const int *__restrict__ p_row_ptr,
+             int M, int N, __half *__restrict__ C, int ldc, float alpha, float beta, unsigned flags)
+{
+    const int slices = (N + 255) / 256, lane = threadIdx.x & 31;
+    const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (w >= (long long)M * slices)
+        return;
+    const int i = (int)(w / slices), n0 = (int)(w - (long long)i * slices) * 256 + lane;
+    if ((flags & TCA_FLAG_KEEP_EMPTY_ROWS) && __ldg(p_row_ptr + i + 1) == __ldg(p_row_ptr + i))
+        return;
+    const size_t r = (size_t)__ldg(perm + i);
+    float v[8];
+#pragma unroll
+    for (int u = 0; u < 8; u++) v[u] = n0 + u * 32 < N ? __ldg(sums + r * lds + n0 + u * 32) : 0.f;
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+        if (n0 + u * 32 >= N)
+            break;
+        __half *c = C + r * ldc + n0 + u * 32;
+        float o = alpha * v[u];
+        if (beta != 0.f) o = fmaf(beta, __half2float(*c), o);
+        *c = __float2half_rn(o);
+    }
+}
+
+template <typename OutT, int LPR> int launch_rows_padded(const RowsBatchT<1> &b, cudaStream_t s)
+{
+    spmm_rows_kernel<OutT, LPR, 8, true, false, 1><<<b.block_start[1], kRowsThreads, 0, s>>>(b);
+    TCA_CUDA_TRY(cudaGetLastError());
+    return TCA_OK;
+}
+
+// The rows kernel over a padded (aligned) copy of B, C as it is.
+template <typename OutT> int rows_over_padded(RowsJob a, cudaStream_t s)
+{
+    const RowsShape sh = rows_shape(a.N, true);
+    RowsBatchT<kMaxCcJobs> all;
+    all.n_jobs = 0;
+    all.block_start[0] = 0;
+    rows_add(all, a, sh);
+    RowsBatchT<1> b;
+    b.n_jobs = 1;
+    b.block_start[0] = 0;
+    b.block_start[1] = all.block_start[1];
+    b.job[0] = all.job[0];
+    switch (sh.lpr) {
+    case 4: return launch_rows_padded<OutT, 4>(b, s);
+    case 8: return launch_rows_padded<OutT, 8>(b, s);
+    case 16: return launch_rows_padded<OutT, 16>(b, s);
+    default: return launch_rows_padded<OutT, 32>(b, s);
+    }
+}
+
+// Stream-ordered scratch of one call.
+struct Scratch {
+    void *p = nullptr;
+    cudaStream_t s;
+    explicit Scratch(cudaStream_t st) : s(st) {}
+    ~Scratch() { dev_free(p, s); }
+};
+
+} // namespace
+
+// A forward whose B or C does not allow 16-byte accesses (an odd N, unaligned
+// rows) through an aligned copy of B, when that pays: two-byte accesses gather
+// B at about half the rate of 16-byte ones (3001 x 1777 at 92 %, N = 203: 48
+// us; 2 us for the copy and 34 us after it), and a plan's tensor-core
+// windows can run on the tensor cores again. That needs an aligned C too, so
+// the sums go to an FP32 buffer and from there to C; only for FP16 C, whose
+// rounding (2^-11) is far above what separates the two kernels' FP32 sums (4096
+// x 4096 at 90 %, N = 1001: 606 -> 45 us).
+// The rule: nnz * N >= 2^25 (below, the two-byte kernel takes less than ~25
+// us and the copy and its launch eat the gain), copies of at most kPadMax
+// bytes, and not under stream capture, where this call allocates nothing.
+// *done = false: the caller runs the two-byte kernel.
+constexpr size_t kPadMax = 64u << 20;
+
+int spmm_padded(const SpmmJob *sj, const int *row_ptr, const int *col, const __half *val, int M, int K, int nnz,
+                const __half *B, int ldb, int N, void *C, int ldc, int c_dtype, float alpha, float beta, unsigned flags,
+                cudaStream_t s, bool *done)
+{
+    *done = false;
+    const int ldp = (N + 63) & ~63;
+    const size_t b_bytes = sizeof(__half) * (size_t)K * ldp, c_bytes = sizeof(float) * (size_t)M * ldp;
+    if ((long long)nnz * N < (1LL << 25) || b_bytes > kPadMax || c_bytes > kPadMax)
+        return TCA_OK;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) {
+        cudaGetLastError();
+        return TCA_OK;
+    }
+    if (cap != cudaStreamCaptureStatusNone)
+        return TCA_OK;
+    const bool tc = sj && sj->p->n_tc > 0 && c_dtype == TCA_DTYPE_F16;
+    Scratch ws(s);
+    if (dev_malloc(&ws.p, b_bytes + (tc ? c_bytes : 0), s) != TCA_OK) {
+        cudaGetLastError();
+        clear_error();
+        return TCA_OK;
+    }
+    *done = true;
+    __half *Bp = static_cast<__half *>(ws.p);
+    const long long warps = (long long)K * ((ldp + 255) / 256);
+    k_pad_rows<<<(unsigned)((warps * 32 + 255) / 256), 256, 0, s>>>(B, K, N, ldb, Bp, ldp);
+    TCA_CUDA_TRY(cudaGetLastError());
+    if (!tc) {
+        RowsJob a{row_ptr, col, sj ? sj->p->perm : nullptr, val, Bp, C, M, K, nnz, N, ldp, ldc, 0, alpha, beta, flags};
+        return c_dtype == TCA_DTYPE_F16 ? rows_over_padded<__half>(a, s) : rows_over_padded<float>(a, s);
+    }
+    float *sums = reinterpret_cast<float *>(static_cast<char *>(ws.p) + b_bytes); // b_bytes: a multiple of 128
+    SpmmJob job = *sj;
+    job.B = Bp;
+    job.ldb = ldp;
+    job.N = ldp;
+    job.C = sums;
+    job.ldc = ldp;
+    job.tc = true;
+    job.n_tile = pick_tc_tile(sj->p, ldp, false);
+    TCA_TRY(run_jobs_with_events(&job, 1, TCA_DTYPE_F32, 1.f, 0.f, 0u, s, nullptr));
+    const long long out_warps = (long long)M * ((N + 255) / 256);
+    k_unpad_rows<<<(unsigned)((out_warps * 32 + 255) / 256), 256, 0, s>>>(
+        sums, ldp, sj->p->perm, sj->p->p_row_ptr, M, N, static_cast<__half *>(C), ldc, alpha, beta, flags);
+    TCA_CUDA_TRY(cudaGetLastError());
+    return TCA_OK;
+}
+
 int launch_spmm_csr_cc(const int *row_ptr, const int *col_idx, const __half *vals, int M, int K, int nnz,
                        const __half *B, int ldb, int N, void *C, int ldc, int c_dtype,
                        float alpha, float beta, unsigned flags, cudaStream_t stream)
 {
     const bool vec = vec_ok(B, ldb, N, C, ldc, c_dtype);
+    if (!vec) {
+        bool done = false;
+        TCA_TRY(spmm_padded(nullptr, row_ptr, col_idx, vals, M, K, nnz, B, ldb, N, C, ldc, c_dtype, alpha, beta, flags,
+                            stream, &done));
+        if (done)
+            return TCA_OK;
+    }
     const RowsShape sh = rows_shape(N, vec);
     RowsBatchT<kMaxCcJobs> b;
     b.n_jobs = 0;
