@@ -63,7 +63,8 @@ constexpr int kEpiWarp0 = 7;     // warps 7-10: epilogue
 constexpr int kEpiThreads = 128;
 constexpr int kThreads = 352;
 constexpr int kAhead = 4;        // chunks by which the entries of a sparse chunk precede its stage
-constexpr int kRecords = 64;     // chunk records kept: two batches of 32
+constexpr int kRecords = 64;     // chunk records of A kept: two batches of 32
+constexpr int kRecordsB = 32;    // of B: one
 constexpr int kMaxCtaItems = 32;      // work items per persistent CTA
 constexpr int kEpiBar = 3;           // named barrier of the epilogue warps
 constexpr int kStagingBytes = ((kImageMinNnz + 3) * 4 + 15) & ~15; // entries of a sparse chunk, 16-byte rounded
@@ -174,14 +175,18 @@ template <int NT, bool F8> struct TcCfg {
     static constexpr int kStagingOff = kStages * kStage;
     // entry staging slots: kStages + kAhead, rounded up to a multiple of the scatter warps (see the scatter role)
     static constexpr int kSlots = (kStages + kAhead + kScatterWarps - 1) / kScatterWarps * kScatterWarps;
-    static constexpr int kRecOff = kStagingOff + kSlots * kStagingBytes;  // TcRecordA, TcRecordB [kRecords]
-    static constexpr int kItemOff = kRecOff + kRecords * 32;              // int4 [kMaxCtaItems]
-    static constexpr int kPendOff = kItemOff + kMaxCtaItems * 16;         // int2 [kSlots]: stage, entries
-    static constexpr int kCumOff = kPendOff + kSlots * 8;                 // int [kMaxCtaItems + 4]: first chunk of each item
+    static constexpr int kColsOff = kStagingOff + kSlots * kStagingBytes; // int4 [kSlots][16]: condensed columns
+    static constexpr int kRecOff = kColsOff + kSlots * kChunkCols * 4;    // TcRecordA [kRecords], TcRecordB [kRecordsB]
+    static constexpr int kItemOff = kRecOff + kRecords * 32 + kRecordsB * 16;            // int4 [kMaxCtaItems]
+    static constexpr int kPendOff = kItemOff + kMaxCtaItems * 16;         // int4 [kSlots]: stage, entries, item (-1: no gather)
+    static constexpr int kCumOff = kPendOff + kSlots * 16;                // int [kMaxCtaItems + 4]: first chunk of each item
     static constexpr int kScaleOff = kCumOff + (kMaxCtaItems + 4) * 4;    // E4M3: float [2][NT] column scales
     static constexpr int kBarOff = kScaleOff + (F8 ? 2 * NT * 4 : 0);
     // full, empty [kStages]; staged [kSlots]; accum_full, accum_empty [2]; drain; TMEM slot
     static constexpr int kSmem = kBarOff + (2 * kStages + kSlots + 5) * 8 + 8;
+    // of the SM's 228 KB, 1 KB per resident block is reserved: this block and two of the CUDA-core kernel
+    // (300 bytes more for E4M3 at N = 256 left room for one: 32-problem step 52.5 -> 63.1 us)
+    static_assert(kSmem + 3 * 1024 <= 228 * 1024, "room for the CUDA-core blocks beside this one");
     static_assert(kSmem <= 227 * 1024, "shared memory budget");
     static_assert(kStage % 1024 == 0 && kATileBytes % 1024 == 0, "swizzled tiles need 1024-byte alignment");
     static_assert(kStagingOff % 16 == 0 && kStagingBytes % 16 == 0 && kPendOff % 16 == 0, "16-byte alignment");
@@ -206,17 +211,20 @@ __device__ __forceinline__ int4 decode_item(const Batch &batch, int item)
     return make_int4(wi.x, wi.y, wi.z, (j << 16) | (local % a.ntiles));
 }
 
-// A chunk as the two loaders issue it (16 bytes of shared memory each).
+// A chunk as the two loaders issue it, in shared memory.
 struct __align__(16) TcRecordA {
-    const void *src; // dense image or (16-byte aligned) first entry
-    int bytes;       // of src: kATileBytes for an image, fewer for entries
-    int ent;         // entries: count << 2 | entries before the first one
+    const void *src;  // dense image or (16-byte aligned) first entry
+    const int *cols;  // condensed sparse chunk: its columns, else NULL
+    int bytes;        // of src: kATileBytes for an image, fewer for entries
+    int ent;          // entries: count << 2 | entries before the first one
+    int item;
 };
+constexpr int kByScatter = (int)0x80000000;
 constexpr int kSlabBits = 26;
 constexpr uint32_t kSlabMask = (1u << kSlabBits) - 1u;
 struct __align__(16) TcRecordB {
     const void *b; // tensor map; condensed columns: the column list
-    int col0;      // first of 64 consecutive columns; condensed columns: -1 - item
+    int col0;      // first of 64 consecutive columns; condensed columns: -1 - item; kByScatter: left to a scatter warp
     uint32_t x;    // 128-byte slab of n0 | slabs of the slice << kSlabBits | top bit: one 3-D box
 };
 
@@ -320,7 +328,9 @@ __device__ __forceinline__ void store_rows(uint32_t acc, OutT *C, int ldc, int o
 //     the entries are in and the stage is free ("staged"), zeroes the A tile,
 //     writes the entries into the swizzled layout and arrives on "full" --
 //     while the chunk's B rows are still on their way; image chunks pass them
-//     by. (A warp per chunk and not all four per chunk: the steps of a chunk
+//     by. A condensed chunk's warp also issues its B rows' gathers (32 ns
+//     each, 64 of them at N = 256: one loader warp would pace the ring; 2000 x
+//     16384 at 99.6 %, N = 256: 102 us, 42 us this way). (A warp per chunk and not all four per chunk: the steps of a chunk
 //     are a chain of ~0.6 us, and four chunks then run through it at once.)
 //     Sparse chunk q uses slot q % kSlots; it is filled when chunk g is
 //     issued, at most kAhead chunks before its own, so sparse chunk q -
@@ -339,7 +349,7 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
     constexpr int S = Cfg::kStages;
     constexpr int kATileBytes = Cfg::kATileBytes;
     extern __shared__ __align__(1024) uint8_t smem[];
-    int2 *pend = reinterpret_cast<int2 *>(smem + Cfg::kPendOff);
+    int4 *pend = reinterpret_cast<int4 *>(smem + Cfg::kPendOff);
     TcRecordA *rec_a = reinterpret_cast<TcRecordA *>(smem + Cfg::kRecOff);
     TcRecordB *rec_b = reinterpret_cast<TcRecordB *>(rec_a + kRecords);
     int4 *items = reinterpret_cast<int4 *>(smem + Cfg::kItemOff);
@@ -381,18 +391,17 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
         return it.y + i;
     };
     // a loader's chunk metadata from the plan, one chunk per lane: the columns
-    // of its ends (B), or its image and entry range (A)
-    int k = 0, c = 0, m0 = 0, m1 = 0, img = -1;
+    // of its ends, its image, and for A its entry range
+    int k = 0, c = 0, m0 = 0, m1 = 0, img = -1, c0 = 0, c1 = 0;
     auto fetch = [&](int g, int k0) {
         k = k0;
         if (g < cum[n_items]) {
             c = locate(g, k);
             const TcJob &a = batch.job[items[k].w >> 16];
-            if (warp == kBLoaderWarp) {
-                m0 = __ldg(a.win_cols + (size_t)c * kChunkCols);
-                m1 = __ldg(a.win_cols + (size_t)c * kChunkCols + kChunkCols - 1);
-            } else {
-                img = __ldg(a.img_idx + c);
+            c0 = __ldg(a.win_cols + (size_t)c * kChunkCols);
+            c1 = __ldg(a.win_cols + (size_t)c * kChunkCols + kChunkCols - 1);
+            img = __ldg(a.img_idx + c);
+            if (warp == kALoaderWarp) {
                 m0 = __ldg(a.tile_ptr + c);
                 m1 = __ldg(a.tile_ptr + c + 1);
             }
@@ -458,12 +467,12 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
                 const TcJob &a = batch.job[it.w >> 16];
                 TcRecordB r;
                 const int n0 = (it.w & 0xffff) * width(a);
-                const bool direct = m0 >= 0 && m1 == m0 + kChunkCols - 1;
+                const bool direct = c0 >= 0 && c1 == c0 + kChunkCols - 1;
                 r.b = direct ? (const void *)&a.tmap_tile : (const void *)(a.win_cols + (size_t)c * kChunkCols);
-                r.col0 = direct ? m0 : -1 - k;
+                r.col0 = direct ? c0 : img < 0 ? kByScatter : -1 - k;
                 r.x = (uint32_t)(n0 / Cfg::kBoxCols) | (uint32_t)(width(a) / Cfg::kBoxCols) << kSlabBits |
                       (a.tile3d ? 0x80000000u : 0u);
-                rec_b[(g0 + lane) % kRecords] = r;
+                rec_b[(g0 + lane) % kRecordsB] = r;
             }
             fetch(g0 + 32 + lane, __shfl_sync(0xffffffffu, k, 31));
             __syncwarp();
@@ -488,12 +497,12 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
             const int ge = min(total_chunks, g + 32);
             int s1 = s;
             uint32_t phase1 = phase;
-            if (__all_sync(0xffffffffu, g + lane >= ge || rec_b[(g + lane) % kRecords].col0 >= 0)) {
+            if (__all_sync(0xffffffffu, g + lane >= ge || rec_b[(g + lane) % kRecordsB].col0 >= 0)) {
                 // direct chunks only: one lane alone
                 if (elect_one()) {
-                    TcRecordB r = rec_b[g % kRecords];
+                    TcRecordB r = rec_b[g % kRecordsB];
                     for (int h = g; h < ge; h++) {
-                        const TcRecordB nxt = rec_b[(h + 1) % kRecords];
+                        const TcRecordB nxt = rec_b[(h + 1) % kRecordsB];
                         if (!mbar_wait(&empty[s1], phase1)) { ok = false; break; }
                         mbar_arrive_expect_tx(&full[s1], (uint32_t)boxes(r) * (kChunkCols * 128));
                         issue_boxes(r, s1);
@@ -504,13 +513,13 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
             } else {
                 int4 ncols = make_int4(-1, -1, -1, -1); // columns of the next chunk, when it is a condensed one
                 auto fetch_cols = [&](const TcRecordB &r) {
-                    if (r.col0 < 0 && lane < 16)
+                    if (r.col0 < 0 && r.col0 != kByScatter && lane < 16)
                         ncols = __ldg(reinterpret_cast<const int4 *>(r.b) + lane);
                 };
-                fetch_cols(rec_b[g % kRecords]);
+                fetch_cols(rec_b[g % kRecordsB]);
                 for (int h = g; h < ge; h++) {
-                    const TcRecordB r = rec_b[h % kRecords];
-                    if (elect_one()) {
+                    const TcRecordB r = rec_b[h % kRecordsB];
+                    if (elect_one() && r.col0 != kByScatter) {
                         ok = mbar_wait(&empty[s1], phase1);
                         if (ok) {
                             mbar_arrive_expect_tx(&full[s1], (uint32_t)boxes(r) * (kChunkCols * 128));
@@ -519,7 +528,7 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
                         }
                     }
                     if (__any_sync(0xffffffffu, !ok)) break; // also: the transaction count is set
-                    if (r.col0 < 0) {
+                    if (r.col0 < 0 && r.col0 != kByScatter) {
                         // condensed columns: gather p = lane, lane + 32, .. reads the 4 columns of lane p % 16
                         const int4 it = items[-1 - r.col0];
                         const TcJob &a = batch.job[it.w >> 16];
@@ -536,7 +545,7 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
                         }
                     }
                     if (h + 1 < ge)
-                        fetch_cols(rec_b[(h + 1) % kRecords]);
+                        fetch_cols(rec_b[(h + 1) % kRecordsB]);
                     if (++s1 == S) { s1 = 0; phase1 ^= 1; }
                 }
             }
@@ -556,6 +565,8 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
                                  : (const void *)(a.entries + (m0 & ~3));
                 r.bytes = img >= 0 ? kATileBytes : m1 > m0 ? ((m1 - (m0 & ~3)) * 4 + 15) & ~15 : 0;
                 r.ent = ((m1 - m0) << 2) | (m0 & 3);
+                r.cols = img < 0 && !(c0 >= 0 && c1 == c0 + kChunkCols - 1) ? a.win_cols + (size_t)c * kChunkCols : nullptr;
+                r.item = k;
                 rec_a[(g0 + lane) % kRecords] = r;
             }
             fetch(g0 + 32 + lane, __shfl_sync(0xffffffffu, k, 31));
@@ -572,6 +583,11 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
                         mbar_expect_tx(&staged[pslot], (uint32_t)r.bytes);
                         bulk_copy_g2s(smem_u32(smem + Cfg::kStagingOff + pslot * kStagingBytes), r.src,
                                       (uint32_t)r.bytes, &staged[pslot]);
+                    }
+                    if (r.cols) {
+                        mbar_expect_tx(&staged[pslot], kChunkCols * 4);
+                        bulk_copy_g2s(smem_u32(smem + Cfg::kColsOff + pslot * kChunkCols * 4), r.cols, kChunkCols * 4,
+                                      &staged[pslot]);
                     }
                     if (++pslot == Cfg::kSlots) pslot = 0;
                 }
@@ -595,7 +611,7 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
                         mbar_arrive_expect_tx(&full[s], kATileBytes);
                         bulk_copy_g2s(smem_u32(smem + s * Cfg::kStage), r.src, kATileBytes, &full[s]);
                     } else {
-                        pend[slot] = make_int2(s, r.ent);
+                        pend[slot] = make_int4(s, r.ent, r.cols ? r.item : -1, 0);
                         mbar_arrive(&staged[slot]); // the scatter warps arrive on "full"
                         if (++slot == Cfg::kSlots) slot = 0;
                     }
@@ -671,8 +687,21 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
         for (int q = warp - kScatterWarp0; q < n_sparse; q += kScatterWarps) {
             const int slot = q % Cfg::kSlots;
             if (!mbar_wait(&staged[slot], (uint32_t)(q / Cfg::kSlots) & 1u)) { ok = false; break; }
-            const int2 pd = pend[slot];
+            const int4 pd = pend[slot];
             uint8_t *At = smem + pd.x * Cfg::kStage;
+            if (pd.z >= 0) { // its B rows: gather g = lane, lane + 32, .. reads the 4 columns of lane g % 16
+                const int4 it = items[pd.z];
+                const TcJob &a = batch.job[it.w >> 16];
+                const int boxes = width(a) / Cfg::kBoxCols, n0 = (it.w & 0xffff) * width(a);
+                if (elect_one())
+                    mbar_arrive_expect_tx(&full[pd.x], (uint32_t)boxes * (kChunkCols * 128));
+                __syncwarp();
+                const int4 y = reinterpret_cast<const int4 *>(smem + Cfg::kColsOff + slot * kChunkCols * 4)[lane & 15];
+                const uint32_t b_s = smem_u32(At) + kATileBytes + (lane & 15) * 512;
+                for (int g = lane; g < 16 * boxes; g += 32)
+                    tma_gather4(b_s + (g >> 4) * (kChunkCols * 128), &a.tmap_b, n0 + (g >> 4) * Cfg::kBoxCols, y.x, y.y,
+                                y.z, y.w, &full[pd.x]);
+            }
 #pragma unroll 8
             for (int o = 0; o < kATileBytes / (16 * 32); o++)
                 reinterpret_cast<uint4 *>(At)[lane + o * 32] = make_uint4(0, 0, 0, 0);
