@@ -1152,6 +1152,19 @@ int build_plan(tca_plan *p, const int *row_ptr, const int *col, const __half *va
     std::vector<int2> cc_items, all_items;
     build_items(cc_list, h_rp, M, cc_items);
     build_items(h_all, h_rp, M, all_items);
+    auto longest = [&](int r0, int r1) {
+        int m = 0;
+        for (int r = r0; r < r1; r++) m = std::max(m, h_rp[r + 1] - h_rp[r]);
+        return m;
+    };
+    p->max_row = longest(0, M);
+    if (!cc_list.empty() && cc_list.back() - cc_list.front() + 1 == (int)cc_list.size()) {
+        p->cc_row0 = cc_list.front() * kWindowRows;
+        p->cc_row_end = std::min(M, (cc_list.back() + 1) * kWindowRows);
+        p->cc_base = h_rp[p->cc_row0];
+        p->cc_end = h_rp[p->cc_row_end];
+        p->cc_max_row = longest(p->cc_row0, p->cc_row_end);
+    }
     p->n_cc_items = (int)cc_items.size();
     p->n_all_items = (int)all_items.size();
 

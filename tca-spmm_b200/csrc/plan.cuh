@@ -68,6 +68,10 @@ struct tca_plan {
     int2 *cc_items = nullptr;
     int2 *all_items = nullptr;
     int n_cc_items = 0, n_all_items = 0;
+    // rows of the CUDA-core windows when those follow one another (else -1):
+    // sorted rows [cc_row0, cc_row_end), nonzeros [cc_base, cc_end), the
+    // longest of them, and the longest of all rows
+    int cc_row0 = -1, cc_row_end = 0, cc_base = 0, cc_end = 0, cc_max_row = 0, max_row = 0;
     // host copy of tile_first: chunk offsets of the tensor-core windows
     // (n_tc + 1), for sizing launches on the host
     std::vector<int> h_tile_first;

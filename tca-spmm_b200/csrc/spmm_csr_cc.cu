@@ -101,6 +101,7 @@ struct RowsJob {
     const __half *val, *B;
     void *C;
     int M, K, nnz, N, ldb, ldc;
+    int base;     // row_ptr[0]: the rows may be a part of a CSR
     int n_blocks; // blocks per N-slice
     float alpha, beta;
     unsigned flags;
@@ -123,6 +124,7 @@ __global__ void __launch_bounds__(kRowsThreads, 2) spmm_rows_kernel(const __grid
     constexpr int U = VEC ? 4 : W >= 8 ? 2 : W >= 4 ? 4 : 8; // nonzeros in flight per lane
     __shared__ int s_start[kRowsMax], s_pre[kRowsMax + 1], s_warp[kRowsThreads / 32], s_range[2];
     __shared__ __align__(16) float s_part[G * LPR * W];
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = lane & (LPR - 1), g = (int)threadIdx.x / LPR;
     const unsigned gmask = LPR == 32 ? 0xffffffffu : (((1u << LPR) - 1u) << (lane & ~(LPR - 1)));
     int jb = 0;
@@ -136,7 +138,7 @@ __global__ void __launch_bounds__(kRowsThreads, 2) spmm_rows_kernel(const __grid
     {
         constexpr int kProbes = kRowsThreads / 2;
         const int half = (int)threadIdx.x / kProbes, p = (int)threadIdx.x % kProbes, part = b + half;
-        const long long bound = ((long long)a.nnz + a.M) * part / a.n_blocks;
+        const long long bound = ((long long)a.nnz - a.base + a.M) * part / a.n_blocks + a.base;
         int lo = 0, len = part == 0 ? 0 : a.M; // the row is in [lo, lo + len]
         if (part == a.n_blocks) {
             lo = a.M;
@@ -373,6 +375,8 @@ __global__ void __launch_bounds__(kRowsThreads, 2) spmm_rows_kernel(const __grid
     }
     __syncthreads(); // the next rows reuse shared memory
     }
+    // beside a tensor-core launch: complete no earlier than it (as the stream kernel)
+    asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // Rows of plans, batched and streamed. Every job (one forward of one plan)
@@ -394,6 +398,7 @@ struct CcJob {
     const float *row_scale, *col_scale;
     int ldq;
     int n_items;
+    int slices; // > 1: an item is taken once per 32 W columns of N, by as many warps
     int M, K, N, ldb, ldc;
     float alpha, beta;
     unsigned flags;
@@ -468,7 +473,7 @@ template <int W> __device__ __forceinline__ void store_out(float *p, const float
 }
 
 struct ItemDesc {
-    int job, r0, nrows; // nrows == 0: no item
+    int job, r0, nrows; // nrows == 0: no item; job | N-slice << 8
 };
 
 template <typename Batch>
@@ -484,8 +489,9 @@ __device__ __forceinline__ ItemDesc load_desc(const Batch &b, int item)
             else
                 hi = mid - 1;
         }
-        const int2 it = __ldg(b.job[j].items + (item - b.item_start[j]));
-        d.job = j;
+        const int slices = b.job[j].slices, local = item - b.item_start[j];
+        const int2 it = __ldg(b.job[j].items + local / slices);
+        d.job = j | local % slices << 8;
         d.r0 = it.x;
         d.nrows = it.y - it.x;
     }
@@ -573,7 +579,7 @@ __global__ void __launch_bounds__(256, 3) spmm_cc_stream_kernel(const __grid_con
         orow = 0;
         sc = 0.f;
         if (lane <= d.nrows && d.nrows > 0) {
-            const CcJob &a = b.job[d.job];
+            const CcJob &a = b.job[d.job & 255];
             rs = __ldg(a.p_row_ptr + d.r0 + lane);
             if (lane < d.nrows) {
                 orow = __ldg(a.perm + d.r0 + lane);
@@ -594,7 +600,7 @@ __global__ void __launch_bounds__(256, 3) spmm_cc_stream_kernel(const __grid_con
         col = 0;
         val = 0;
         if (d.nrows > 0 && j0 + lane < j1) {
-            const CcJob &a = b.job[d.job];
+            const CcJob &a = b.job[d.job & 255];
             col = __ldg(a.p_col + j0 + lane);
             val = value(a, j0 + lane);
         }
@@ -619,7 +625,7 @@ __global__ void __launch_bounds__(256, 3) spmm_cc_stream_kernel(const __grid_con
         const ItemDesc d3 = load_desc(b, item + 3 * n_warps);
 
         // ---- item i
-        const CcJob &a = b.job[d0.job];
+        const CcJob &a = b.job[d0.job & 255];
         const int nrows = d0.nrows;
         const int j0 = __shfl_sync(full, rs0, 0), j1 = __shfl_sync(full, rs0, nrows);
         const bool keep = (a.flags & TCA_FLAG_KEEP_EMPTY_ROWS) != 0;
@@ -628,7 +634,8 @@ __global__ void __launch_bounds__(256, 3) spmm_cc_stream_kernel(const __grid_con
         // rows' B vectors in flight and no row-boundary tracking.
         const int rs_next = __shfl_down_sync(full, rs0, 1);
         const bool singles = __all_sync(full, lane >= nrows || rs_next - rs0 == 1);
-        for (int nb = 0; singles && nb < a.N; nb += 32 * W) {
+        const int nb0 = (d0.job >> 8) * 32 * W, nb1 = a.slices > 1 ? min(a.N, nb0 + 32 * W) : a.N;
+        for (int nb = nb0; singles && nb < nb1; nb += 32 * W) {
             const int n0 = nb + lane * W;
             const bool active = n0 < a.N;
             const uint8_t *Bn = F8 ? a.Bq + (active ? n0 : 0)
@@ -668,7 +675,7 @@ __global__ void __launch_bounds__(256, 3) spmm_cc_stream_kernel(const __grid_con
                 }
             }
         }
-        for (int nb = 0; !singles && nb < a.N; nb += 32 * W) {
+        for (int nb = nb0; !singles && nb < nb1; nb += 32 * W) {
             const int n0 = nb + lane * W;
             const bool active = n0 < a.N;
             const uint8_t *Bn = F8 ? a.Bq + (active ? n0 : 0)
@@ -772,7 +779,7 @@ RowsShape rows_shape(int N, bool vec)
 }
 int rows_blocks(const RowsJob &a, const RowsShape &sh, int slices) // per N-slice
 {
-    const long long groups = kRowsThreads / sh.lpr, keys = (long long)a.nnz + a.M;
+    const long long groups = kRowsThreads / sh.lpr, keys = (long long)a.nnz - a.base + a.M;
     const long long wave = 2 * kSMs; // resident blocks
     // whole waves over all slices (3001 x 1777 at 92 %, N = 203: 419 blocks, 1.4 waves, 41.6 us; 296 34.5 us)
     const long long waves = std::max(1LL, (keys * slices / (groups * 64) + wave / 2) / wave);
@@ -780,42 +787,52 @@ int rows_blocks(const RowsJob &a, const RowsShape &sh, int slices) // per N-slic
     return (int)std::max<long long>(1, std::min<long long>(n, a.M));
 }
 
+// beside: a programmatic dependent of the tensor-core launch before it (as
+// launch_stream_cap).
 template <typename OutT, int LPR, int W, bool VEC>
-int launch_rows(const RowsBatchT<kMaxCcJobs> &b, cudaStream_t s)
+int launch_rows(const RowsBatchT<kMaxCcJobs> &b, cudaStream_t s, bool beside)
 {
     const int grid = b.block_start[b.n_jobs];
     if (b.n_jobs == 0 || grid == 0)
         return TCA_OK;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3(kRowsThreads);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = beside ? 1 : 0;
     if (b.n_jobs == 1) {
         RowsBatchT<1> one;
         one.n_jobs = 1;
         one.block_start[0] = 0;
         one.block_start[1] = grid;
         one.job[0] = b.job[0];
-        spmm_rows_kernel<OutT, LPR, W, VEC, VEC, 1><<<grid, kRowsThreads, 0, s>>>(one);
+        TCA_CUDA_TRY(cudaLaunchKernelEx(&cfg, spmm_rows_kernel<OutT, LPR, W, VEC, VEC, 1>, one));
     } else {
-        spmm_rows_kernel<OutT, LPR, W, VEC, VEC, kMaxCcJobs><<<grid, kRowsThreads, 0, s>>>(b);
+        TCA_CUDA_TRY(cudaLaunchKernelEx(&cfg, spmm_rows_kernel<OutT, LPR, W, VEC, VEC, kMaxCcJobs>, b));
     }
-    TCA_CUDA_TRY(cudaGetLastError());
     return TCA_OK;
 }
 
 template <typename OutT>
-int launch_rows_shape(const RowsBatchT<kMaxCcJobs> &b, const RowsShape &sh, bool vec, cudaStream_t s)
+int launch_rows_shape(const RowsBatchT<kMaxCcJobs> &b, const RowsShape &sh, bool vec, cudaStream_t s, bool beside = false)
 {
     if (vec) {
         switch (sh.lpr) {
-        case 4: return launch_rows<OutT, 4, 8, true>(b, s);
-        case 8: return launch_rows<OutT, 8, 8, true>(b, s);
-        case 16: return launch_rows<OutT, 16, 8, true>(b, s);
-        default: return launch_rows<OutT, 32, 8, true>(b, s);
+        case 4: return launch_rows<OutT, 4, 8, true>(b, s, beside);
+        case 8: return launch_rows<OutT, 8, 8, true>(b, s, beside);
+        case 16: return launch_rows<OutT, 16, 8, true>(b, s, beside);
+        default: return launch_rows<OutT, 32, 8, true>(b, s, beside);
         }
     }
     switch (sh.w) {
-    case 1: return launch_rows<OutT, 32, 1, false>(b, s);
-    case 2: return launch_rows<OutT, 32, 2, false>(b, s);
-    case 4: return launch_rows<OutT, 32, 4, false>(b, s);
-    default: return launch_rows<OutT, 32, 8, false>(b, s);
+    case 1: return launch_rows<OutT, 32, 1, false>(b, s, beside);
+    case 2: return launch_rows<OutT, 32, 2, false>(b, s, beside);
+    case 4: return launch_rows<OutT, 32, 4, false>(b, s, beside);
+    default: return launch_rows<OutT, 32, 8, false>(b, s, beside);
     }
 }
 
@@ -963,7 +980,7 @@ int spmm_padded(const SpmmJob *sj, const int *row_ptr, const int *col, const __h
     k_pad_rows<<<(unsigned)((warps * 32 + 255) / 256), 256, 0, s>>>(B, K, N, ldb, Bp, ldp);
     TCA_CUDA_TRY(cudaGetLastError());
     if (!tc) {
-        RowsJob a{row_ptr, col, sj ? sj->p->perm : nullptr, val, Bp, C, M, K, nnz, N, ldp, ldc, 0, alpha, beta, flags};
+        RowsJob a{row_ptr, col, sj ? sj->p->perm : nullptr, val, Bp, C, M, K, nnz, N, ldp, ldc, 0, 0, alpha, beta, flags};
         return c_dtype == TCA_DTYPE_F16 ? rows_over_padded<__half>(a, s) : rows_over_padded<float>(a, s);
     }
     float *sums = reinterpret_cast<float *>(static_cast<char *>(ws.p) + b_bytes); // b_bytes: a multiple of 128
@@ -999,7 +1016,7 @@ int launch_spmm_csr_cc(const int *row_ptr, const int *col_idx, const __half *val
     RowsBatchT<kMaxCcJobs> b;
     b.n_jobs = 0;
     b.block_start[0] = 0;
-    RowsJob a{row_ptr, col_idx, nullptr, vals, B, C, M, K, nnz, N, ldb, ldc, 0, alpha, beta, flags};
+    RowsJob a{row_ptr, col_idx, nullptr, vals, B, C, M, K, nnz, N, ldb, ldc, 0, 0, alpha, beta, flags};
     rows_add(b, a, sh);
     return c_dtype == TCA_DTYPE_F16 ? launch_rows_shape<__half>(b, sh, vec, stream)
                                     : launch_rows_shape<float>(b, sh, vec, stream);
@@ -1066,7 +1083,7 @@ __global__ void __launch_bounds__(kMmaWarps * 32, 2) spmm_cc_mma_kernel(const __
         rs = 0;
         orow = 0;
         if (lane <= d.nrows && d.nrows > 0) {
-            const CcJob &a = b.job[d.job];
+            const CcJob &a = b.job[d.job & 255];
             rs = __ldg(a.p_row_ptr + d.r0 + lane);
             if (lane < d.nrows)
                 orow = __ldg(a.perm + d.r0 + lane);
@@ -1077,7 +1094,7 @@ __global__ void __launch_bounds__(kMmaWarps * 32, 2) spmm_cc_mma_kernel(const __
         col = 0;
         val = 0;
         if (d.nrows > 0 && j0 + lane < j1) {
-            const CcJob &a = b.job[d.job];
+            const CcJob &a = b.job[d.job & 255];
             col = __ldg(a.p_col + j0 + lane);
             val = __half_as_ushort(a.p_val[j0 + lane]);
         }
@@ -1098,7 +1115,7 @@ __global__ void __launch_bounds__(kMmaWarps * 32, 2) spmm_cc_mma_kernel(const __
         load_rows(d2, rs2, out2);
         const ItemDesc d3 = load_desc(b, item + 3 * n_warps);
 
-        const CcJob &a = b.job[d0.job];
+        const CcJob &a = b.job[d0.job & 255];
         const int R = d0.nrows;
         const int j0 = __shfl_sync(full, rs0, 0), j1 = __shfl_sync(full, rs0, R);
         const int Z = j1 - j0;
@@ -1333,6 +1350,9 @@ int launch_cc_typed(const CcBatch &b, int w, bool f8, int beside_regs, cudaStrea
 
 } // namespace
 
+// Fewer items than this leave warps of the stream kernel without one (16 warps per SM).
+constexpr int kFewItems = 16 * kSMs;
+
 int launch_cc_jobs(const SpmmJob *jobs, int n_jobs, int c_dtype, float alpha, float beta, unsigned flags,
                    cudaStream_t s, LaunchList *defer, int beside_regs)
 {
@@ -1341,19 +1361,30 @@ int launch_cc_jobs(const SpmmJob *jobs, int n_jobs, int c_dtype, float alpha, fl
         any = jobs[i].N > 0 && (!jobs[i].tc || jobs[i].p->n_cc_items > 0);
     if (!any)
         return TCA_OK;
-    // jobs whose operands do not allow 16-byte accesses (every window of the
-    // plan: the tensor-core kernel needs them too): the rows kernel
-    for (int w : {1, 2, 4, 8}) {
+    // The rows kernel takes the jobs whose operands do not allow 16-byte
+    // accesses (every window of the plan: the tensor-core kernel needs them
+    // too), and those whose few rows are long: a row of more than kItemNnz
+    // nonzeros is one warp's item in the stream kernel, a serial chain, which
+    // only many other items hide (the ragged last window of 401 x 2286 at 93 %,
+    // N = 624, 17 rows of 164: 66 us; 14 us here).
+    auto long_rows = [&](const SpmmJob &sj) {
+        const tca_plan *p = sj.p;
+        return !sj.f8 && sj.cc_w == 0 && vec_ok(sj.B, sj.ldb, sj.N, sj.C, sj.ldc, c_dtype) &&
+               (sj.tc ? p->cc_row0 >= 0 && p->cc_max_row > kItemNnz && p->n_cc_items < kFewItems
+                      : p->max_row > kItemNnz && p->n_all_items < kFewItems);
+    };
+    for (int kind : {1, 2, 4, 8, -4, -8, -16, -32}) { // columns per lane, or minus the lanes per row (16-byte accesses)
+        const int w = kind;
         RowsBatchT<kMaxCcJobs> b;
         b.n_jobs = 0;
         b.block_start[0] = 0;
         auto flush = [&]() -> int {
             if (b.n_jobs == 0)
                 return TCA_OK;
-            auto run = [c_dtype, w](const RowsBatchT<kMaxCcJobs> &bb, cudaStream_t st) {
-                const RowsShape sh{32, w};
-                return c_dtype == TCA_DTYPE_F16 ? launch_rows_shape<__half>(bb, sh, false, st)
-                                                : launch_rows_shape<float>(bb, sh, false, st);
+            auto run = [c_dtype, w, beside_regs](const RowsBatchT<kMaxCcJobs> &bb, cudaStream_t st) {
+                const RowsShape sh = w > 0 ? RowsShape{32, w} : RowsShape{-w, 8};
+                return c_dtype == TCA_DTYPE_F16 ? launch_rows_shape<__half>(bb, sh, w < 0, st, beside_regs > 0)
+                                                : launch_rows_shape<float>(bb, sh, w < 0, st, beside_regs > 0);
             };
             int status = TCA_OK;
             if (defer) {
@@ -1368,13 +1399,23 @@ int launch_cc_jobs(const SpmmJob *jobs, int n_jobs, int c_dtype, float alpha, fl
         for (int i = 0; i < n_jobs; i++) {
             const SpmmJob &sj = jobs[i];
             const tca_plan *p = sj.p;
-            if (sj.f8 || sj.N <= 0 || p->M == 0 || vec_ok(sj.B, sj.ldb, sj.N, sj.C, sj.ldc, c_dtype))
+            if (sj.f8 || sj.N <= 0 || p->M == 0)
                 continue;
-            const RowsShape sh = rows_shape(sj.N, false);
-            if (sh.w != w)
+            const bool vec = vec_ok(sj.B, sj.ldb, sj.N, sj.C, sj.ldc, c_dtype);
+            if (vec && !long_rows(sj))
+                continue;
+            const RowsShape sh = rows_shape(sj.N, vec);
+            if ((vec ? -sh.lpr : sh.w) != w)
                 continue;
             RowsJob a{p->p_row_ptr, p->p_col, p->perm, p->p_val, sj.B, sj.C, p->M, p->K, p->nnz, sj.N, sj.ldb, sj.ldc,
-                      0, alpha, beta, flags};
+                      0, 0, alpha, beta, flags};
+            if (vec && sj.tc) { // the rows of the CUDA-core windows
+                a.row_ptr += p->cc_row0;
+                a.perm += p->cc_row0;
+                a.M = p->cc_row_end - p->cc_row0;
+                a.nnz = p->cc_end;
+                a.base = p->cc_base;
+            }
             rows_add(b, a, sh);
             if (b.n_jobs == kMaxCcJobs)
                 TCA_TRY(flush());
@@ -1414,7 +1455,7 @@ int launch_cc_jobs(const SpmmJob *jobs, int n_jobs, int c_dtype, float alpha, fl
             if (n_items == 0 || sj.N <= 0)
                 continue;
             // E4M3 jobs always qualify (B is the library's own aligned copy; C was checked)
-            if (!sj.f8 && !vec_ok(sj.B, sj.ldb, sj.N, sj.C, sj.ldc, c_dtype))
+            if (!sj.f8 && (!vec_ok(sj.B, sj.ldb, sj.N, sj.C, sj.ldc, c_dtype) || long_rows(sj)))
                 continue;
             int w = (sj.cc_w == 2 || sj.cc_w == 4 || sj.cc_w == 8) ? sj.cc_w : pick_w(sj.N);
             if (sj.cc_w == kCcMma && !sj.f8)
@@ -1435,6 +1476,9 @@ int launch_cc_jobs(const SpmmJob *jobs, int n_jobs, int c_dtype, float alpha, fl
             a.col_scale = sj.col_scale;
             a.ldq = sj.ldq;
             a.n_items = n_items;
+            // few items: the slices of N go to different warps (with many, the
+            // repeated loads of an item's rows and nonzeros cost more)
+            a.slices = w != kCcMma && n_items < kFewItems ? (sj.N + 32 * w - 1) / (32 * w) : 1;
             a.M = p->M;
             a.K = p->K;
             a.N = sj.N;
@@ -1443,7 +1487,7 @@ int launch_cc_jobs(const SpmmJob *jobs, int n_jobs, int c_dtype, float alpha, fl
             a.alpha = alpha;
             a.beta = beta;
             a.flags = flags;
-            b.item_start[b.n_jobs + 1] = b.item_start[b.n_jobs] + a.n_items;
+            b.item_start[b.n_jobs + 1] = b.item_start[b.n_jobs] + a.n_items * a.slices;
             b.n_jobs++;
             if (b.n_jobs == kMaxCcJobs)
                 TCA_TRY(flush());
