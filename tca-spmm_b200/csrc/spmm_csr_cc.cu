@@ -514,6 +514,7 @@ struct CcJob {
     int ldq;
     int n_items;
     int slices; // > 1: an item is taken once per 32 W columns of N, by as many warps
+    int parts;  // > 1: its rows are cut among as many warps
     int M, K, N, ldb, ldc;
     float alpha, beta;
     unsigned flags;
@@ -588,7 +589,7 @@ template <int W> __device__ __forceinline__ void store_out(float *p, const float
 }
 
 struct ItemDesc {
-    int job, r0, nrows; // nrows == 0: no item; job | N-slice << 8
+    int job, r0, nrows; // job | N-slice << 8
 };
 
 template <typename Batch>
@@ -604,11 +605,13 @@ __device__ __forceinline__ ItemDesc load_desc(const Batch &b, int item)
             else
                 hi = mid - 1;
         }
-        const int slices = b.job[j].slices, local = item - b.item_start[j];
-        const int2 it = __ldg(b.job[j].items + local / slices);
+        const int slices = b.job[j].slices, parts = b.job[j].parts, local = item - b.item_start[j];
+        const int rest = local / slices, part = rest % parts;
+        const int2 it = __ldg(b.job[j].items + rest / parts);
+        const int rows = it.y - it.x, first = rows * part / parts;
         d.job = j | local % slices << 8;
-        d.r0 = it.x;
-        d.nrows = it.y - it.x;
+        d.r0 = it.x + first;
+        d.nrows = rows * (part + 1) / parts - first; // no rows: nothing to do in this part
     }
     return d;
 }
@@ -729,7 +732,7 @@ __global__ void __launch_bounds__(256, 3) spmm_cc_stream_kernel(const __grid_con
     load_rows(d1, rs1, out1, sc1);
     load_nz(d0, rs0, col0, val0);
 
-    while (d0.nrows > 0) {
+    while (item < b.item_start[b.n_jobs]) {
         // ---- pipeline: nonzeros of i+1, rows of i+2, descriptor of i+3
         int col1;
         unsigned short val1;
@@ -748,7 +751,7 @@ __global__ void __launch_bounds__(256, 3) spmm_cc_stream_kernel(const __grid_con
         // matrices): C[row] = alpha v B[col] (+ beta C[row]) row by row, with U
         // rows' B vectors in flight and no row-boundary tracking.
         const int rs_next = __shfl_down_sync(full, rs0, 1);
-        const bool singles = __all_sync(full, lane >= nrows || rs_next - rs0 == 1);
+        const bool singles = __all_sync(full, lane >= nrows || rs_next - rs0 == 1); // (also without rows)
         const int nb0 = (d0.job >> 8) * 32 * W, nb1 = a.slices > 1 ? min(a.N, nb0 + 32 * W) : a.N;
         for (int nb = nb0; singles && nb < nb1; nb += 32 * W) {
             const int n0 = nb + lane * W;
@@ -1489,11 +1492,12 @@ constexpr int kFewItems = 16 * kSMs;
 int launch_cc_jobs(const SpmmJob *jobs, int n_jobs, int c_dtype, float alpha, float beta, unsigned flags,
                    cudaStream_t s, LaunchList *defer, int beside_regs)
 {
-    bool any = false; // rows left for this path
-    for (int i = 0; i < n_jobs && !any; i++)
-        any = jobs[i].N > 0 && (!jobs[i].tc || jobs[i].p->n_cc_items > 0);
-    if (!any)
+    long long all_items = 0; // of all jobs: what fills the warps
+    for (int i = 0; i < n_jobs; i++)
+        if (jobs[i].N > 0) all_items += jobs[i].tc ? jobs[i].p->n_cc_items : jobs[i].p->n_all_items;
+    if (all_items == 0)
         return TCA_OK;
+    const bool few = all_items < kFewItems;
     // The rows kernel takes the jobs whose operands do not allow 16-byte
     // accesses (every window of the plan: the tensor-core kernel needs them
     // too), and those whose few rows are long: a row of more than kItemNnz
@@ -1503,8 +1507,7 @@ int launch_cc_jobs(const SpmmJob *jobs, int n_jobs, int c_dtype, float alpha, fl
     auto long_rows = [&](const SpmmJob &sj) {
         const tca_plan *p = sj.p;
         return !sj.f8 && sj.cc_w == 0 && vec_ok(sj.B, sj.ldb, sj.N, sj.C, sj.ldc, c_dtype) &&
-               (sj.tc ? p->cc_row0 >= 0 && p->cc_max_row > kItemNnz && p->n_cc_items < kFewItems
-                      : p->max_row > kItemNnz && p->n_all_items < kFewItems);
+               few && (sj.tc ? p->cc_row0 >= 0 && p->cc_max_row > kItemNnz : p->max_row > kItemNnz);
     };
     for (int kind : {1, 2, 4, 8, -4, -8, -16, -32}) { // columns per lane, or minus the lanes per row (16-byte accesses)
         const int w = kind;
@@ -1611,7 +1614,10 @@ int launch_cc_jobs(const SpmmJob *jobs, int n_jobs, int c_dtype, float alpha, fl
             a.n_items = n_items;
             // few items: the slices of N go to different warps (with many, the
             // repeated loads of an item's rows and nonzeros cost more)
-            a.slices = w != kCcMma && n_items < kFewItems ? (sj.N + 32 * w - 1) / (32 * w) : 1;
+            a.slices = w != kCcMma && few ? (sj.N + 32 * w - 1) / (32 * w) : 1;
+            // fewer still: their rows too (an item of 31 rows is a chain of 8
+            // rounds of loads: 4096 x 1024 at 80 %, N = 256, 290 items, 11.6 -> 5.1 us)
+            a.parts = w != kCcMma && few ? (int)std::max(1LL, std::min(4LL, kFewItems / (all_items * a.slices))) : 1;
             a.M = p->M;
             a.K = p->K;
             a.N = sj.N;
@@ -1620,7 +1626,7 @@ int launch_cc_jobs(const SpmmJob *jobs, int n_jobs, int c_dtype, float alpha, fl
             a.alpha = alpha;
             a.beta = beta;
             a.flags = flags;
-            b.item_start[b.n_jobs + 1] = b.item_start[b.n_jobs] + a.n_items * a.slices;
+            b.item_start[b.n_jobs + 1] = b.item_start[b.n_jobs] + a.n_items * a.slices * a.parts;
             b.n_jobs++;
             if (b.n_jobs == kMaxCcJobs)
                 TCA_TRY(flush());
