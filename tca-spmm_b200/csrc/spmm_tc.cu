@@ -44,8 +44,12 @@
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <algorithm>
+#include <climits>
+#include <functional>
 #include <memory>
 #include <mutex>
+#include <queue>
+#include <utility>
 #include <vector>
 #include "tca_internal.cuh"
 #include "plan.cuh"
@@ -92,14 +96,24 @@ struct TcJob {
 
 // A launch's jobs. The kernel is also built for CAP = 1: a single forward's
 // parameter block is then ~0.4 KB instead of ~12 KB (measured: the launch
-// took 5-15 us of host time with the full block).
+// took 5-15 us of host time with the full block); and for CAP = kOrdered,
+// whose block also carries the order of the items (9 KB more, 1 us of a
+// launch that does not need it).
+constexpr int kOrdered = kMaxJobs + 1;
 template <int CAP>
 struct TcBatchT {
+    static constexpr int kJobs = CAP == kOrdered ? kMaxJobs : CAP;
     int n_jobs;
-    int item_start[CAP + 1];
-    TcJob job[CAP];
+    int item_start[kJobs + 1];
+    TcJob job[kJobs];
+    // Item k of CTA b: b + k * gridDim.x; kOrdered: order[k * gridDim.x + b]
+    // (kNoItem: no more), which the host dealt so that the CTAs end together
+    // (schedule_items).
+    uint16_t order[CAP == kOrdered ? kMaxCtaItems * kSMs : 1];
 };
 using TcBatch = TcBatchT<kMaxJobs>;
+using TcOrdered = TcBatchT<kOrdered>;
+constexpr uint16_t kNoItem = 0xffffu;
 
 using namespace ptx;
 
@@ -301,8 +315,8 @@ __device__ __forceinline__ void store_rows(uint32_t acc, OutT *C, int ldc, int o
     }
 }
 
-// Persistent CTAs, one per SM: CTA b processes work items b, b + gridDim.x,
-// ... (at most kMaxCtaItems), as one continuous stream of total_chunks chunks
+// Persistent CTAs, one per SM: CTA b processes its work items (TcBatchT; at
+// most kMaxCtaItems), as one continuous stream of total_chunks chunks
 // through the stage ring; every role runs over exactly those chunks. Roles
 // (kThreads threads):
 //   warps 0 and 1 (loaders of B and of A): a TMA instruction takes its issuer
@@ -372,11 +386,12 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
 
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int total = batch.item_start[batch.n_jobs];
-    const int n_items = blockIdx.x < total ? min(kMaxCtaItems, (total - 1 - (int)blockIdx.x) / (int)gridDim.x + 1) : 0;
+    // this CTA's items (kOrdered: counted by the loaders, below)
+    int n_items = blockIdx.x < total ? min(kMaxCtaItems, (total - 1 - (int)blockIdx.x) / (int)gridDim.x + 1) : 0;
     // a job's N-slice width: a single forward runs in the kernel of its own width
     auto width = [](const TcJob &a) { return CAP == 1 ? NT : a.nt; };
     if (smem_u32(smem) & 1023u) { // the swizzled tiles and TMA destinations need a 1024-byte aligned base
-        if (threadIdx.x == 0 && n_items > 0)
+        if (threadIdx.x == 0 && total > 0)
             atomicOr(batch.job[0].status, kStatusLayout);
         return;
     }
@@ -414,8 +429,15 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
         // their way during the rest of the set-up (a chain of cold misses:
         // parameters, window list, chunk lists, then the data).
         int z = 0;
+        int item = (int)blockIdx.x + lane * (int)gridDim.x;
+        if constexpr (CAP == kOrdered) {
+            item = batch.order[lane * (int)gridDim.x + (int)blockIdx.x];
+            n_items = __popc(__ballot_sync(0xffffffffu, item != kNoItem));
+            if (lane == 0)
+                cum[kMaxCtaItems + 1] = n_items;
+        }
         if (lane < n_items) {
-            const int4 it = decode_item(batch, blockIdx.x + lane * gridDim.x);
+            const int4 it = decode_item(batch, item);
             items[lane] = it;
             z = it.z;
         }
@@ -451,6 +473,8 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    if constexpr (CAP == kOrdered)
+        n_items = cum[kMaxCtaItems + 1];
     if constexpr (F8) {
         asm volatile("griddepcontrol.wait;" ::: "memory"); // B is quantized
         asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -1557,6 +1581,55 @@ int tc_block_regs(bool f8, int *regs)
     return TCA_OK;
 }
 
+namespace {
+
+// Time of an item: its chunks by the width of its slice, and its epilogue
+// (units of 25 ns: 0.40, 0.27 and 0.25 us a chunk, 2.5 us; %clock traces).
+int item_cost(int chunks, int n_tile) { return chunks * (n_tile == 256 ? 16 : n_tile == 128 ? 11 : 10) + 100; }
+
+// Deals a launch's items to its CTAs, the longest first, each to the CTA with
+// the least so far, when there is more than one round of them and they differ
+// by a quarter.
+// Round-robin left 24 layers of mixed shapes with CTAs ending between 9 and 36
+// us (43.0 us a replay, 39.3 dealt out); a launch of about equal items keeps it
+// (false).
+bool schedule_items(const TcBatch &b, const SpmmJob *const *jobs, std::vector<uint16_t> &order)
+{
+    const int total = b.item_start[b.n_jobs];
+    if (b.n_jobs < 2 || total <= kSMs || total > kSMs * kMaxCtaItems)
+        return false;
+    std::vector<std::pair<int, int>> items; // -cost, item
+    items.reserve((size_t)total);
+    int lo = INT_MAX, hi = 0;
+    for (int j = 0; j < b.n_jobs; j++) {
+        const std::vector<int> &first = jobs[j]->p->h_tile_first;
+        for (int t = 0; t < jobs[j]->p->n_tc; t++) {
+            const int c = item_cost(first[t + 1] - first[t], b.job[j].nt);
+            lo = std::min(lo, c);
+            hi = std::max(hi, c);
+            for (int n = 0; n < b.job[j].ntiles; n++)
+                items.emplace_back(-c, b.item_start[j] + t * b.job[j].ntiles + n);
+        }
+    }
+    if (4 * hi < 5 * lo) // nearly equal: neighbours in time stay neighbours in a problem
+        return false;
+    std::sort(items.begin(), items.end());
+    order.assign((size_t)kMaxCtaItems * kSMs, kNoItem);
+    int count[kSMs] = {};
+    using Load = std::pair<int, int>; // time so far, CTA
+    std::priority_queue<Load, std::vector<Load>, std::greater<Load>> ctas;
+    for (int c = 0; c < kSMs; c++) ctas.emplace(0, c);
+    for (const auto &it : items) { // at most kMaxCtaItems each: a full CTA leaves the queue
+        const Load l = ctas.top();
+        ctas.pop();
+        order[count[l.second] * kSMs + l.second] = (uint16_t)it.second;
+        if (++count[l.second] < kMaxCtaItems) ctas.emplace(l.first - it.first, l.second);
+    }
+    return true;
+}
+
+} // namespace
+
 // A window alone on a CTA pair keeps two SMs for one window's chunks, so the
 // pair kernel takes a plan when at least two thirds of its tensor-core
 // windows are paired.
@@ -1604,9 +1677,9 @@ int launch_tc_jobs(const SpmmJob *jobs, int n_jobs, int c_dtype, float alpha, fl
     // launches run one after the other, each with its own set-up and its own
     // partly filled last round (24 layers with N of 64 to 1024: three launches
     // 73.9 us, one 43.5 us). Jobs with more chunks per item first: rounds of
-    // equal items, the short ones last, to fill the CTAs evenly.
-    auto cost = [](const SpmmJob &j) { // of one item: chunks, weighted by the width of the slice
-        return (long long)(j.p->n_tc_chunks / std::max(1, j.p->n_tc)) * (j.n_tile + 128);
+    // equal items, the short ones last (schedule_items deals them out).
+    auto cost = [](const SpmmJob &j) { // of one item, on average
+        return item_cost(j.p->n_tc_chunks / std::max(1, j.p->n_tc), j.n_tile);
     };
     for (bool f8 : {false, true}) {
         for (bool pair : {false, true}) {
@@ -1630,6 +1703,21 @@ int launch_tc_jobs(const SpmmJob *jobs, int n_jobs, int c_dtype, float alpha, fl
                     b.item_start[b.n_jobs + 1] = b.item_start[b.n_jobs] + units * b.job[b.n_jobs].ntiles;
                     b.n_jobs++;
                     if (!pair) NT = std::max(NT, sj.n_tile);
+                }
+                std::vector<uint16_t> order;
+                if (!pair && schedule_items(b, &sel[i0], order)) {
+                    auto held = std::make_shared<TcOrdered>();
+                    held->n_jobs = b.n_jobs;
+                    std::copy(b.item_start, b.item_start + kMaxJobs + 1, held->item_start);
+                    std::copy(b.job, b.job + b.n_jobs, held->job);
+                    std::copy(order.begin(), order.end(), held->order);
+                    if (!defer)
+                        TCA_TRY(launch_typed(*held, NT, f8, c_dtype, dependent, s));
+                    else
+                        defer->push_back([held, NT, f8, c_dtype, dependent](cudaStream_t st) {
+                            return launch_typed(*held, NT, f8, c_dtype, dependent, st);
+                        });
+                    continue;
                 }
                 TCA_TRY(emit(b, NT, f8));
             }
