@@ -1617,7 +1617,13 @@ int launch_cc_jobs(const SpmmJob *jobs, int n_jobs, int c_dtype, float alpha, fl
             a.slices = w != kCcMma && few ? (sj.N + 32 * w - 1) / (32 * w) : 1;
             // fewer still: their rows too (an item of 31 rows is a chain of 8
             // rounds of loads: 4096 x 1024 at 80 %, N = 256, 290 items, 11.6 -> 5.1 us)
-            a.parts = w != kCcMma && few ? (int)std::max(1LL, std::min(4LL, kFewItems / (all_items * a.slices))) : 1;
+            // With a few rounds of items the last, partial round counts: halves
+            // (32 problems, 5,056 items on 2,368 warps: the step 48.2 -> 46.6
+            // us; thirds 48.5: the loads ahead no longer cover an item).
+            a.parts = w == kCcMma            ? 1
+                      : few                  ? (int)std::max(1LL, std::min(4LL, kFewItems / (all_items * a.slices)))
+                      : all_items < 4LL * kFewItems ? 2
+                                             : 1;
             a.M = p->M;
             a.K = p->K;
             a.N = sj.N;
