@@ -71,7 +71,10 @@ TCA_API const char *tca_status_string(int status);
  * Replaces the device part of our_spmm_balanced (src/our_spmm.cu:472-588,
  * kernel at :290-346) without the per-call host schedule
  * (workload_manager, :347-471). N % 8 == 0 with 16-byte aligned B and C rows
- * takes the vectorised path; any other N or alignment a scalar one.        */
+ * takes the vectorised path. Any other N or alignment goes through an aligned
+ * copy of B in stream-ordered memory of the library's pool where nnz * N >=
+ * 2^25 (given back in stream order; not under stream capture, and never more
+ * than 64 MiB), else through a two-byte path.                              */
 /* ------------------------------------------------------------------ */
 TCA_API int tca_spmm_csr(const int *d_row_ptr, const int *d_col_idx, const void *d_vals_f16,
                  int M, int K, int nnz,
@@ -171,7 +174,13 @@ TCA_API int tca_plan_destroy(tca_plan_t plan);
  * tensor-core kernel over the plan's tensor-core windows and the CUDA-core
  * kernel over the rest, in that order, on `stream`. N % 8 == 0, ldb % 8 == 0,
  * ldc * sizeof(C) % 16 == 0 and 16-byte aligned B and C are needed for the
- * tensor-core kernel; otherwise every window runs on CUDA cores.
+ * tensor-core kernel on the operands as they are. Otherwise, where nnz * N >=
+ * 2^25 and the call is not being captured, B is first copied to aligned rows
+ * (stream-ordered memory of the library's pool, at most 64 MiB): with FP16 C
+ * and tensor-core windows the forward runs as usual into FP32 sums (at most 64
+ * MiB more) that are rounded into C once, unless B holds an infinity or NaN,
+ * and with FP32 C every window runs on CUDA cores over the copy. Without the
+ * copy every window runs on CUDA cores.
  * Replaces the device work of our_spmm_balanced (src/our_spmm.cu:547-559). */
 TCA_API int tca_spmm(tca_plan_t plan, const void *d_B_f16, int ldb, int N,
              void *d_C, int ldc, int c_dtype, float alpha, float beta,
@@ -197,9 +206,9 @@ typedef struct tca_batch_item {
 } tca_batch_item_t;
 
 /* Forwards of many plans (layers of different shapes and sparsity) in a
- * handful of launches: one tensor-core launch per N-slice width over every
- * item's tensor-core windows, then one CUDA-core launch per row width over
- * every item's remaining rows (at most 32 items per launch). Same results as
+ * handful of launches: one tensor-core launch over every item's tensor-core
+ * windows, whatever their N-slice widths, then one CUDA-core launch per row
+ * width over every item's remaining rows (at most 32 items per launch). Same results as
  * calling tca_spmm per item. events: as in tca_spmm_events (may be NULL).
  * No device memory is allocated: the work list travels as kernel parameters,
  * so the call can be captured in a CUDA graph. */
@@ -211,10 +220,10 @@ TCA_API int tca_spmm_batched(const tca_batch_item_t *items, int n_items, int c_d
 /* ------------------------------------------------------------------ */
 /* dA on A's pattern (SDDMM): out[j] = alpha * sum_n dY[r_j, n] * B[c_j, n]
  * for every nonzero j in the caller's CSR order; dY is M x N (ldy), B is
- * K x N (ldb), out is nnz values of out_dtype (F16 or F32). Where A is dense
- * enough (and M * K * 4 <= 256 MiB) it computes dY B^T with one cuBLAS GEMM
- * into stream-ordered scratch from the library's pool and samples it; else a
- * sparse kernel; FP32 accumulation either way. */
+ * K x N (ldb), out is nnz values of out_dtype (F16 or F32). Tiles of dY B^T on
+ * the tensor cores for the tensor-core windows (parts of the n range, where it
+ * is cut, are summed in a fixed order from stream-ordered memory of the
+ * library's pool), a warp per row elsewhere; FP32 accumulation either way. */
 TCA_API int tca_sddmm(tca_plan_t plan, const void *d_dY_f16, int ldy, const void *d_B_f16, int ldb, int N,
                       void *d_out, int out_dtype, float alpha, tca_stream_t stream);
 /* dB = alpha * A^T dY + beta * dB (dY M x N, dB K x N of dB_dtype). Runs the
@@ -269,10 +278,9 @@ TCA_API int tca_spmm_fp8_batched(const tca_batch_item_t *items, int n_items, int
  * The first call on each device looks up the array's device address; make
  * that first call before any stream capture. The address is kept for the
  * process: after a cudaDeviceReset of a device, do not call this on that
- * device again. Every call on a device shares the one array (the call clears
- * what it needs cleared): calls whose work overlaps on the GPU -- on
- * different streams, or from different threads -- race and give wrong
- * results. K == 0 writes C = beta * C through tca_spmm (no quantization, no
+ * device again. Every call on a device shares the one array (nothing in it
+ * outlives a call): calls whose work overlaps on the GPU -- on different
+ * streams, or from different threads -- race and give wrong results. K == 0 writes C = beta * C through tca_spmm (no quantization, no
  * allocation). Otherwise as tca_spmm_fp8, with the same launches. */
 #define TCA_FP8_STATIC_SCRATCH_BYTES (16u << 20)
 TCA_API int tca_spmm_fp8_static(tca_plan_t plan, const void *d_B_f16, int ldb, int N, void *d_C, int ldc, int c_dtype,

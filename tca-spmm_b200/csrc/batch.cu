@@ -9,13 +9,12 @@
 //
 // The autotuner picks, per item, the tensor-core N-slice width (n_tile) and
 // the CUDA-core columns per lane (cc_cols) by timing each candidate on the
-// item alone with CUDA events (median of a few runs). Items with different
-// picks run in different launches, and launches of a batch run one after the
-// other, so the per-item picks are then weighed as a whole against every
-// uniform (n_tile, cc_cols) -- one tensor-core and one CUDA-core launch --
-// by replaying each as a captured graph; the fastest is written back into
-// the items (measured on a 24-layer batch: per-item picks in 3 launches
-// 157 us, one uniform configuration in 2 launches 123 us). The reference has
+// item alone with CUDA events (median of a few runs). Items of all n_tile share
+// a tensor-core launch, but items with different cc_cols run in different
+// CUDA-core launches, and an item's best width alone need not be its best in a
+// batch that fills the GPU, so the per-item picks are then weighed as a whole
+// against every uniform (n_tile, cc_cols) by replaying each as a captured
+// graph; the fastest is written back into the items. The reference has
 // neither (its launch geometry is fixed by workload_manager,
 // src/our_spmm.cu:347-471).
 #include <algorithm>

@@ -95,7 +95,7 @@ constexpr int kMaxQJobs = 32;
 struct QJob {
     const __half *B;
     uint8_t *Bq;
-    unsigned *colmax; // column maxima as FP32 bit patterns, then the scales (in place)
+    unsigned *scale; // column scales (FP32 bit patterns)
     int ldb, ldq, K, N;
 };
 struct QBatch {
@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(256, 4) k_quant_b(const __grid_constant__ QBat
         const float sc = scale_of(v);
         s_scale[threadIdx.x] = sc;
         if (rank == 0 && n0 + (int)threadIdx.x < q.N)
-            q.colmax[n0 + threadIdx.x] = __float_as_uint(sc);
+            q.scale[n0 + threadIdx.x] = __float_as_uint(sc);
     }
     ptx::cluster_sync_all(); // the scales are there; no block of the cluster reads another's maxima any more
     if (n >= q.N)
@@ -495,8 +495,7 @@ int tca_spmm_fp8_batched(const tca_batch_item_t *items, int n_items, int c_dtype
 // loads it and held until the process exits.
 //
 // Layout of the scratch for one call: Bq (K rows of ldq = N rounded up to 16
-// bytes), rounded up to 256 bytes, then ldq FP32 words that first hold the
-// column maxima (cleared by the call itself) and then the column scales.
+// bytes), rounded up to 256 bytes, then ldq FP32 column scales.
 // ---------------------------------------------------------------------------
 static __device__ __align__(256) unsigned char g_fp8_scratch[TCA_FP8_STATIC_SCRATCH_BYTES];
 

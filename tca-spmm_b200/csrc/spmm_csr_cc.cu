@@ -990,10 +990,14 @@ __global__ void __launch_bounds__(256) k_pad_rows(const __half *__restrict__ src
 
 // C = alpha * S + beta * C from FP32 sums S (rows of lds), FP16 C of any
 // alignment; rows without nonzeros are skipped with KEEP_EMPTY_ROWS. A warp
-// per 256 columns of a sorted row.
+// per 256 columns of a sorted row. A tile product multiplies a row's zeros by
+// the chunk's other rows of B as well, so an infinity or NaN in B reaches the
+// sums of rows that hold no nonzero of its column: a sum that is not finite is
+// formed anew from the row's nonzeros and the padded B (rows of lds).
 __global__ void __launch_bounds__(256)
 k_unpad_rows(const float *__restrict__ sums, int lds, const int *__restrict__ perm, const int *__restrict__ p_row_ptr,
-             int M, int N, __half *__restrict__ C, int ldc, float alpha, float beta, unsigned flags)
+             const int *__restrict__ p_col, const __half *__restrict__ p_val, const __half *__restrict__ B, int M,
+             int N, __half *__restrict__ C, int ldc, float alpha, float beta, unsigned flags)
 {
     const int slices = (N + 255) / 256, lane = threadIdx.x & 31;
     const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -1011,6 +1015,11 @@ k_unpad_rows(const float *__restrict__ sums, int lds, const int *__restrict__ pe
         if (n0 + u * 32 >= N)
             break;
         __half *c = C + r * ldc + n0 + u * 32;
+        if (!isfinite(v[u])) {
+            v[u] = 0.f;
+            for (int j = __ldg(p_row_ptr + i); j < __ldg(p_row_ptr + i + 1); j++)
+                v[u] = fmaf(__half2float(p_val[j]), __half2float(B[(size_t)p_col[j] * lds + n0 + u * 32]), v[u]);
+        }
         float o = alpha * v[u];
         if (beta != 0.f) o = fmaf(beta, __half2float(*c), o);
         *c = __float2half_rn(o);
@@ -1127,7 +1136,7 @@ int spmm_padded(const SpmmJob *sj, const int *row_ptr, const int *col, const __h
     TCA_TRY(run_jobs_with_events(&job, 1, TCA_DTYPE_F32, 1.f, 0.f, 0u, s, nullptr));
     const long long out_warps = (long long)M * ((N + 255) / 256);
     k_unpad_rows<<<(unsigned)((out_warps * 32 + 255) / 256), 256, 0, s>>>(
-        sums, ldp, sj->p->perm, sj->p->p_row_ptr, M, N, static_cast<__half *>(C), ldc, alpha, beta, flags);
+        sums, ldp, sj->p->perm, row_ptr, col, val, Bp, M, N, static_cast<__half *>(C), ldc, alpha, beta, flags);
     TCA_CUDA_TRY(cudaGetLastError());
     return TCA_OK;
 }

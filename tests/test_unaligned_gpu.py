@@ -91,3 +91,30 @@ def test_unaligned_capture(cuda):
     mag = np.abs(A) @ np.abs(Bh.astype(np.float64))
     d = np.abs(C.cpu().numpy().astype(np.float64) - eager.cpu().numpy())
     assert np.all(d <= 2 * n_r * 2.0 ** -23 * mag + 2.0 ** -10 * np.abs(A @ Bh.astype(np.float64)) + 2.0 ** -23)
+
+
+@pytest.mark.parametrize("bad", [float("inf"), float("-inf"), float("nan")])
+@pytest.mark.parametrize("out", ["f16", "f32"])
+def test_unaligned_nonfinite(cuda, bad, out):
+    """An infinity or NaN in B reaches the rows that hold a nonzero of its
+    column and no other, as in forwards without a copy."""
+    M, K, N = 700, 1100, 99
+    (rp, ci, v), Bh, A, n_r = case(M, K, N, 0.5, cuda, 5)
+    clean = np.zeros((M, N), dtype=bool)
+    clean[:] = (A[:, 17] == 0)[:, None]
+    clean[:, np.arange(N) != 40] = True
+    b64 = Bh.astype(np.float64)
+    ref, mag = A @ b64, np.abs(A) @ np.abs(b64)
+    Bh[17, 40] = bad
+    dt = torch.float16 if out == "f16" else torch.float32
+    C = torch.full((M, N), 0.5, dtype=dt, device=cuda)
+    tca_spmm.Plan(rp, ci, v, K).spmm(torch.from_numpy(Bh).to(cuda), out=C, alpha=2.0, beta=0.5)
+    got, want = C.cpu().numpy().astype(np.float64), 2 * ref + 0.25
+    tol = 2 * n_r * 2.0 ** -23 * mag + 2.0 ** -23 * np.abs(want)
+    if out == "f16":
+        tol = tol + 2.0 ** -11 * np.abs(want) + 2.0 ** -24
+    assert np.all(np.abs(got - want)[clean] <= tol[clean])
+    hit = got[~clean]
+    assert hit.size and not np.isfinite(hit).any()
+    if np.isinf(bad):
+        assert np.all(np.sign(hit) == np.sign(bad * A[:, 17][A[:, 17] != 0]))
