@@ -6,7 +6,7 @@
 // using mma.sync as a dot-product engine.
 //
 // Kernels:
-//   * spmm_rows_kernel: straight from a CSR, blocks of strided rows whose
+//   * spmm_rows_kernel: straight from a CSR, blocks of consecutive rows whose
 //     nonzeros are cut into equal runs -- the plan-free forward
 //     (tca_spmm_csr), and planned forwards whose dense operands are not
 //     16-byte aligned;
@@ -81,7 +81,7 @@ constexpr int kMaxCcJobs = 32;
 //
 // A row of a skewed matrix can hold every column (one group of lanes walking
 // 1024 nonzeros took 120 us), so no row belongs to one group. Block b takes
-// the rows whose key row_ptr[r] + r lies in the b-th of equal parts (found by a
+// the rows whose key row_ptr[r] + w * r lies in the b-th of equal parts (found by a
 // 32-way search: rows and nonzeros are both balanced, whatever the order of
 // the rows) and cuts their nonzeros, laid end to end, into equal runs, one per
 // group of LPR lanes. A group writes the rows that lie in its run; of a row
@@ -93,6 +93,14 @@ constexpr int kMaxCcJobs = 32;
 // checked, as everywhere in this file.
 // ---------------------------------------------------------------------------
 constexpr int kRowsThreads = 512;
+// A row's weight beside a nonzero's in the cut: sorted rows lie with others of
+// their length, so by nonzeros alone the last blocks hold hundreds of short
+// rows, whose writes and offsets cost more than their nonzeros (2048 x 2048,
+// Zipf rows of 5 %, N = 301: 113 us, 61 with weight 4, 49 with 8; 4096 x 1024
+// at 20 %, N = 201: 113, 85, 79, and 78 with 16). In the caller's order long
+// and short rows mix and the weight gives as often as it takes (1024 x 1024,
+// N = 256: 33 -> 27 us; 1500 x 900, N = 301: 48 -> 56).
+constexpr long long kSortedRowKey = 8;
 constexpr int kRowsMax = kRowsThreads; // rows in shared memory at a time: a thread each
 
 struct RowsJob {
@@ -133,12 +141,13 @@ __global__ void __launch_bounds__(kRowsThreads, 2) spmm_rows_kernel(const __grid
     const int local = (int)blockIdx.x - batch.block_start[jb];
     const int slice = local / a.n_blocks, b = local - slice * a.n_blocks;
 
+    const long long row_key = a.perm ? kSortedRowKey : 1;
     // this block's rows: each half of the threads finds the first row whose
     // key is at least its bound, kRowsThreads / 2 probes at a time
     {
         constexpr int kProbes = kRowsThreads / 2;
         const int half = (int)threadIdx.x / kProbes, p = (int)threadIdx.x % kProbes, part = b + half;
-        const long long bound = ((long long)a.nnz - a.base + a.M) * part / a.n_blocks + a.base;
+        const long long bound = ((long long)a.nnz - a.base + row_key * a.M) * part / a.n_blocks + a.base;
         int lo = 0, len = part == 0 ? 0 : a.M; // the row is in [lo, lo + len]
         if (part == a.n_blocks) {
             lo = a.M;
@@ -150,7 +159,7 @@ __global__ void __launch_bounds__(kRowsThreads, 2) spmm_rows_kernel(const __grid
             __syncthreads();
             if (p * step < len) {
                 const int r = lo + p * step;
-                if ((long long)min(max(__ldg(a.row_ptr + r), 0), a.nnz) + r >= bound) atomicMin(&s_range[half], p);
+                if ((long long)min(max(__ldg(a.row_ptr + r), 0), a.nnz) + row_key * r >= bound) atomicMin(&s_range[half], p);
             }
             __syncthreads();
             const int first = s_range[half];
