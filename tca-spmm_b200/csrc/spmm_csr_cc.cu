@@ -101,6 +101,16 @@ constexpr int kRowsThreads = 512;
 // and short rows mix and the weight gives as often as it takes (1024 x 1024,
 // N = 256: 33 -> 27 us; 1500 x 900, N = 301: 48 -> 56).
 constexpr long long kSortedRowKey = 8;
+// U nonzeros that lie in one row and whose columns are valid, as almost all do,
+// need neither predicates nor zeros for absent loads: 16 warp instructions per
+// nonzero instead of 50 (4096 x 4096 at 95 %, N = 512: 118 -> 82 us; 4096 x 1024
+// at 80 %, Zipf, N = 256: 73 -> 53 us, 8.1 TB/s of B rows from L2; 3001 x 1777, N =
+// 203: 40 -> 29 us). Groups of fewer lanes meet too many row ends side by side
+// in a warp, which then runs both paths (300 x 4096, N = 32: 23.4 us without, 27.8
+// with), and so do groups of 16 lanes where rows are short on average (4096 x
+// 1024 at 5 %, Zipf, 51 per row, N = 128: 24.4 without, 25.0 with; 4096 x 4096 at
+// 90 %, N = 99: 76 without, 58 with).
+constexpr int kFastLpr = 16, kFastMean = 64;
 constexpr int kRowsMax = kRowsThreads; // rows in shared memory at a time: a thread each
 
 struct RowsJob {
@@ -124,7 +134,7 @@ template <int CAP> struct RowsBatchT {
 // B read in 16-byte accesses (16-byte aligned rows of at least N rounded up to
 // 8 columns), C written so too with VC (N % 8 == 0, 16-byte aligned rows);
 // else every LPR-th column.
-template <typename OutT, int LPR, int W, bool VEC, bool VC, int CAP>
+template <typename OutT, int LPR, int W, bool VEC, bool VC, int CAP, bool FAST>
 __global__ void __launch_bounds__(kRowsThreads, 2) spmm_rows_kernel(const __grid_constant__ RowsBatchT<CAP> batch)
 {
     static_assert(!VEC || W == 8, "16-byte accesses cover 8 columns");
@@ -278,6 +288,9 @@ __global__ void __launch_bounds__(kRowsThreads, 2) spmm_rows_kernel(const __grid
             ce = cr < n_rows ? s_pre[cr + 1] : 0x7fffffff;
         };
         const __half *Bn = a.B + n0;
+        // lanes past N read the first columns instead; their sums go nowhere
+        const char *Bs = reinterpret_cast<const char *>(a.B + (col_ok(0) ? n0 : 0));
+        const unsigned ldb_bytes = 2u * (unsigned)a.ldb;
         // nonzero of this lane in the LPR from `base` on
         auto load_nz = [&](int base, int &c, unsigned short &x) {
             c = -1;
@@ -304,7 +317,28 @@ __global__ void __launch_bounds__(kRowsThreads, 2) spmm_rows_kernel(const __grid
             x = xn;
             load_nz(base + LPR, cn, xn);
             const int cnt = min(LPR, v1 - base);
+            // no malformed columns: U nonzeros of one row take the short path
+            const bool valid = FAST && !__any_sync(gmask, sub < cnt && c < 0);
             for (int t = 0; t < cnt; t += U) {
+                if constexpr (FAST) {
+                    if (valid && t + U <= cnt && base + t + U <= ce) {
+                        uint4 bv[U];
+                        unsigned short xf[U];
+#pragma unroll
+                        for (int u = 0; u < U; u++) {
+                            const unsigned cf = (unsigned)__shfl_sync(gmask, c, t + u, LPR);
+                            xf[u] = (unsigned short)__shfl_sync(gmask, (int)x, t + u, LPR);
+                            bv[u] = __ldg(reinterpret_cast<const uint4 *>(Bs + (unsigned long long)cf * ldb_bytes));
+                        }
+#pragma unroll
+                        for (int u = 0; u < U; u++) {
+                            const unsigned short *h = reinterpret_cast<const unsigned short *>(&bv[u]);
+#pragma unroll
+                            for (int w = 0; w < 8; w++) acc[w] = ptx::fma_f16_f32(xf[u], h[w], acc[w]);
+                        }
+                        continue;
+                    }
+                }
                 int cu[U];
                 unsigned short xu[U];
 #pragma unroll
@@ -409,6 +443,9 @@ __global__ void __launch_bounds__(kRowsThreads, 2) spmm_rows_short_kernel(const 
     const int n0 = (int)blockIdx.y * LPR * 8 + sub * 8;
     const bool active = n0 < a.N;
     const __half *Bn = a.B + n0;
+    // lanes past N read the first columns instead; their sums go nowhere
+    const char *Bs = reinterpret_cast<const char *>(a.B + (active ? n0 : 0));
+    const unsigned ldb_bytes = 2u * (unsigned)a.ldb;
     if (threadIdx.x == 0)
         s_n = 0;
     __syncthreads();
@@ -429,8 +466,25 @@ __global__ void __launch_bounds__(kRowsThreads, 2) spmm_rows_short_kernel(const 
                 if (c < 0 || c >= a.K) { c = -1; x = 0; }
             }
             const int cnt = min(LPR, end - base);
+            const bool valid = LPR >= kFastLpr && !__any_sync(gmask, sub < cnt && c < 0); // no malformed columns
             for (int t = 0; t < cnt; t += U) {
                 uint4 bv[U];
+                if (valid && t + U <= cnt) {
+                    unsigned short xf[U];
+#pragma unroll
+                    for (int u = 0; u < U; u++) {
+                        const unsigned cf = (unsigned)__shfl_sync(gmask, c, t + u, LPR);
+                        xf[u] = (unsigned short)__shfl_sync(gmask, (int)x, t + u, LPR);
+                        bv[u] = __ldg(reinterpret_cast<const uint4 *>(Bs + (unsigned long long)cf * ldb_bytes));
+                    }
+#pragma unroll
+                    for (int u = 0; u < U; u++) {
+                        const unsigned short *h = reinterpret_cast<const unsigned short *>(&bv[u]);
+#pragma unroll
+                        for (int w = 0; w < 8; w++) acc[w] = ptx::fma_f16_f32(xf[u], h[w], acc[w]);
+                    }
+                    continue;
+                }
 #pragma unroll
                 for (int u = 0; u < U; u++) {
                     const int cu = __shfl_sync(gmask, c, (t + u) & (LPR - 1), LPR);
@@ -908,10 +962,25 @@ int rows_blocks(const RowsJob &a, const RowsShape &sh, int slices) // per N-slic
 {
     const long long groups = kRowsThreads / sh.lpr, keys = (long long)a.nnz - a.base + a.M;
     const long long wave = 2 * kSMs; // resident blocks
-    // whole waves over all slices (3001 x 1777 at 92 %, N = 203: 419 blocks, 1.4 waves, 41.6 us; 296 34.5 us)
+    // whole waves over all slices (3001 x 1777 at 92 %, N = 203: 419 blocks, 1.4 waves, 41.6 us; 296 34.5 us, before the short path)
     const long long waves = std::max(1LL, (keys * slices / (groups * 64) + wave / 2) / wave);
     const long long n = std::min(std::max(1LL, waves * wave / slices), (keys + groups * 8 - 1) / (groups * 8));
     return (int)std::max<long long>(1, std::min<long long>(n, a.M));
+}
+
+// The kernel with the short path (kFastLpr) or without.
+template <typename OutT, int LPR, int W, bool VEC, bool VC, int CAP> auto rows_kernel(const RowsBatchT<CAP> &b)
+{
+    if constexpr (!VEC || LPR < kFastLpr) {
+        return &spmm_rows_kernel<OutT, LPR, W, VEC, VC, CAP, false>;
+    } else if constexpr (LPR == 32) {
+        return &spmm_rows_kernel<OutT, LPR, W, VEC, VC, CAP, true>;
+    } else {
+        for (int i = 0; i < b.n_jobs; i++)
+            if ((long long)b.job[i].nnz - b.job[i].base <= (long long)kFastMean * b.job[i].M)
+                return &spmm_rows_kernel<OutT, LPR, W, VEC, VC, CAP, false>;
+        return &spmm_rows_kernel<OutT, LPR, W, VEC, VC, CAP, true>;
+    }
 }
 
 // beside: a programmatic dependent of the tensor-core launch before it (as
@@ -937,9 +1006,9 @@ int launch_rows(const RowsBatchT<kMaxCcJobs> &b, cudaStream_t s, bool beside)
         one.block_start[0] = 0;
         one.block_start[1] = grid;
         one.job[0] = b.job[0];
-        TCA_CUDA_TRY(cudaLaunchKernelEx(&cfg, spmm_rows_kernel<OutT, LPR, W, VEC, VEC, 1>, one));
+        TCA_CUDA_TRY(cudaLaunchKernelEx(&cfg, rows_kernel<OutT, LPR, W, VEC, VEC, 1>(one), one));
     } else {
-        TCA_CUDA_TRY(cudaLaunchKernelEx(&cfg, spmm_rows_kernel<OutT, LPR, W, VEC, VEC, kMaxCcJobs>, b));
+        TCA_CUDA_TRY(cudaLaunchKernelEx(&cfg, rows_kernel<OutT, LPR, W, VEC, VEC, kMaxCcJobs>(b), b));
     }
     return TCA_OK;
 }
@@ -1051,7 +1120,7 @@ template <typename OutT> int launch_rows_short(const RowsJob &a, int lpr, int sl
 
 template <typename OutT, int LPR> int launch_rows_padded(const RowsBatchT<1> &b, cudaStream_t s)
 {
-    spmm_rows_kernel<OutT, LPR, 8, true, false, 1><<<b.block_start[1], kRowsThreads, 0, s>>>(b);
+    rows_kernel<OutT, LPR, 8, true, false, 1>(b)<<<b.block_start[1], kRowsThreads, 0, s>>>(b);
     TCA_CUDA_TRY(cudaGetLastError());
     return TCA_OK;
 }
@@ -1090,7 +1159,7 @@ struct Scratch {
 // A forward whose B or C does not allow 16-byte accesses (an odd N, unaligned
 // rows) through an aligned copy of B, when that pays: two-byte accesses gather
 // B at about half the rate of 16-byte ones (3001 x 1777 at 92 %, N = 203: 48
-// us; 2 us for the copy and 34 us after it), and a plan's tensor-core
+// us; 2 us for the copy and 26 us after it), and a plan's tensor-core
 // windows can run on the tensor cores again. That needs an aligned C too, so
 // the sums go to an FP32 buffer and from there to C; only for FP16 C, whose
 // rounding (2^-11) is far above what separates the two kernels' FP32 sums (4096

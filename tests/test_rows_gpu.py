@@ -91,3 +91,29 @@ def test_rows_malformed(cuda):
         C = tca_spmm.spmm_csr(rp, ci, v, B[:, :N].contiguous(), K=8, out_dtype=torch.float32)
         torch.cuda.synchronize()
         assert C.shape == (5, N)
+
+
+@pytest.mark.parametrize("N", [64, 128, 136, 256])
+@pytest.mark.parametrize("per_row", [20, 100])  # the short rows kernel, the rows kernel
+def test_rows_malformed_columns(cuda, N, per_row):
+    """Columns out of range among valid ones, at the start, inside and at the end
+    of a row: they add nothing, also over infinite rows of B; the others add up."""
+    rng = np.random.default_rng(N + per_row)
+    M, K = 37, 300
+    col = np.concatenate([np.sort(rng.choice(np.arange(1, K), per_row, replace=False)) for _ in range(M)])
+    col = col.astype(np.int32)
+    bad = rng.random(col.size) < 0.04
+    bad[[0, per_row, col.size - 1]] = True
+    bad[5 * per_row:9 * per_row] = False
+    ok = np.where(bad, 0, col)
+    col[bad] = rng.choice([-1, K, -2 ** 31, 2 ** 31 - 1], bad.sum())
+    vals = rng.standard_normal(col.size).astype(np.float16)
+    B = rng.uniform(-1, 1, (K, N)).astype(np.float16)
+    A = np.zeros((M, K))
+    A[np.repeat(np.arange(M), per_row)[~bad], ok[~bad]] = vals[~bad]
+    ref, mag = A @ B.astype(np.float64), np.abs(A) @ np.abs(B.astype(np.float64))
+    B[0] = np.inf  # no valid nonzero has column 0
+    rp = torch.arange(0, M * per_row + 1, per_row, dtype=torch.int32, device=cuda)
+    dev = [torch.from_numpy(x).to(cuda) for x in (col, vals, B)]
+    C = tca_spmm.spmm_csr(rp, *dev, K=K, out_dtype=torch.float32)
+    assert np.all(np.abs(C.cpu().numpy() - ref) <= per_row * 2.0 ** -23 * mag)
