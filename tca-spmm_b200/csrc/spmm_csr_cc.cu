@@ -102,8 +102,8 @@ constexpr int kRowsThreads = 512;
 // N = 256: 33 -> 27 us; 1500 x 900, N = 301: 48 -> 56).
 constexpr long long kSortedRowKey = 8;
 // U nonzeros that lie in one row and whose columns are valid, as almost all do,
-// need neither predicates nor zeros for absent loads: 16 warp instructions per
-// nonzero instead of 50 (4096 x 4096 at 95 %, N = 512: 118 -> 82 us; 4096 x 1024
+// need neither predicates nor zeros for absent loads (54 warp instructions per
+// nonzero without this path; 4096 x 4096 at 95 %, N = 512: 118 -> 82 us; 4096 x 1024
 // at 80 %, Zipf, N = 256: 73 -> 53 us, 8.1 TB/s of B rows from L2; 3001 x 1777, N =
 // 203: 40 -> 29 us). Groups of fewer lanes meet too many row ends side by side
 // in a warp, which then runs both paths (300 x 4096, N = 32: 23.4 us without, 27.8
