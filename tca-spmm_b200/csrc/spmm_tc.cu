@@ -238,7 +238,7 @@ constexpr int kSlabBits = 26;
 constexpr uint32_t kSlabMask = (1u << kSlabBits) - 1u;
 struct __align__(16) TcRecordB {
     const void *b; // tensor map; condensed columns: the column list
-    int col0;      // first of 64 consecutive columns; condensed columns: -1 - item; kByScatter: left to a scatter warp
+    int col0;      // first of 64 consecutive columns; condensed columns: -1 - item; kByScatter: a scatter warp gathers them
     uint32_t x;    // 128-byte slab of n0 | slabs of the slice << kSlabBits | top bit: one 3-D box
 };
 
@@ -325,7 +325,12 @@ __device__ __forceinline__ void store_rows(uint32_t acc, OutT *C, int ldc, int o
 //     range -- are made 32 at a time, one per lane, from loads issued 32
 //     chunks ahead, and kept in shared memory, so that one elected lane can
 //     walk the chunks alone: acquire the stage ("empty"), set its part of the
-//     "full" transaction count and issue. B: ONE 3-D box of 64 rows x NT
+//     "full" transaction count and issue. Both do the first two for every
+//     chunk, whoever issues its copies: "full" then needs them once per pass
+//     over the ring, and "empty" holds them back, so neither is ever more than
+//     one phase from a barrier it waits on or arrives at (a parity tells no
+//     more apart; a loader that skipped chunks would run ahead, or fall
+//     behind, by whole passes). B: ONE 3-D box of 64 rows x NT
 //     columns for a direct chunk (64-column slabs as the third dimension; 2-D
 //     boxes of one slab each when N is not whole slabs), tile::gather4 for
 //     condensed ones (by all lanes). A: the dense image (cp.async.bulk), or
@@ -344,7 +349,9 @@ __device__ __forceinline__ void store_rows(uint32_t acc, OutT *C, int ldc, int o
 //     while the chunk's B rows are still on their way; image chunks pass them
 //     by. A condensed chunk's warp also issues its B rows' gathers (32 ns
 //     each, 64 of them at N = 256: one loader warp would pace the ring; 2000 x
-//     16384 at 99.6 %, N = 256: 102 us, 42 us this way). (A warp per chunk and not all four per chunk: the steps of a chunk
+//     16384 at 99.6 %, N = 256: 102 us, 42 us this way); the loader of B
+//     counts their bytes in, before or after they land ("full" cannot complete
+//     without its arrival). (A warp per chunk and not all four per chunk: the steps of a chunk
 //     are a chain of ~0.6 us, and four chunks then run through it at once.)
 //     Sparse chunk q uses slot q % kSlots; it is filled when chunk g is
 //     issued, at most kAhead chunks before its own, so sparse chunk q -
@@ -521,15 +528,17 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
             const int ge = min(total_chunks, g + 32);
             int s1 = s;
             uint32_t phase1 = phase;
-            if (__all_sync(0xffffffffu, g + lane >= ge || rec_b[(g + lane) % kRecordsB].col0 >= 0)) {
-                // direct chunks only: one lane alone
+            // direct chunks and those whose gathers a scatter warp issues: one lane alone
+            const int first_col = g + lane < ge ? rec_b[(g + lane) % kRecordsB].col0 : 0;
+            if (__all_sync(0xffffffffu, first_col >= 0 || first_col == kByScatter)) {
                 if (elect_one()) {
                     TcRecordB r = rec_b[g % kRecordsB];
                     for (int h = g; h < ge; h++) {
                         const TcRecordB nxt = rec_b[(h + 1) % kRecordsB];
                         if (!mbar_wait(&empty[s1], phase1)) { ok = false; break; }
                         mbar_arrive_expect_tx(&full[s1], (uint32_t)boxes(r) * (kChunkCols * 128));
-                        issue_boxes(r, s1);
+                        if (r.col0 >= 0)
+                            issue_boxes(r, s1);
                         if (++s1 == S) { s1 = 0; phase1 ^= 1; }
                         r = nxt;
                     }
@@ -543,7 +552,7 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
                 fetch_cols(rec_b[g % kRecordsB]);
                 for (int h = g; h < ge; h++) {
                     const TcRecordB r = rec_b[h % kRecordsB];
-                    if (elect_one() && r.col0 != kByScatter) {
+                    if (elect_one()) {
                         ok = mbar_wait(&empty[s1], phase1);
                         if (ok) {
                             mbar_arrive_expect_tx(&full[s1], (uint32_t)boxes(r) * (kChunkCols * 128));
@@ -717,9 +726,6 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
                 const int4 it = items[pd.z];
                 const TcJob &a = batch.job[it.w >> 16];
                 const int boxes = width(a) / Cfg::kBoxCols, n0 = (it.w & 0xffff) * width(a);
-                if (elect_one())
-                    mbar_arrive_expect_tx(&full[pd.x], (uint32_t)boxes * (kChunkCols * 128));
-                __syncwarp();
                 const int4 y = reinterpret_cast<const int4 *>(smem + Cfg::kColsOff + slot * kChunkCols * 4)[lane & 15];
                 const uint32_t b_s = smem_u32(At) + kATileBytes + (lane & 15) * 512;
                 for (int g = lane; g < 16 * boxes; g += 32)
