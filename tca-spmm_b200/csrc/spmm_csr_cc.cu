@@ -112,6 +112,12 @@ constexpr long long kSortedRowKey = 8;
 // 90 %, N = 99: 76 without, 58 with).
 constexpr int kFastLpr = 16, kFastMean = 64;
 constexpr int kRowsMax = kRowsThreads; // rows in shared memory at a time: a thread each
+// Positions of those rows' nonzeros, laid end to end, are 32-bit numbers.
+// Offsets that are not increasing can make rows overlap, so that 512 of them
+// hold more than that: the rows taken at a time end where the next one would
+// pass this many (two groups' lanes below the largest int, as positions are
+// looked at that far ahead).
+constexpr int kRowsNnz = 0x7fffffff - 64;
 
 struct RowsJob {
     const int *row_ptr, *col;
@@ -183,8 +189,8 @@ __global__ void __launch_bounds__(kRowsThreads, 2) spmm_rows_kernel(const __grid
     }
     __syncthreads();
     const int row_end = s_range[1];
-    for (int row0 = s_range[0]; row0 < row_end; row0 += kRowsMax) {
-    const int n_rows = min(kRowsMax, row_end - row0);
+    for (int row0 = s_range[0], n_rows = 0; row0 < row_end; row0 += n_rows) {
+    n_rows = min(kRowsMax, row_end - row0);
     { // the rows' starts and the prefix sums of their lengths
         int len = 0;
         if ((int)threadIdx.x < n_rows) {
@@ -193,25 +199,27 @@ __global__ void __launch_bounds__(kRowsThreads, 2) spmm_rows_kernel(const __grid
             len = en - st;
             s_start[threadIdx.x] = st;
         }
+        auto add = [](int x, int y) -> int { return (int)min((unsigned)x + (unsigned)y, 0x7fffffffu); }; // saturating
         int sum = len;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const int v = __shfl_up_sync(0xffffffffu, sum, o);
-            if (lane >= o) sum += v;
+            if (lane >= o) sum = add(sum, v);
         }
         if (lane == 31) s_warp[warp] = sum;
         __syncthreads();
         int carry = 0;
-        for (int k = 0; k < warp; k++) carry += s_warp[k];
-        if ((int)threadIdx.x < n_rows) s_pre[threadIdx.x + 1] = carry + sum;
+        for (int k = 0; k < warp; k++) carry = add(carry, s_warp[k]);
+        sum = add(carry, sum);
+        if ((int)threadIdx.x < n_rows) s_pre[threadIdx.x + 1] = sum;
         if (threadIdx.x == 0) s_pre[0] = 0;
+        n_rows = max(1, __syncthreads_count((int)threadIdx.x < n_rows && sum <= kRowsNnz));
     }
-    __syncthreads();
     const int total = s_pre[n_rows];
     // a valid CSR's rows follow one another: position v is nonzero first + v
     const int first = s_start[0];
     const bool dense = __syncthreads_and((int)threadIdx.x >= n_rows ||
-                                         s_start[threadIdx.x] == first + s_pre[threadIdx.x]);
+                                         (unsigned)s_start[threadIdx.x] == (unsigned)first + (unsigned)s_pre[threadIdx.x]);
     auto run_start = [&](int k) -> int { return (int)((long long)total * k / G); };
     // the row that holds position v of the block's nonzeros: the last one starting at or before v
     auto row_of = [&](int v) -> int {
