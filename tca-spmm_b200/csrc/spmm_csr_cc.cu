@@ -18,6 +18,7 @@
 // Malformed CSR never faults: row ranges are clamped to [0, nnz] and
 // nonzeros whose column is outside [0, K) contribute nothing.
 #include <algorithm>
+#include <climits>
 #include <memory>
 #include <vector>
 #include <cuda_fp8.h>
@@ -170,18 +171,19 @@ __global__ void __launch_bounds__(kRowsThreads, 2) spmm_rows_kernel(const __grid
             len = 0;
         }
         while (__syncthreads_or(len > 0)) { // both halves take the same number of rounds
-            const int step = (len + kProbes - 1) / kProbes;
+            // (unsigned: with nearly 2^31 rows the last probes' offsets pass the largest int)
+            const unsigned step = ((unsigned)len + kProbes - 1) / kProbes, probe = (unsigned)p * step;
             if (p == 0) s_range[half] = kProbes; // probe p is row lo + p * step
             __syncthreads();
-            if (p * step < len) {
-                const int r = lo + p * step;
+            if (probe < (unsigned)len) {
+                const int r = lo + (int)probe;
                 if ((long long)min(max(__ldg(a.row_ptr + r), 0), a.nnz) + row_key * r >= bound) atomicMin(&s_range[half], p);
             }
             __syncthreads();
-            const int first = s_range[half];
+            const unsigned first = (unsigned)s_range[half];
             if (len > 0) { // the row lies after probe first - 1 and not after probe first
-                const int hi = lo + min(len, first * step);
-                if (first > 0) lo += (min(first, (len + step - 1) / step) - 1) * step + 1;
+                const int hi = lo + (int)min((unsigned)len, first * step);
+                if (first > 0) lo += (int)((min(first, ((unsigned)len + step - 1) / step) - 1) * step) + 1;
                 len = hi - lo;
             }
         }
@@ -457,7 +459,6 @@ __global__ void __launch_bounds__(kRowsThreads, 2) spmm_rows_short_kernel(const 
     if (threadIdx.x == 0)
         s_n = 0;
     __syncthreads();
-    auto row_of = [&](int i) { return (int)blockIdx.x + i * (int)gridDim.x; };
     auto range = [&](int r, int &start, int &end) {
         start = __ldg(a.row_ptr + r);
         end = __ldg(a.row_ptr + r + 1);
@@ -528,8 +529,8 @@ __global__ void __launch_bounds__(kRowsThreads, 2) spmm_rows_short_kernel(const 
         store8(cp, o);
     };
     float acc[8];
-    const int r = row_of(g);
-    if (r < a.M) { // uniform across the group
+    const int r = (int)(blockIdx.x + (unsigned)g * gridDim.x);
+    if ((unsigned)r < (unsigned)a.M) { // uniform across the group; (the rounded-up row count can pass the largest int)
         int start, end;
         range(r, start, end);
         if (end - start > kShortRow) {
@@ -973,7 +974,7 @@ int rows_blocks(const RowsJob &a, const RowsShape &sh, int slices) // per N-slic
     // whole waves over all slices (3001 x 1777 at 92 %, N = 203: 419 blocks, 1.4 waves, 41.6 us; 296 34.5 us, before the short path)
     const long long waves = std::max(1LL, (keys * slices / (groups * 64) + wave / 2) / wave);
     const long long n = std::min(std::max(1LL, waves * wave / slices), (keys + groups * 8 - 1) / (groups * 8));
-    return (int)std::max<long long>(1, std::min<long long>(n, a.M));
+    return (int)std::max<long long>(1, std::min<long long>({n, a.M, INT_MAX / slices}));
 }
 
 // The kernel with the short path (kFastLpr) or without.
@@ -1115,7 +1116,7 @@ k_unpad_rows(const float *__restrict__ sums, int lds, const int *__restrict__ pe
 template <typename OutT> int launch_rows_short(const RowsJob &a, int lpr, int slices, cudaStream_t s)
 {
     const int groups = kRowsThreads / lpr;
-    const dim3 grid((unsigned)((a.M + groups - 1) / groups), (unsigned)slices);
+    const dim3 grid(((unsigned)a.M + groups - 1) / groups, (unsigned)slices);
     switch (lpr) {
     case 4: spmm_rows_short_kernel<OutT, 4><<<grid, kRowsThreads, 0, s>>>(a); break;
     case 8: spmm_rows_short_kernel<OutT, 8><<<grid, kRowsThreads, 0, s>>>(a); break;
