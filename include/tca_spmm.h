@@ -156,7 +156,9 @@ TCA_API int tca_plan_create(const int *d_row_ptr, const int *d_col_idx, const vo
 /* Re-gathers new values for the same sparsity pattern into the plan. */
 TCA_API int tca_plan_update_values(tca_plan_t plan, const void *d_vals_f16, tca_stream_t stream);
 /* How many times the plan's values have been replaced: a caller that replaced
- * them and still finds the same count knows that the plan holds its values. */
+ * them and still finds the same count, which is not 0, knows that the plan
+ * holds its values. 0: never, or not known -- an update has been captured in a
+ * CUDA graph, and no replay of it is counted. */
 TCA_API int tca_plan_values_version(tca_plan_t plan, unsigned long long *version);
 TCA_API int tca_plan_info(tca_plan_t plan, tca_plan_info_t *info);
 /* Copies one plan array (tca_plan_array_t) to host memory; *out_bytes gets its

@@ -1327,6 +1327,11 @@ int tca_plan_update_values(tca_plan_t p, const void *d_vals_f16, tca_stream_t st
     auto blocks = [](const ValueJob &j) { return j.val_blocks + j.n_chunks; };
     const ValueJob a = job(p, nullptr), t = p->tplan ? job(p->tplan, p->t_src) : a;
     const int first = blocks(a), total = first + (p->tplan ? blocks(t) : 0);
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        p->values_captured = true;
+    }
     p->values_version++;
     k_update_values<<<total, 256, 0, s>>>(a, t, first, (const __half *)d_vals_f16);
     TCA_CUDA_TRY(cudaGetLastError());
@@ -1337,7 +1342,7 @@ int tca_plan_values_version(tca_plan_t p, unsigned long long *version)
 {
     clear_error();
     if (!p || !version) return set_error(TCA_ERR_INVALID_ARG, "NULL argument");
-    *version = p->values_version.load();
+    *version = p->values_captured ? 0 : p->values_version.load();
     return TCA_OK;
 }
 

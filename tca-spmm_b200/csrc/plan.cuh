@@ -83,8 +83,10 @@ struct tca_plan {
     // all_items, images).
     void *arena[3] = {nullptr, nullptr, nullptr};
     size_t bytes = 0;
-    // counts tca_plan_update_values calls
+    // counts tca_plan_update_values calls; values_captured: one of them was
+    // captured in a CUDA graph, whose replays replace the values uncounted
     std::atomic<unsigned long long> values_version{0};
+    std::atomic<bool> values_captured{false};
     // A^T as a plan of its own (built on first use by tca_spmm_t or by
     // tca_plan_build_transpose), with t_src mapping each of its entries to the
     // caller's nonzero index.

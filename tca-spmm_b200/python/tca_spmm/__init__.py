@@ -296,7 +296,8 @@ class Plan:
         _check(self._lib.tca_plan_update_values(self._h, _ptr(vals), _stream_handle(stream)))
 
     def values_version(self) -> int:
-        """How many times the plan's values have been replaced (tca_plan_values_version)."""
+        """How many times the plan's values have been replaced; 0: never, or not
+        known because an update was captured in a CUDA graph (tca_plan_values_version)."""
         v = ctypes.c_ulonglong()
         _check(self._lib.tca_plan_values_version(self._h, ctypes.byref(v)))
         return v.value

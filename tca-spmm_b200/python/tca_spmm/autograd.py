@@ -33,8 +33,10 @@ class SpMMFunction(torch.autograd.Function):
         plan = ctx.plan
         dY16 = dY.to(torch.float16).contiguous()
         d_vals = d_B = None
-        # the pattern's values as they were in forward: another forward may have replaced them
-        if ctx.needs_input_grad[1] and plan.values_version() != ctx.values_version:
+        # the pattern's values as they were in forward: another forward may have
+        # replaced them, or may before a capture of this backward is replayed
+        if ctx.needs_input_grad[1] and (ctx.values_version == 0 or plan.values_version() != ctx.values_version or
+                                        torch.cuda.is_current_stream_capturing()):
             plan.update_values(v16)
         # gradients in the inputs' types: FP32 sums, rounded once by the kernel that forms them
         direct = (torch.float16, torch.float32)
