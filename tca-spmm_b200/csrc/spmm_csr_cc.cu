@@ -677,13 +677,23 @@ __device__ __forceinline__ ItemDesc load_desc(const Batch &b, int item)
             else
                 hi = mid - 1;
         }
-        const int slices = b.job[j].slices, parts = b.job[j].parts, local = item - b.item_start[j];
-        const int rest = local / slices, part = rest % parts;
-        const int2 it = __ldg(b.job[j].items + rest / parts);
-        const int rows = it.y - it.x, first = rows * part / parts;
-        d.job = j | local % slices << 8;
+        const CcJob &a = b.job[j];
+        const int slices = a.slices, parts = a.parts;
+        int local = item - b.item_start[j];
+        d.job = j;
+        if (slices > 1) {
+            d.job = j | local % slices << 8;
+            local /= slices;
+        }
+        int part = 0;
+        if (parts > 1) { // one part after the other: side by side the same part would fall to a warp every time
+            part = local / a.n_items;
+            local -= part * a.n_items;
+        }
+        const int2 it = __ldg(a.items + local);
+        const int rows = it.y - it.x, first = parts > 1 ? rows * part / parts : 0;
         d.r0 = it.x + first;
-        d.nrows = rows * (part + 1) / parts - first; // no rows: nothing to do in this part
+        d.nrows = (parts > 1 ? rows * (part + 1) / parts : rows) - first; // no rows: nothing to do in this part
     }
     return d;
 }
@@ -1715,11 +1725,21 @@ int launch_cc_jobs(const SpmmJob *jobs, int n_jobs, int c_dtype, float alpha, fl
             // rounds of loads: 4096 x 1024 at 80 %, N = 256, 290 items, 11.6 -> 5.1 us)
             // With a few rounds of items the last, partial round counts: halves
             // (32 problems, 5,056 items on 2,368 warps: the step 48.2 -> 46.6
-            // us; thirds 48.5: the loads ahead no longer cover an item).
-            a.parts = w == kCcMma            ? 1
-                      : few                  ? (int)std::max(1LL, std::min(4LL, kFewItems / (all_items * a.slices)))
-                      : all_items < 4LL * kFewItems ? 2
-                                             : 1;
+            // us; thirds 48.5: the loads ahead no longer cover an item). They
+            // pay where an item is long: its rows several times over N (5,000
+            // items of 8 rows of 4, N = 512 30.4 -> 28.7 us, N = 1024 57.4 -> 52.3;
+            // of 2 rows of 16, N = 1024 45.6 -> 41.9), or in one pass many rows and
+            // few rounds (31 rows of 1, N = 256, 5,000 items 20.1 -> 19.3, 8,500
+            // even; 3 rows of 10 14.4 -> 15.2), but not at fewer columns a lane (8 rows of 4,
+            // N = 32, 2,600 items 8.3 -> 9.0), nor with a row an item (of 50,
+            // N = 256: 19.7 -> 27.5, as halves side by side).
+            const long long rows = sj.tc ? std::min((long long)p->M, (long long)p->n_cc * kWindowRows) : p->M;
+            const bool halves = sj.N > 32 * w ? rows >= 2LL * n_items && all_items < 4LL * kFewItems
+                                              : w == 8 && rows >= 8LL * n_items && 2 * all_items < 5LL * kFewItems;
+            a.parts = w == kCcMma ? 1
+                      : few       ? (int)std::max(1LL, std::min(4LL, kFewItems / (all_items * a.slices)))
+                      : halves    ? 2
+                                  : 1;
             a.M = p->M;
             a.K = p->K;
             a.N = sj.N;
