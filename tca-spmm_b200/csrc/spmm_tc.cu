@@ -12,16 +12,16 @@
 // Work items are (job, window, NT-wide slice of N); persistent CTAs (one per
 // SM) stream the chunks of their items through a ring of kStages (A tile,
 // B tile) stages, with decoupled roles:
-//   * two loader warps move every byte through the TMA engine: one the 64 B
-//     rows of the chunk -- one box for the whole slice when its columns are 64
-//     consecutive rows of B, else tile::gather4 of the condensed columns (4
-//     rows x 128 bytes per instruction into a 128-byte swizzled N-major tile;
-//     padding columns and n >= N are out of the tensor and arrive as zeros) --,
-//     the other the chunk's pre-rendered, pre-swizzled dense A tile (chunks
-//     with >= 512 nonzeros: one 16 KB cp.async.bulk) or its packed entries
-//     (cp.async.bulk into a staging slot, four chunks ahead);
-//   * scatter warps, once a sparse chunk's entries landed and its stage is
-//     free, zero its A tile and scatter them into the swizzled K-major layout;
+//   * two loader warps: one brings the 64 B rows of a chunk whose columns are
+//     64 consecutive rows of B, one TMA box for the whole slice; the other the
+//     chunk's pre-rendered, pre-swizzled dense A tile (chunks with >= 512
+//     nonzeros: one 16 KB cp.async.bulk) or its packed entries and condensed
+//     columns (cp.async.bulk into a staging slot, four chunks ahead);
+//   * scatter warps, once those landed and the stage is free, issue a condensed
+//     chunk's tile::gather4 (4 rows x 128 bytes each into a 128-byte swizzled
+//     N-major tile; padding columns and n >= N are out of the tensor and arrive
+//     as zeros) and zero a sparse chunk's A tile and scatter its entries into
+//     the swizzled K-major layout;
 //   * one MMA lane issues 4 tcgen05.mma (K = 16 each) per chunk into the FP32
 //     accumulator in tensor memory and releases the stage with tcgen05.commit;
 //   * finally 4 warps read the accumulator (TMEM lane = row) and store
@@ -61,7 +61,7 @@ namespace {
 constexpr int kBLoaderWarp = 0;  // TMA issue of the B rows
 constexpr int kALoaderWarp = 1;  // TMA issue of the A images and entries
 constexpr int kMmaWarp = 2;      // TMEM allocation, tcgen05.mma issue
-constexpr int kScatterWarp0 = 3; // warps 3-6: sparse-entry scatter
+constexpr int kScatterWarp0 = 3; // warps 3-6: scatter of sparse entries, gathers of condensed columns
 constexpr int kScatterWarps = 4;
 constexpr int kEpiWarp0 = 7;     // warps 7-10: epilogue
 constexpr int kEpiThreads = 128;
@@ -90,6 +90,7 @@ struct TcJob {
     int M, N, ldb, ldc, ntiles;
     int nt;                  // width of its N-slices, at most the kernel's
     int tile3d;              // tmap_tile covers the whole NT-wide slice in one box
+    int gathers;             // some chunk's columns are not 64 consecutive ones
     float alpha, beta;
     unsigned flags;
 };
@@ -228,18 +229,17 @@ __device__ __forceinline__ int4 decode_item(const Batch &batch, int item)
 // A chunk as the two loaders issue it, in shared memory.
 struct __align__(16) TcRecordA {
     const void *src;  // dense image or (16-byte aligned) first entry
-    const int *cols;  // condensed sparse chunk: its columns, else NULL
+    const int *cols;  // condensed chunk: its columns, else NULL
     int bytes;        // of src: kATileBytes for an image, fewer for entries
     int ent;          // entries: count << 2 | entries before the first one
     int item;
 };
-constexpr int kByScatter = (int)0x80000000;
 constexpr int kSlabBits = 26;
 constexpr uint32_t kSlabMask = (1u << kSlabBits) - 1u;
 struct __align__(16) TcRecordB {
-    const void *b; // tensor map; condensed columns: the column list
-    int col0;      // first of 64 consecutive columns; condensed columns: -1 - item; kByScatter: a scatter warp gathers them
-    uint32_t x;    // 128-byte slab of n0 | slabs of the slice << kSlabBits | top bit: one 3-D box
+    const CUtensorMap *map;
+    int col0;   // first of 64 consecutive columns; -1: condensed ones, whose rows a scatter warp gathers
+    uint32_t x; // 128-byte slab of n0 | slabs of the slice << kSlabBits | top bit: one 3-D box
 };
 
 // 16-byte unit u of an output row: alpha x 8 accumulators as FP16, or 4 as FP32.
@@ -332,32 +332,37 @@ __device__ __forceinline__ void store_rows(uint32_t acc, OutT *C, int ldc, int o
 //     more apart; a loader that skipped chunks would run ahead, or fall
 //     behind, by whole passes). B: ONE 3-D box of 64 rows x NT
 //     columns for a direct chunk (64-column slabs as the third dimension; 2-D
-//     boxes of one slab each when N is not whole slabs), tile::gather4 for
-//     condensed ones (by all lanes). A: the dense image (cp.async.bulk), or
-//     the release of a sparse chunk to the scatter warps ("staged"), whose
-//     entries were sent for kAhead chunks before (cp.async.bulk into a
-//     staging slot, completing on its "staged").
+//     boxes of one slab each when N is not whole slabs), nothing for a
+//     condensed one, whose gathers a scatter warp issues. A: the dense image
+//     (cp.async.bulk); and the release of a sparse or condensed chunk to the
+//     scatter warps ("staged"), whose entries and columns were sent for kAhead
+//     chunks before (cp.async.bulk into a staging slot, completing on its
+//     "staged").
 //     Jobs of narrower N-slices than the kernel's run in the same launch
 //     (smaller boxes, narrower MMAs).
 //   warp 2, one lane (MMA): per chunk wait "full"; on an item's first chunk
 //     wait until its TMEM accumulator buffer (item parity) is drained
 //     ("accum_empty"); 4 x tcgen05.mma (2 for E4M3); commit "empty"; on the
 //     item's last chunk commit "accum_full".
-//   warps 3-6 (scatter): sparse chunk q belongs to warp q % 4, which, once
-//     the entries are in and the stage is free ("staged"), zeroes the A tile,
-//     writes the entries into the swizzled layout and arrives on "full" --
-//     while the chunk's B rows are still on their way; image chunks pass them
-//     by. A condensed chunk's warp also issues its B rows' gathers (32 ns
-//     each, 64 of them at N = 256: one loader warp would pace the ring; 2000 x
-//     16384 at 99.6 %, N = 256: 102 us, 42 us this way); the loader of B
-//     counts their bytes in, before or after they land ("full" cannot complete
-//     without its arrival). (A warp per chunk and not all four per chunk: the steps of a chunk
-//     are a chain of ~0.6 us, and four chunks then run through it at once.)
-//     Sparse chunk q uses slot q % kSlots; it is filled when chunk g is
-//     issued, at most kAhead chunks before its own, so sparse chunk q -
-//     kSlots lies at least kStages chunks before g and is consumed; kSlots is
-//     a multiple of 4, so a slot always belongs to one warp and no wait is
-//     more than one phase behind its barrier.
+//   warps 3-6 (scatter): the q-th sparse or condensed chunk belongs to warp
+//     q % 4, which, once its entries and columns are in and the stage is free
+//     ("staged"), issues the tile::gather4 of a condensed chunk's B rows and,
+//     for a sparse chunk, zeroes the A tile, writes the entries into the
+//     swizzled layout and arrives on "full" -- while the B rows are still on
+//     their way. Direct image chunks pass them by. A warp issues a gather every
+//     32 ns, 64 of them per chunk at N = 256, so one loader warp would pace the
+//     ring (2000 x 16384 at 99.6 %, sparse chunks, N = 256: 102 us against 42;
+//     15246 x 12743 with a few full columns, 4 in 10 chunks images, N = 128: 74
+//     us against 28; 12799 x 19423, half of them, N = 256: 65 against 22);
+//     the loader of B counts the bytes in, before or after they land ("full"
+//     cannot complete without its arrival). A warp per chunk and not all four
+//     per chunk: the steps of a chunk are a chain of ~0.6 us, and four chunks
+//     then run through it at once.
+//     Chunk q uses slot q % kSlots; it is filled when chunk g is issued, at most
+//     kAhead chunks before its own, so chunk q - kSlots lies at least kStages
+//     chunks before g and is consumed; kSlots is a multiple of 4, so a slot
+//     always belongs to one warp and no wait is more than one phase behind its
+//     barrier.
 //   warps 7-10 (epilogue): per item wait "accum_full", tcgen05.ld the rows
 //     (warp w reads TMEM lanes 32 (w % 4) ..), alpha/beta, store to C[perm],
 //     arrive "accum_empty" -- overlapping the next item's main loop.
@@ -465,7 +470,7 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     } else if (warp == kScatterWarp0 && lane == 0) {
         for (int s = 0; s < S; s++) {
-            mbar_init(&full[s], 2); // both loaders' parts (of a sparse chunk: the scatter warps')
+            mbar_init(&full[s], 2); // both loaders' parts (of a sparse chunk: the loader of B's and a scatter warp's)
             mbar_init(&empty[s], 1);
         }
         for (int s = 0; s < Cfg::kSlots; s++) mbar_init(&staged[s], 1);
@@ -498,9 +503,8 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
                 const TcJob &a = batch.job[it.w >> 16];
                 TcRecordB r;
                 const int n0 = (it.w & 0xffff) * width(a);
-                const bool direct = c0 >= 0 && c1 == c0 + kChunkCols - 1;
-                r.b = direct ? (const void *)&a.tmap_tile : (const void *)(a.win_cols + (size_t)c * kChunkCols);
-                r.col0 = direct ? c0 : img < 0 ? kByScatter : -1 - k;
+                r.map = &a.tmap_tile;
+                r.col0 = c0 >= 0 && c1 == c0 + kChunkCols - 1 ? c0 : -1;
                 r.x = (uint32_t)(n0 / Cfg::kBoxCols) | (uint32_t)(width(a) / Cfg::kBoxCols) << kSlabBits |
                       (a.tile3d ? 0x80000000u : 0u);
                 rec_b[(g0 + lane) % kRecordsB] = r;
@@ -512,13 +516,12 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
         // a direct chunk's B rows into stage s
         auto issue_boxes = [&](const TcRecordB &r, int s) {
             const uint32_t b_s = smem_u32(smem + s * Cfg::kStage) + kATileBytes;
-            const CUtensorMap *map = static_cast<const CUtensorMap *>(r.b);
             const int slab = (int)(r.x & kSlabMask);
             if (r.x >> 31) {
-                tma_tile3d(b_s, map, 0, r.col0, slab, &full[s]);
+                tma_tile3d(b_s, r.map, 0, r.col0, slab, &full[s]);
             } else {
                 for (int bx = 0; bx < boxes(r); bx++)
-                    tma_tile2d(b_s + bx * (kChunkCols * 128), map, (slab + bx) * Cfg::kBoxCols, r.col0, &full[s]);
+                    tma_tile2d(b_s + bx * (kChunkCols * 128), r.map, (slab + bx) * Cfg::kBoxCols, r.col0, &full[s]);
             }
         };
         int s = 0;
@@ -528,62 +531,20 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
             const int ge = min(total_chunks, g + 32);
             int s1 = s;
             uint32_t phase1 = phase;
-            // direct chunks and those whose gathers a scatter warp issues: one lane alone
-            const int first_col = g + lane < ge ? rec_b[(g + lane) % kRecordsB].col0 : 0;
-            if (__all_sync(0xffffffffu, first_col >= 0 || first_col == kByScatter)) {
-                if (elect_one()) {
-                    TcRecordB r = rec_b[g % kRecordsB];
-                    for (int h = g; h < ge; h++) {
-                        const TcRecordB nxt = rec_b[(h + 1) % kRecordsB];
-                        if (!mbar_wait(&empty[s1], phase1)) { ok = false; break; }
-                        mbar_arrive_expect_tx(&full[s1], (uint32_t)boxes(r) * (kChunkCols * 128));
-                        if (r.col0 >= 0)
-                            issue_boxes(r, s1);
-                        if (++s1 == S) { s1 = 0; phase1 ^= 1; }
-                        r = nxt;
-                    }
-                }
-            } else {
-                int4 ncols = make_int4(-1, -1, -1, -1); // columns of the next chunk, when it is a condensed one
-                auto fetch_cols = [&](const TcRecordB &r) {
-                    if (r.col0 < 0 && r.col0 != kByScatter && lane < 16)
-                        ncols = __ldg(reinterpret_cast<const int4 *>(r.b) + lane);
-                };
-                fetch_cols(rec_b[g % kRecordsB]);
+            if (elect_one()) {
+                TcRecordB r = rec_b[g % kRecordsB];
                 for (int h = g; h < ge; h++) {
-                    const TcRecordB r = rec_b[h % kRecordsB];
-                    if (elect_one()) {
-                        ok = mbar_wait(&empty[s1], phase1);
-                        if (ok) {
-                            mbar_arrive_expect_tx(&full[s1], (uint32_t)boxes(r) * (kChunkCols * 128));
-                            if (r.col0 >= 0)
-                                issue_boxes(r, s1);
-                        }
-                    }
-                    if (__any_sync(0xffffffffu, !ok)) break; // also: the transaction count is set
-                    if (r.col0 < 0 && r.col0 != kByScatter) {
-                        // condensed columns: gather p = lane, lane + 32, .. reads the 4 columns of lane p % 16
-                        const int4 it = items[-1 - r.col0];
-                        const TcJob &a = batch.job[it.w >> 16];
-                        const uint32_t b_s = smem_u32(smem + s1 * Cfg::kStage) + kATileBytes;
-                        const int src = lane & 15, n0 = (int)(r.x & kSlabMask) * Cfg::kBoxCols;
-                        const int y0 = __shfl_sync(0xffffffffu, ncols.x, src);
-                        const int y1 = __shfl_sync(0xffffffffu, ncols.y, src);
-                        const int y2 = __shfl_sync(0xffffffffu, ncols.z, src);
-                        const int y3 = __shfl_sync(0xffffffffu, ncols.w, src);
-                        for (int p = lane; p < 16 * boxes(r); p += 32) {
-                            const int bx = p >> 4;
-                            tma_gather4(b_s + bx * (kChunkCols * 128) + src * 512, &a.tmap_b, n0 + bx * Cfg::kBoxCols,
-                                        y0, y1, y2, y3, &full[s1]);
-                        }
-                    }
-                    if (h + 1 < ge)
-                        fetch_cols(rec_b[(h + 1) % kRecordsB]);
+                    const TcRecordB nxt = rec_b[(h + 1) % kRecordsB];
+                    if (!mbar_wait(&empty[s1], phase1)) { ok = false; break; }
+                    mbar_arrive_expect_tx(&full[s1], (uint32_t)boxes(r) * (kChunkCols * 128));
+                    if (r.col0 >= 0)
+                        issue_boxes(r, s1);
                     if (++s1 == S) { s1 = 0; phase1 ^= 1; }
+                    r = nxt;
                 }
             }
             if (__any_sync(0xffffffffu, !ok)) { ok = false; break; }
-            // the ring's place after this run of chunks (the elected lane may have walked it alone)
+            // the ring's place after this run of chunks, which the elected lane walked alone
             phase ^= (uint32_t)((s + ge - g) / S) & 1u;
             s = (s + ge - g) % S;
             g = ge;
@@ -598,32 +559,31 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
                                  : (const void *)(a.entries + (m0 & ~3));
                 r.bytes = img >= 0 ? kATileBytes : m1 > m0 ? ((m1 - (m0 & ~3)) * 4 + 15) & ~15 : 0;
                 r.ent = ((m1 - m0) << 2) | (m0 & 3);
-                r.cols = img < 0 && !(c0 >= 0 && c1 == c0 + kChunkCols - 1) ? a.win_cols + (size_t)c * kChunkCols : nullptr;
+                r.cols = c0 >= 0 && c1 == c0 + kChunkCols - 1 ? nullptr : a.win_cols + (size_t)c * kChunkCols;
                 r.item = k;
                 rec_a[(g0 + lane) % kRecords] = r;
             }
             fetch(g0 + 32 + lane, __shfl_sync(0xffffffffu, k, 31));
             __syncwarp();
         };
-        // send for the entries of chunk h if it is a sparse one
+        // send for the entries (a sparse chunk) and the columns (a condensed one) of chunk h
         int pslot = 0, slot = 0, s = 0;
         uint32_t phase = 1;
         auto prefetch = [&](int h) {
             if (h < total_chunks) {
                 const TcRecordA r = rec_a[h % kRecords];
-                if (r.bytes != kATileBytes) {
-                    if (r.bytes) {
-                        mbar_expect_tx(&staged[pslot], (uint32_t)r.bytes);
-                        bulk_copy_g2s(smem_u32(smem + Cfg::kStagingOff + pslot * kStagingBytes), r.src,
-                                      (uint32_t)r.bytes, &staged[pslot]);
-                    }
-                    if (r.cols) {
-                        mbar_expect_tx(&staged[pslot], kChunkCols * 4);
-                        bulk_copy_g2s(smem_u32(smem + Cfg::kColsOff + pslot * kChunkCols * 4), r.cols, kChunkCols * 4,
-                                      &staged[pslot]);
-                    }
-                    if (++pslot == Cfg::kSlots) pslot = 0;
+                const bool image = r.bytes == kATileBytes;
+                if (!image && r.bytes) {
+                    mbar_expect_tx(&staged[pslot], (uint32_t)r.bytes);
+                    bulk_copy_g2s(smem_u32(smem + Cfg::kStagingOff + pslot * kStagingBytes), r.src, (uint32_t)r.bytes,
+                                  &staged[pslot]);
                 }
+                if (r.cols) {
+                    mbar_expect_tx(&staged[pslot], kChunkCols * 4);
+                    bulk_copy_g2s(smem_u32(smem + Cfg::kColsOff + pslot * kChunkCols * 4), r.cols, kChunkCols * 4,
+                                  &staged[pslot]);
+                }
+                if ((!image || r.cols) && ++pslot == Cfg::kSlots) pslot = 0;
             }
         };
         make_records(0);
@@ -640,12 +600,14 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
                 for (int h = g; h < ge; h++) {
                     const TcRecordA nxt = rec_a[(h + 1) % kRecords];
                     if (!mbar_wait(&empty[s], phase)) { ok = false; break; }
-                    if (r.bytes == kATileBytes) {
+                    const bool image = r.bytes == kATileBytes;
+                    if (image) {
                         mbar_arrive_expect_tx(&full[s], kATileBytes);
                         bulk_copy_g2s(smem_u32(smem + s * Cfg::kStage), r.src, kATileBytes, &full[s]);
-                    } else {
-                        pend[slot] = make_int4(s, r.ent, r.cols ? r.item : -1, 0);
-                        mbar_arrive(&staged[slot]); // the scatter warps arrive on "full"
+                    }
+                    if (!image || r.cols) {
+                        pend[slot] = make_int4(s, r.ent, r.cols ? r.item : -1, image ? 1 : 0);
+                        mbar_arrive(&staged[slot]); // of a sparse chunk the scatter warp arrives on "full"
                         if (++slot == Cfg::kSlots) slot = 0;
                     }
                     prefetch(h + kAhead);
@@ -708,16 +670,22 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
         __syncwarp();
     } else if (warp < kEpiWarp0) {
         // ---------------- scatter ----------------
-        int n_sparse = 0, k = 0; // sparse chunks of this CTA
+        int n_mine = 0, k = 0; // sparse or condensed chunks of this CTA
         for (int g0 = 0; g0 < total_chunks; g0 += 32) {
-            bool sparse = false;
+            bool mine = false;
             if (g0 + lane < total_chunks) {
                 const int c = locate(g0 + lane, k);
-                sparse = __ldg(batch.job[items[k].w >> 16].img_idx + c) < 0;
+                const TcJob &a = batch.job[items[k].w >> 16];
+                mine = __ldg(a.img_idx + c) < 0;
+                if (a.gathers) {
+                    const int first = __ldg(a.win_cols + (size_t)c * kChunkCols);
+                    const int last = __ldg(a.win_cols + (size_t)c * kChunkCols + kChunkCols - 1);
+                    mine = mine || first < 0 || last != first + kChunkCols - 1;
+                }
             }
-            n_sparse += __popc(__ballot_sync(0xffffffffu, sparse));
+            n_mine += __popc(__ballot_sync(0xffffffffu, mine));
         }
-        for (int q = warp - kScatterWarp0; q < n_sparse; q += kScatterWarps) {
+        for (int q = warp - kScatterWarp0; q < n_mine; q += kScatterWarps) {
             const int slot = q % Cfg::kSlots;
             if (!mbar_wait(&staged[slot], (uint32_t)(q / Cfg::kSlots) & 1u)) { ok = false; break; }
             const int4 pd = pend[slot];
@@ -732,6 +700,8 @@ __global__ void __maxnreg__(64) spmm_tc_kernel(const __grid_constant__ TcBatchT<
                     tma_gather4(b_s + (g >> 4) * (kChunkCols * 128), &a.tmap_b, n0 + (g >> 4) * Cfg::kBoxCols, y.x, y.y,
                                 y.z, y.w, &full[pd.x]);
             }
+            if (pd.w) // its A tile is an image
+                continue;
 #pragma unroll 8
             for (int o = 0; o < kATileBytes / (16 * 32); o++)
                 reinterpret_cast<uint4 *>(At)[lane + o * 32] = make_uint4(0, 0, 0, 0);
@@ -1366,6 +1336,7 @@ int make_job(const SpmmJob &sj, float alpha, float beta, unsigned flags, int NT,
     // 48 KB chunks: 0.38 us per chunk against 0.44 us with a 2-D box per slab);
     // else the tensor map must know where a row ends inside a slab.
     j.tile3d = NT > 0 && sj.N % slab == 0;
+    j.gathers = p->has_gathers;
     if (NT == 0)
         NT = kPairN;
     if (sj.f8) {
