@@ -162,8 +162,11 @@ k_order_small(const int *__restrict__ row_nnz, const int *__restrict__ row_sorte
 }
 
 // Exclusive prefix sum of n values into out[0, n] (out[n] = the total), by one
-// block: the tile offsets of up to kScanSmallMax chunks.
-constexpr int kScanThreads = 1024, kScanItems = 8, kScanSmallMax = 8 * kScanThreads * kScanItems;
+// block: the tile offsets of up to kScanSmallMax chunks. Having k_tile_count's
+// last block do it saves a launch and costs each of its blocks a fence and an
+// atomic on one address, 3 ns each (14,649 chunks, 58,596 blocks: 559 us, 375
+// without).
+constexpr int kScanThreads = 1024, kScanItems = 8, kScanSmallMax = 512;
 using SmallScan = cub::BlockScan<int, kScanThreads>;
 
 __device__ void scan_small(const int *in, int n, int *out, typename SmallScan::TempStorage &tmp)
@@ -491,14 +494,14 @@ constexpr int kTileBlocksPerChunk = kWindowRows / 32;
 // which is zeroed beforehand.
 // (Two blocks per SM: the scan at the end would otherwise double the registers
 // of every block, 8.8 -> 19.8 us for the headline problem.)
-__global__ void __launch_bounds__(1024, 2)
+template <bool SCAN> // the last block turns the counts into tile_ptr
+__global__ void __launch_bounds__(1024, SCAN ? 2 : 1)
 k_tile_count(const int2 *__restrict__ chunk_win, const int4 *__restrict__ win_info,
              const int *__restrict__ p_row_ptr, const int *__restrict__ p_col, const int *__restrict__ win_cols,
              int M, int *chunk_nnz, int2 *__restrict__ row_range, int n_chunks, int *done, int *__restrict__ tile_ptr)
 {
     static_assert(kScanThreads == 1024, "the block that scans has k_tile_count's threads");
-    __shared__ typename SmallScan::TempStorage s_scan;
-    __shared__ int s_sum, s_last;
+    __shared__ int s_sum;
     const int chunk = blockIdx.x / kTileBlocksPerChunk;
     const int lane = threadIdx.x & 31, lr = (blockIdx.x % kTileBlocksPerChunk) * 32 + (threadIdx.x >> 5);
     if (threadIdx.x == 0)
@@ -528,17 +531,19 @@ k_tile_count(const int2 *__restrict__ chunk_win, const int4 *__restrict__ win_in
     if (threadIdx.x == 0) {
         if (s_sum > 0)
             atomicAdd(&chunk_nnz[chunk], s_sum); // integer sums: order-independent
-        if (tile_ptr) {
+    }
+    if constexpr (SCAN) {
+        __shared__ typename SmallScan::TempStorage s_scan;
+        __shared__ int s_last;
+        if (threadIdx.x == 0) {
             __threadfence();
             s_last = atomicAdd(done, 1) == (int)gridDim.x - 1;
         }
-    }
-    if (!tile_ptr)
-        return;
-    __syncthreads();
-    if (s_last) { // every block's counts are in: this one turns them into the tile offsets
-        __threadfence();
-        scan_small(chunk_nnz, n_chunks, tile_ptr, s_scan);
+        __syncthreads();
+        if (s_last) { // every block's counts are in
+            __threadfence();
+            scan_small(chunk_nnz, n_chunks, tile_ptr, s_scan);
+        }
     }
 }
 
@@ -1127,9 +1132,10 @@ int build_plan(tca_plan *p, const int *row_ptr, const int *col, const __half *va
         int *d_done5 = d_cn + n_ch + 1;
         k_tile_cols<<<n_tc, 1024, smem, s>>>(p->tc_win_info, p->p_row_ptr, p->p_col, M, K, d_bm, p->win_cols, d_cn, n_ch,
                                              d_done5, p->tile_entries + p->tc_nnz);
-        k_tile_count<<<(unsigned)n_ch * kTileBlocksPerChunk, 1024, 0, s>>>(
-            d_cw, p->tc_win_info, p->p_row_ptr, p->p_col, p->win_cols, M, d_cn, d_rr, n_ch, d_done5,
-            small_scan ? p->tile_ptr : nullptr);
+        auto count = small_scan ? k_tile_count<true> : k_tile_count<false>;
+        count<<<(unsigned)n_ch * kTileBlocksPerChunk, 1024, 0, s>>>(d_cw, p->tc_win_info, p->p_row_ptr, p->p_col,
+                                                                    p->win_cols, M, d_cn, d_rr, n_ch, d_done5,
+                                                                    p->tile_ptr);
         if (!small_scan) {
             TCA_CUDA_TRY(cub::DeviceScan::ExclusiveSum(at<char>(tb5, o_tmp), tmp, d_cn, p->tile_ptr, n_ch + 1, s));
         }
