@@ -435,9 +435,13 @@ __global__ void __launch_bounds__(kRowsThreads, 2) spmm_rows_kernel(const __grid
 // Short rows on average (at most kShortMean nonzeros), plan-free, 16-byte
 // accesses: a group of LPR lanes per row, so that a row costs four dependent
 // loads and none of the balancing above (4096 x 1024 at 99 %, N = 128: 3.4 us
-// against 8.3 us). A row of more than kShortRow nonzeros waits until the block's
-// other rows are done; then all of the block's groups take equal runs of it,
-// whose parts are added in run order. Block b takes rows b, b + gridDim.x, ..,
+// against 8.3 us). The rows of more than kShortRow nonzeros wait until the
+// block's other rows are done; then its groups are dealt to them in proportion
+// to their lengths, at least one each, take equal runs of their row, and the
+// row's first group adds the parts in run order. (All groups on one long row
+// after the other pay barriers and a sum per row: 20000 x 110, Zipf rows of 12,
+// N = 32, 58.7 us against 16.0; of 26, N = 256, 55.5 against 36.5; 16000 x 2000,
+// one row of 90 among 50 of 1, N = 32, 22.7 against 7.2.) Block b takes rows b, b + gridDim.x, ..,
 // so that neither sorted nor clustered long rows meet in one block. blockIdx.y:
 // the slice of 8 LPR columns.
 constexpr int kShortMean = 32, kShortRow = 64;
@@ -447,7 +451,7 @@ __global__ void __launch_bounds__(kRowsThreads, 2) spmm_rows_short_kernel(const 
 {
     constexpr int G = kRowsThreads / LPR, U = 4;
     __shared__ __align__(16) float s_part[G * LPR * 8];
-    __shared__ int s_list[G], s_n;
+    __shared__ int s_row[G], s_beg[G], s_end[G], s_last[G], s_n; // the long rows; the group after each one's last
     const int lane = threadIdx.x & 31, sub = lane & (LPR - 1), g = (int)threadIdx.x / LPR;
     const unsigned gmask = LPR == 32 ? 0xffffffffu : (((1u << LPR) - 1u) << (lane & ~(LPR - 1)));
     const int n0 = (int)blockIdx.y * LPR * 8 + sub * 8;
@@ -534,8 +538,12 @@ __global__ void __launch_bounds__(kRowsThreads, 2) spmm_rows_short_kernel(const 
         int start, end;
         range(r, start, end);
         if (end - start > kShortRow) {
-            if (sub == 0)
-                s_list[atomicAdd(&s_n, 1)] = r;
+            if (sub == 0) {
+                const int q = atomicAdd(&s_n, 1);
+                s_row[q] = r;
+                s_beg[q] = start;
+                s_end[q] = end;
+            }
         } else if (start < end || !(a.flags & TCA_FLAG_KEEP_EMPTY_ROWS)) {
 #pragma unroll
             for (int w = 0; w < 8; w++) acc[w] = 0.f;
@@ -545,24 +553,55 @@ __global__ void __launch_bounds__(kRowsThreads, 2) spmm_rows_short_kernel(const 
     }
     __syncthreads();
     const int n_long = s_n;
-    for (int q = 0; q < n_long; q++) {
-        const int lr = s_list[q];
-        int start, end;
-        range(lr, start, end);
-        const long long len = end - start;
+    if (n_long == 0)
+        return;
+    int q = 0, first = 0, parts = G; // the row of this group, the row's first group, their number
+    if (n_long > 1) {
+        if (threadIdx.x < 32) { // a group for each long row, the others in proportion to the rows' lengths
+            long long total = 0;
+            for (int i = lane; i < n_long; i += 32) total += s_end[i] - s_beg[i];
 #pragma unroll
-        for (int w = 0; w < 8; w++) acc[w] = 0.f;
-        run(start + (int)(len * g / G), start + (int)(len * (g + 1) / G), acc);
+            for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+            int base = 0;
+            for (int i0 = 0; i0 < n_long; i0 += 32) {
+                const int i = i0 + lane;
+                int sum = i < n_long ? 1 + (int)((long long)(G - n_long) * (s_end[i] - s_beg[i]) / total) : 0;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int v = __shfl_up_sync(0xffffffffu, sum, o);
+                    if (lane >= o) sum += v;
+                }
+                if (i < n_long) s_last[i] = base + sum;
+                base += __shfl_sync(0xffffffffu, sum, 31);
+            }
+        }
+        __syncthreads();
+        int hi = n_long; // the first row whose groups end after this one
+        while (q < hi) {
+            const int mid = (q + hi) >> 1;
+            if (s_last[mid] <= g) q = mid + 1;
+            else hi = mid;
+        }
+        first = q > 0 ? s_last[q - 1] : 0;
+        parts = q < n_long ? s_last[q] - first : 0;
+    }
+#pragma unroll
+    for (int w = 0; w < 8; w++) acc[w] = 0.f;
+    if (parts > 0) {
+        const int start = s_beg[q];
+        const long long len = s_end[q] - start;
+        run(start + (int)(len * (g - first) / parts), start + (int)(len * (g - first + 1) / parts), acc);
+    }
+    if (g > first) {
 #pragma unroll
         for (int w = 0; w < 8; w++) s_part[(g * LPR + sub) * 8 + w] = acc[w];
-        __syncthreads();
-        if (g == 0) {
-            for (int k = 1; k < G; k++)
+    }
+    __syncthreads();
+    if (parts > 0 && g == first) {
+        for (int k = g + 1; k < first + parts; k++)
 #pragma unroll
-                for (int w = 0; w < 8; w++) acc[w] += s_part[(k * LPR + sub) * 8 + w];
-            write(lr, acc);
-        }
-        __syncthreads(); // the parts are read before the next row's are written
+            for (int w = 0; w < 8; w++) acc[w] += s_part[(k * LPR + sub) * 8 + w];
+        write(s_row[q], acc);
     }
 }
 
