@@ -108,10 +108,11 @@ constexpr long long kSortedRowKey = 8;
 // at 80 %, Zipf, N = 256: 73 -> 53 us, 8.1 TB/s of B rows from L2; 3001 x 1777, N =
 // 203: 40 -> 29 us). Groups of fewer lanes meet too many row ends side by side
 // in a warp, which then runs both paths (300 x 4096, N = 32: 23.4 us without, 27.8
-// with), and so do groups of 16 lanes where rows are short on average (4096 x
-// 1024 at 5 %, Zipf, 51 per row, N = 128: 24.4 without, 25.0 with; 4096 x 4096 at
-// 90 %, N = 99: 76 without, 58 with).
-constexpr int kFastLpr = 16, kFastMean = 64;
+// with), and so do groups of 16 lanes where rows are short on average, from about
+// kFastMean on less than it gives (4096 x 1024 at 5 %, Zipf, 51 per row, N = 128:
+// 24.4 without, 25.0 with; equal rows of 40, 16000 x 2000, N = 96: 25.2 without,
+// 22.4 with, of 60 38.5 and 32.4; 4096 x 4096 at 90 %, N = 99: 76 and 58).
+constexpr int kFastLpr = 16, kFastMean = 32;
 constexpr int kRowsMax = kRowsThreads; // rows in shared memory at a time: a thread each
 // Positions of those rows' nonzeros, laid end to end, are 32-bit numbers.
 // Offsets that are not increasing can make rows overlap, so that 512 of them
