@@ -1205,12 +1205,19 @@ template <typename OutT> int rows_over_padded(RowsJob a, cudaStream_t s)
     }
 }
 
-// Stream-ordered scratch of one call.
+// Stream-ordered scratch of one call on a stream that is not being captured.
+// Allocating is refused while another thread captures (in the global mode), and
+// the attempt would break that capture: this thread's mode is relaxed meanwhile.
 struct Scratch {
     void *p = nullptr;
     cudaStream_t s;
-    explicit Scratch(cudaStream_t st) : s(st) {}
-    ~Scratch() { dev_free(p, s); }
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    explicit Scratch(cudaStream_t st) : s(st) { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~Scratch()
+    {
+        dev_free(p, s);
+        cudaThreadExchangeStreamCaptureMode(&mode);
+    }
 };
 
 } // namespace
