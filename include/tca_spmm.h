@@ -178,11 +178,11 @@ TCA_API int tca_plan_destroy(tca_plan_t plan);
  * ldc * sizeof(C) % 16 == 0 and 16-byte aligned B and C are needed for the
  * tensor-core kernel on the operands as they are. Otherwise, where nnz * N >=
  * 2^25 and the call is not being captured, B is first copied to aligned rows
- * (stream-ordered memory of the library's pool, at most 64 MiB): with FP16 C
- * and tensor-core windows the forward runs as usual into FP32 sums (at most 64
- * MiB more) that are rounded into C once, unless B holds an infinity or NaN,
- * and with FP32 C every window runs on CUDA cores over the copy. Without the
- * copy every window runs on CUDA cores.
+ * (stream-ordered memory of the library's pool, at most 64 MiB), over which
+ * every window runs on CUDA cores. Only with path 2 (tensor cores) and FP16 C
+ * the tensor-core windows run as usual, into FP32 sums (at most 64 MiB more)
+ * that are rounded into C once; sums that are not finite are formed anew on
+ * CUDA cores. Without the copy every window runs on CUDA cores.
  * Replaces the device work of our_spmm_balanced (src/our_spmm.cu:547-559). */
 TCA_API int tca_spmm(tca_plan_t plan, const void *d_B_f16, int ldb, int N,
              void *d_C, int ldc, int c_dtype, float alpha, float beta,

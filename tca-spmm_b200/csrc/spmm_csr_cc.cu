@@ -1225,11 +1225,14 @@ struct Scratch {
 // A forward whose B or C does not allow 16-byte accesses (an odd N, unaligned
 // rows) through an aligned copy of B, when that pays: two-byte accesses gather
 // B at about half the rate of 16-byte ones (3001 x 1777 at 92 %, N = 203: 48
-// us; 2 us for the copy and 26 us after it), and a plan's tensor-core
-// windows can run on the tensor cores again. That needs an aligned C too, so
-// the sums go to an FP32 buffer and from there to C; only for FP16 C, whose
-// rounding (2^-11) is far above what separates the two kernels' FP32 sums (4096
-// x 4096 at 90 %, N = 1001: 606 -> 45 us).
+// us; 2 us for the copy and 26 us after it). The rows kernel takes the copy,
+// FP32 FMAs as without it. For a plan whose caller asked for tensor cores (path
+// 2) its tensor-core windows run there: that needs an aligned C too, so the sums
+// go to an FP32 buffer and from there to an FP16 C (4096 x 4096 at 90 %, N =
+// 1001: 45 us, 324 on CUDA cores). Not unasked: tensor-core sums lie 4 to 100
+// times as far from those in 64 bits (1058 x 3570 at 74 %, positive operands:
+// 7.6e-6 against 6.6e-8), of which the rounding to FP16 leaves little (12 drawn
+// problems: 1.000001 to 1.001 times the error of the result) but not nothing.
 // The rule: nnz * N >= 2^25 (below, the two-byte kernel takes less than ~25
 // us and the copy and its launch eat the gain), copies of at most kPadMax
 // bytes, and not under stream capture, where this call allocates nothing.
@@ -1252,7 +1255,7 @@ int spmm_padded(const SpmmJob *sj, const int *row_ptr, const int *col, const __h
     }
     if (cap != cudaStreamCaptureStatusNone)
         return TCA_OK;
-    const bool tc = sj && sj->p->n_tc > 0 && c_dtype == TCA_DTYPE_F16;
+    const bool tc = sj && sj->p->opts.path == 2 && sj->p->n_tc > 0 && c_dtype == TCA_DTYPE_F16;
     Scratch ws(s);
     if (dev_malloc(&ws.p, b_bytes + (tc ? c_bytes : 0), s) != TCA_OK) {
         cudaGetLastError();
