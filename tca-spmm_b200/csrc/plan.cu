@@ -643,21 +643,22 @@ k_update_values(const ValueJob a, const ValueJob t, int first_blocks, const __ha
         if (j.via) k = __ldg(j.via + k);
         return __ldg(vals + k);
     };
-    if (b < j.val_blocks) {
-        const int i0 = b * kValuesPerBlock + (int)threadIdx.x;
+    if (b < j.val_blocks) { // (unsigned: the last block's positions may pass the largest int)
+        const unsigned i0 = (unsigned)b * kValuesPerBlock + threadIdx.x, n = (unsigned)j.nnz;
         __half v[kValuesPerBlock / 256];
 #pragma unroll
         for (int u = 0; u < kValuesPerBlock / 256; u++)
-            if (i0 + u * 256 < j.nnz) v[u] = value(i0 + u * 256);
+            if (i0 + u * 256 < n) v[u] = value((int)(i0 + u * 256));
 #pragma unroll
         for (int u = 0; u < kValuesPerBlock / 256; u++)
-            if (i0 + u * 256 < j.nnz) j.p_val[i0 + u * 256] = v[u];
+            if (i0 + u * 256 < n) j.p_val[i0 + u * 256] = v[u];
         return;
     }
     const int c = b - j.val_blocks;
-    const int e0 = __ldg(j.tile_ptr + c), e1 = __ldg(j.tile_ptr + c + 1), img = __ldg(j.img_idx + c);
+    const unsigned e0 = (unsigned)__ldg(j.tile_ptr + c), e1 = (unsigned)__ldg(j.tile_ptr + c + 1);
+    const int img = __ldg(j.img_idx + c);
     uint8_t *image = reinterpret_cast<uint8_t *>(j.images + (size_t)max(img, 0) * kWindowRows * kChunkCols);
-    for (int e = e0 + (int)threadIdx.x; e < e1; e += 4 * 256) {
+    for (unsigned e = e0 + threadIdx.x; e < e1; e += 4 * 256) {
         uint32_t w[4];
         __half v[4];
 #pragma unroll
