@@ -168,7 +168,8 @@ struct SpmmJob {
 using LaunchList = std::vector<std::function<int(cudaStream_t)>>;
 
 // Tensor-core (tcgen05) forward over the tensor-core windows of every job
-// (jobs with tc set), in as few launches as the N-slice widths allow. With
+// (jobs with tc set), in one launch per precision and 32 jobs, whatever their
+// N-slice widths (pairs in their own). With
 // `defer` the prepared launches are appended to it instead of issued. With
 // `dependent` the E4M3 launches are programmatic dependents of the kernel
 // before them on the stream (B's quantization): their set-up runs while it ends.
