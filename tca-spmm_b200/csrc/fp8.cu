@@ -14,6 +14,7 @@
 #include <cuda_fp8.h>
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 #include "tca_internal.cuh"
 #include <cuda.h>
@@ -128,21 +129,20 @@ __device__ __forceinline__ uint4 load8raw(const QJob &q, int k, int n, bool vec)
 // reads its rows once (whole 128-byte lines, 8 of a thread's loads in flight),
 // keeps them in shared memory and folds them into column maxima; the cluster's
 // blocks read each other's maxima (distributed shared memory) and every block
-// quantizes its own rows from shared memory. HBM-bound in the limit (2 bytes
-// read and 1 written per element); at these sizes it is two dependent trips to
-// memory and a cluster barrier. It replaces four launches (clear, maxima with
-// atomics, quantize, scales; 4096 x 1024, issued one by one: 24 us from the
-// first to the last, now 7.7; as a graph 8.0, now 7.6) and, for batches, a
-// block per strip of 16 columns (32 matrices of 1024 x 256: 11.6 -> 10.0 us;
-// 1024 x 256 alone 6.7 -> 4.6). KEEP = false: the rows do not fit shared
-// memory (K > 100,000 for few columns) and are read again, from L2 for the
-// most part.
+// quantizes its own rows from shared memory. At these sizes it is two dependent
+// trips to memory and a cluster barrier. Against the tiles above (four launches;
+// 4096 x 1024, issued one by one: 24 us from the first to the last, 7.7 this way;
+// as a graph 9.3, 8.3) and, for batches, a block per strip of 16 columns (32
+// matrices of 1024 x 256: 11.6 -> 10.0 us; 1024 x 256 alone 6.7 -> 4.6). A strip
+// of few rows has one block and no cluster (64 x 2048: 4.7 us as a cluster of one,
+// 3.7). KEEP = false: the rows do not fit shared memory and are read again, from
+// L2 for the most part (narrow matrices only: the others are tiled then).
 constexpr int kQLoads = 8;                // rows a thread loads before the first use
 constexpr int kQMaxCluster = 8;
 constexpr size_t kQSmemTwo = 96 * 1024;   // two blocks per SM
 constexpr size_t kQSmemMax = 200 * 1024;
 
-template <int kQCols, bool KEEP> // kQCols: columns per strip
+template <int kQCols, bool KEEP, bool CLUSTER> // kQCols: columns per strip; a block alone: no cluster
 __global__ void __launch_bounds__(256, 4) k_quant_b(const __grid_constant__ QBatch b, int cluster)
 {
     constexpr int kQRowThreads = kQCols / 8; // threads per row (8 columns each)
@@ -201,17 +201,20 @@ __global__ void __launch_bounds__(256, 4) k_quant_b(const __grid_constant__ QBat
         for (int w = 0; w < 8; w++) v = fmaxf(v, s_m[w][threadIdx.x]);
         s_max[threadIdx.x] = v;
     }
-    ptx::cluster_sync_all(); // (a cluster of one: a block barrier)
+    if constexpr (CLUSTER) ptx::cluster_sync_all();
+    else __syncthreads();
     if ((int)threadIdx.x < kQCols) {
-        float v = 0.f;
-        for (int r = 0; r < cluster; r++)
+        float v = CLUSTER ? 0.f : s_max[threadIdx.x];
+        for (int r = 0; CLUSTER && r < cluster; r++)
             v = fmaxf(v, ptx::ld_cluster_f32(ptx::cluster_map(ptx::smem_u32(&s_max[threadIdx.x]), (uint32_t)r)));
         const float sc = scale_of(v);
         s_scale[threadIdx.x] = sc;
         if (rank == 0 && n0 + (int)threadIdx.x < q.N)
             q.scale[n0 + threadIdx.x] = __float_as_uint(sc);
     }
-    ptx::cluster_sync_all(); // the scales are there; no block of the cluster reads another's maxima any more
+    // the scales are there; no block of the cluster reads another's maxima any more
+    if constexpr (CLUSTER) ptx::cluster_sync_all();
+    else __syncthreads();
     if (n >= q.N)
         return;
     float sc[8]; // reciprocals of the column scales (B is multiplied by them)
@@ -238,6 +241,165 @@ __global__ void __launch_bounds__(256, 4) k_quant_b(const __grid_constant__ QBat
         else
             for (int i = 0; n + i < q.N && i < 8; i++) dst[i] = (uint8_t)(w[i >> 2] >> (8 * (i & 3)));
     }
+}
+
+__global__ void k_col_zero(const __grid_constant__ QBatch b)
+{
+    const QJob &q = b.job[blockIdx.z];
+    for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < q.N; n += gridDim.x * blockDim.x) q.scale[n] = 0u;
+}
+
+__device__ __forceinline__ void load8h(const QJob &q, int k, int n, bool vec, float *v)
+{
+    const __half *row = q.B + (size_t)k * q.ldb;
+    if (vec && n + 8 <= q.N) {
+        const uint4 u = __ldg(reinterpret_cast<const uint4 *>(row + n));
+        const __half2 *h = reinterpret_cast<const __half2 *>(&u);
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const float2 f = __half22float2(h[i]);
+            v[2 * i] = f.x;
+            v[2 * i + 1] = f.y;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; i++) v[i] = n + i < q.N ? __half2float(row[n + i]) : 0.f;
+    }
+}
+
+// Large matrices: four launches over tiles of 64 rows x 256 columns (maxima
+// cleared; maxima; quantization; scales in their place), the second read of B
+// from L2 where it fits. HBM-bound (60,000 x 1024, 307 MB: 61 us, 5.0 TB/s).
+// Thread (x, y) of a 32 x 8 block takes the 8 consecutive columns (one 16-byte
+// vector) 8 x of the tile's columns in the 8 consecutive rows 8 y .. of its rows,
+// so that a warp reads whole 512-byte row segments; all 8 loads of a thread are
+// issued before the first is used (blockIdx.z = matrix).
+constexpr int kQTileRows = 64, kQTileCols = 256, kQRows = kQTileRows / 8;
+
+struct QTile {
+    int n, k0, k1;
+    bool fast; // full 16-byte vectors and all kQRows rows in range
+};
+
+__device__ __forceinline__ QTile q_tile(const QJob &q)
+{
+    QTile t;
+    t.n = blockIdx.x * kQTileCols + threadIdx.x * 8;
+    t.k0 = blockIdx.y * kQTileRows + threadIdx.y * kQRows;
+    t.k1 = min(q.K, t.k0 + kQRows);
+    t.fast = vec8_ok(q) && t.n + 8 <= q.N && t.k0 + kQRows <= q.K;
+    return t;
+}
+
+__device__ __forceinline__ void load_rows8(const QJob &q, const QTile &t, uint4 *r)
+{
+#pragma unroll
+    for (int j = 0; j < kQRows; j++)
+        r[j] = __ldg(reinterpret_cast<const uint4 *>(q.B + (size_t)(t.k0 + j) * q.ldb + t.n));
+    asm volatile("" ::: "memory"); // every load issued before the first use
+}
+
+// Column absolute maxima (FP32 bit patterns order like the non-negative
+// values): per thread the maxima of its rows, per block the maxima over its
+// 8 row slices (shared memory), then one atomicMax per column and block.
+__global__ void __launch_bounds__(256) k_col_absmax(const __grid_constant__ QBatch b)
+{
+    const QJob &q = b.job[blockIdx.z];
+    if ((int)blockIdx.x * kQTileCols >= q.N || (int)blockIdx.y * kQTileRows >= q.K)
+        return; // whole block
+    __shared__ float s_m[8][8][32]; // [row slice][column in vector][vector]
+    const QTile t = q_tile(q);
+    float m[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (t.fast) {
+        uint4 r[kQRows];
+        load_rows8(q, t, r);
+#pragma unroll
+        for (int j = 0; j < kQRows; j++) {
+            const __half2 *h = reinterpret_cast<const __half2 *>(&r[j]);
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float2 f = __half22float2(h[i]);
+                m[2 * i] = fmaxf(m[2 * i], fabsf(f.x));
+                m[2 * i + 1] = fmaxf(m[2 * i + 1], fabsf(f.y));
+            }
+        }
+    } else if (t.n < q.N) {
+        const bool vec = vec8_ok(q);
+        for (int k = t.k0; k < t.k1; k++) {
+            float v[8];
+            load8h(q, k, t.n, vec, v);
+#pragma unroll
+            for (int i = 0; i < 8; i++) m[i] = fmaxf(m[i], fabsf(v[i]));
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; i++) s_m[threadIdx.y][i][threadIdx.x] = m[i];
+    __syncthreads();
+    const int c = threadIdx.y * 32 + threadIdx.x; // column of the block: vector c / 8, element c % 8
+    float v = 0.f;
+#pragma unroll
+    for (int y = 0; y < 8; y++) v = fmaxf(v, s_m[y][c & 7][c >> 3]);
+    const int col = blockIdx.x * kQTileCols + c;
+    if (col < q.N && v > 0.f) // the maxima start at 0
+        atomicMax(q.scale + col, __float_as_uint(v));
+}
+
+// Bq[k, n] = E4M3(B[k, n] / s[n]) over the thread's rows and columns.
+__global__ void __launch_bounds__(256) k_quant_cols(const __grid_constant__ QBatch b)
+{
+    const QJob &q = b.job[blockIdx.z];
+    const QTile t = q_tile(q);
+    if (t.n >= q.N || t.k0 >= q.K)
+        return;
+    float s[8]; // reciprocals of the column scales (B is multiplied by them)
+#pragma unroll
+    for (int i = 0; i < 8; i++) s[i] = 1.f / (t.n + i < q.N ? scale_of(__uint_as_float(q.scale[t.n + i])) : 1.f);
+    const bool st8 = (q.ldq & 7) == 0 && (reinterpret_cast<uintptr_t>(q.Bq) & 7u) == 0;
+    if (t.fast && st8) {
+        uint4 r[kQRows];
+        load_rows8(q, t, r);
+#pragma unroll
+        for (int j = 0; j < kQRows; j++) {
+            const __half2 *h = reinterpret_cast<const __half2 *>(&r[j]);
+            uint32_t w[2];
+#pragma unroll
+            for (int p = 0; p < 2; p++) {
+                const float2 f0 = __half22float2(h[2 * p]), f1 = __half22float2(h[2 * p + 1]);
+                const uint32_t q0 = __nv_cvt_float2_to_fp8x2(make_float2(f0.x * s[4 * p], f0.y * s[4 * p + 1]),
+                                                             __NV_SATFINITE, __NV_E4M3);
+                const uint32_t q1 = __nv_cvt_float2_to_fp8x2(make_float2(f1.x * s[4 * p + 2], f1.y * s[4 * p + 3]),
+                                                             __NV_SATFINITE, __NV_E4M3);
+                w[p] = (q0 & 0xffffu) | (q1 << 16);
+            }
+            *reinterpret_cast<uint2 *>(q.Bq + (size_t)(t.k0 + j) * q.ldq + t.n) = make_uint2(w[0], w[1]);
+        }
+        return;
+    }
+    const bool vec = vec8_ok(q);
+    for (int k = t.k0; k < t.k1; k++) {
+        float v[8];
+        load8h(q, k, t.n, vec, v);
+        uint32_t lo = 0, hi = 0;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            lo |= (uint32_t)to_e4m3(v[i] * s[i]) << (8 * i);
+            hi |= (uint32_t)to_e4m3(v[4 + i] * s[4 + i]) << (8 * i);
+        }
+        uint8_t *dst = q.Bq + (size_t)k * q.ldq + t.n;
+        if (t.n + 8 <= q.N && (reinterpret_cast<uintptr_t>(dst) & 7u) == 0) {
+            *reinterpret_cast<uint2 *>(dst) = make_uint2(lo, hi);
+        } else {
+            for (int i = 0; t.n + i < q.N && i < 8; i++) dst[i] = (uint8_t)((i < 4 ? lo : hi) >> (8 * (i & 3)));
+        }
+    }
+}
+
+// column maxima -> scales, in place
+__global__ void k_col_scale(const __grid_constant__ QBatch b)
+{
+    const QJob &q = b.job[blockIdx.z];
+    for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < q.N; n += gridDim.x * blockDim.x)
+        q.scale[n] = __float_as_uint(scale_of(__uint_as_float(q.scale[n])));
 }
 
 unsigned blocks(long long n, int per) { return (unsigned)((n + per - 1) / per); }
@@ -267,10 +429,37 @@ int quantize_b_batch(const QBatch &b, cudaStream_t s)
     while (cluster < kQMaxCluster &&
            ((strips * cluster < 2 * kSMs && maxK / (2 * cluster) >= 64) || bytes(cluster) > kQSmemTwo))
         cluster *= 2;
+    // Tiles in four launches where the matrices are large: clusters with more
+    // than 96 KB a block (75 KB for narrow strips) and more blocks than clusters
+    // of one block per SM find places for (104) take two rounds, with more than
+    // 160 KB they read most rows twice by few blocks, and in large batches the
+    // tiles keep more loads in flight (8192 x 1024: 19.2 us as clusters, 11.8 as
+    // tiles; 20,000 x 256 13.4, 10.8; 60,000 x 1024 198, 61; 8 of 8192 x 1024 109,
+    // 72). Below, the launches cost more than they give (4096 x 1024: 8.3, 9.3).
+    long long elements = 0;
+    for (int i = 0; i < b.n; i++) elements += (long long)b.job[i].K * b.job[i].N;
+    const bool narrow = cols == 64 && maxN <= 64; // a tile has 256 columns
+    const bool large = elements >= (1LL << 24) && maxK >= 1024;
+    const bool spills = bytes(cluster) > (160u << 10) ||
+                        (strips * cluster > 104 && bytes(cluster) > (cols == 64 ? 96u << 10 : 75u << 10));
+    if (!narrow && (large || spills) && blocks(maxK, kQTileRows) <= 65535u) {
+        const unsigned z = (unsigned)b.n;
+        const dim3 tiles(blocks(maxN, kQTileCols), blocks(maxK, kQTileRows), z), tile_threads(32, 8);
+        k_col_zero<<<dim3(blocks(maxN, 256), 1, z), 256, 0, s>>>(b);
+        k_col_absmax<<<tiles, tile_threads, 0, s>>>(b);
+        k_quant_cols<<<tiles, tile_threads, 0, s>>>(b);
+        k_col_scale<<<dim3(blocks(maxN, 256), 1, z), 256, 0, s>>>(b);
+        TCA_CUDA_TRY(cudaGetLastError());
+        return TCA_OK;
+    }
     const bool keep = bytes(cluster) <= kQSmemMax;
-    auto kernel = cols == 64 ? (keep ? k_quant_b<64, true> : k_quant_b<64, false>)
-                : cols == 16 ? (keep ? k_quant_b<16, true> : k_quant_b<16, false>)
-                             : (keep ? k_quant_b<8, true> : k_quant_b<8, false>);
+    auto pick = [&](auto clustered) {
+        constexpr bool c = decltype(clustered)::value;
+        return cols == 64 ? (keep ? k_quant_b<64, true, c> : k_quant_b<64, false, c>)
+             : cols == 16 ? (keep ? k_quant_b<16, true, c> : k_quant_b<16, false, c>)
+                          : (keep ? k_quant_b<8, true, c> : k_quant_b<8, false, c>);
+    };
+    auto kernel = cluster > 1 ? pick(std::true_type{}) : pick(std::false_type{});
     if (keep)
         TCA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kQSmemMax));
     cudaLaunchConfig_t cfg = {};
@@ -284,7 +473,7 @@ int quantize_b_batch(const QBatch &b, cudaStream_t s)
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = cluster > 1 ? 1 : 0;
     TCA_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, b, cluster));
     return TCA_OK;
 }
