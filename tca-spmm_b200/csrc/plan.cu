@@ -25,6 +25,7 @@
 //      work items (host).
 #include <cub/cub.cuh>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 #include <algorithm>
 #include "tca_internal.cuh"
@@ -618,20 +619,29 @@ __global__ void k_update_p_val(const int *__restrict__ src, const __half *__rest
 // in one launch: the re-ordered values, the tile entries and the dense images
 // (whose zeros stay where they are). It was seven launches (values, entries,
 // images of both plans, the transpose's gather) of 2-3 us each, the images
-// re-rendered; what bounds it now is the chain of index loads per value.
+// re-rendered; what bounds it now is the chain of index loads per value, so that
+// a thread should not walk more entries than it must: a chunk without an image
+// (fewer than 512 entries) takes half a block and one round; an image a block, or
+// four while there are few (40 images of up to 8,192 entries: 12.6 us with one,
+// 5.7 with four). Thousands of chunks of few entries are walked flat, without
+// their chunks (36,798 chunks of 100: 42 us with a block each, 18 flat; kFlatChunks).
 // 2048 x 512 at 90 % with its transpose 13.9 -> 5.3 us, 4096 x 4096 at 90 %
 // 61.5 -> 43 us.
 struct ValueJob {
     const int *src;  // position in sorted order -> nonzero (of the transpose: entry of t_src)
     const int *via;  // the transpose: entry -> caller's nonzero; NULL: src is that already
     __half *p_val;
-    const int *tile_ptr, *tile_src, *img_idx;
+    const int *tile_ptr, *tile_src, *img_idx, *img_chunk;
     uint32_t *entries;
     uint16_t *images;
     int nnz, n_chunks;
-    int val_blocks; // blocks of kValuesPerBlock values, then one per chunk
+    unsigned n_entries;
+    // blocks of kValuesPerBlock values; of kSparsePerBlock chunks without an
+    // image, or (flat) of kValuesPerBlock entries; then image_parts per image
+    int val_blocks, entry_blocks, image_parts;
+    bool flat;
 };
-constexpr int kValuesPerBlock = 1024;
+constexpr int kValuesPerBlock = 1024, kSparsePerBlock = 2, kFlatChunks = 4096;
 
 __global__ void __launch_bounds__(256)
 k_update_values(const ValueJob a, const ValueJob t, int first_blocks, const __half *__restrict__ vals)
@@ -654,27 +664,46 @@ k_update_values(const ValueJob a, const ValueJob t, int first_blocks, const __ha
             if (i0 + u * 256 < n) j.p_val[i0 + u * 256] = v[u];
         return;
     }
-    const int c = b - j.val_blocks;
-    const unsigned e0 = (unsigned)__ldg(j.tile_ptr + c), e1 = (unsigned)__ldg(j.tile_ptr + c + 1);
-    const int img = __ldg(j.img_idx + c);
-    uint8_t *image = reinterpret_cast<uint8_t *>(j.images + (size_t)max(img, 0) * kWindowRows * kChunkCols);
-    for (unsigned e = e0 + threadIdx.x; e < e1; e += 4 * 256) {
-        uint32_t w[4];
-        __half v[4];
+    // every `stride`-th of the entries [first, end), U of a thread at a time
+    auto entries = [&](int img, unsigned first, unsigned end, unsigned stride) {
+        constexpr int U = 4;
+        uint8_t *image = reinterpret_cast<uint8_t *>(j.images + (size_t)max(img, 0) * kWindowRows * kChunkCols);
+        for (unsigned e = first; e < end; e += U * stride) {
+            uint32_t w[U];
+            __half v[U];
 #pragma unroll
-        for (int u = 0; u < 4; u++)
-            if (e + u * 256 < e1) {
-                w[u] = j.entries[e + u * 256];
-                v[u] = value(__ldg(j.tile_src + e + u * 256));
-            }
+            for (int u = 0; u < U; u++)
+                if (e + u * stride < end) {
+                    w[u] = j.entries[e + u * stride];
+                    v[u] = value(__ldg(j.tile_src + e + u * stride));
+                }
 #pragma unroll
-        for (int u = 0; u < 4; u++)
-            if (e + u * 256 < e1) {
-                const uint32_t x = (uint32_t)__half_as_ushort(v[u]);
-                j.entries[e + u * 256] = (w[u] & 0xffff0000u) | x;
-                if (img >= 0)
-                    *reinterpret_cast<uint16_t *>(image + swz128_offset(w[u] >> 22, (w[u] >> 16) & 63u)) = (uint16_t)x;
-            }
+            for (int u = 0; u < U; u++)
+                if (e + u * stride < end) {
+                    const uint32_t x = (uint32_t)__half_as_ushort(v[u]);
+                    j.entries[e + u * stride] = (w[u] & 0xffff0000u) | x;
+                    if (img >= 0)
+                        *reinterpret_cast<uint16_t *>(image + swz128_offset(w[u] >> 22, (w[u] >> 16) & 63u)) = (uint16_t)x;
+                }
+        }
+    };
+    const int m = b - j.val_blocks - j.entry_blocks;
+    if (m >= 0) { // (a part of) an image chunk
+        const int img = m / j.image_parts, part = m - img * j.image_parts, c = __ldg(j.img_chunk + img);
+        const unsigned e0 = (unsigned)__ldg(j.tile_ptr + c), n = (unsigned)__ldg(j.tile_ptr + c + 1) - e0;
+        entries(img, e0 + n * part / j.image_parts + threadIdx.x, e0 + n * (part + 1) / j.image_parts, 256);
+    } else if (j.flat) { // entries of any chunks
+        const unsigned e0 = (unsigned)(b - j.val_blocks) * kValuesPerBlock;
+        entries(-1, e0 + threadIdx.x, min(e0 + kValuesPerBlock, j.n_entries), 256);
+    } else { // a chunk without an image: half a block, one round
+        constexpr int kThreads = 256 / kSparsePerBlock;
+        static_assert(kThreads * 4 >= kImageMinNnz, "a chunk without an image takes one round");
+        const int c = (b - j.val_blocks) * kSparsePerBlock + (int)threadIdx.x / kThreads;
+        if (c >= j.n_chunks)
+            return;
+        const unsigned e0 = (unsigned)__ldg(j.tile_ptr + c), e1 = (unsigned)__ldg(j.tile_ptr + c + 1);
+        if (__ldg(j.img_idx + c) < 0)
+            entries(-1, e0 + threadIdx.x % kThreads, e1, kThreads);
     }
 }
 
@@ -1328,12 +1357,17 @@ int tca_plan_update_values(tca_plan_t p, const void *d_vals_f16, tca_stream_t st
     if (!d_vals_f16) return set_error(TCA_ERR_INVALID_ARG, "values are NULL");
     cudaStream_t s = (cudaStream_t)stream;
     auto job = [](const tca_plan *q, const int *via) {
-        return ValueJob{q->src, via, q->p_val, q->tile_ptr, q->tile_src, q->img_idx, q->tile_entries, q->images,
-                        q->nnz, q->n_tc_chunks, (int)blocks_for(q->nnz, kValuesPerBlock)};
+        const bool flat = q->n_tc_chunks >= kFlatChunks && q->tc_nnz < 256LL * q->n_tc_chunks;
+        return ValueJob{q->src, via, q->p_val, q->tile_ptr, q->tile_src, q->img_idx, q->img_chunk, q->tile_entries,
+                        q->images, q->nnz, q->n_tc_chunks, (unsigned)q->tc_nnz, (int)blocks_for(q->nnz, kValuesPerBlock),
+                        (int)(flat ? blocks_for(q->tc_nnz, kValuesPerBlock) : blocks_for(q->n_tc_chunks, kSparsePerBlock)),
+                        q->n_images <= 2 * kSMs ? 4 : 1, flat};
     };
-    auto blocks = [](const ValueJob &j) { return j.val_blocks + j.n_chunks; };
+    auto blocks = [](const ValueJob &j, const tca_plan *q) {
+        return j.val_blocks + j.entry_blocks + j.image_parts * q->n_images;
+    };
     const ValueJob a = job(p, nullptr), t = p->tplan ? job(p->tplan, p->t_src) : a;
-    const int first = blocks(a), total = first + (p->tplan ? blocks(t) : 0);
+    const int first = blocks(a, p), total = first + (p->tplan ? blocks(t, p->tplan) : 0);
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
         cudaGetLastError();
